@@ -662,6 +662,9 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
         s_l = b;
         if (b > l) h(b, b - 1) = mk(0.0, 0.0);
       }
+      // shifts left by the deflation window, read between two barriers: warp 0
+      // takes them below while other warps may still be choosing their way
+      const int pend0 = s_pend;
       __syncthreads();
       l = s_l;
       if (tid == 0) stamp(0);
@@ -670,7 +673,7 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
       // (skipped at the exceptional-shift iterations and while shifts from
       // the previous one are pending).
       const bool exceptional = its == 10 || its == 20;
-      if (aed_min > 0 && !exceptional && s_pend == 0 && i - l + 1 >= aed_min) {
+      if (aed_min > 0 && !exceptional && pend0 == 0 && i - l + 1 >= aed_min) {
         const int jw = min(aed_w, i - l + 1), kw = i - jw + 1;
         const cplx s0 = kw > l ? h(kw, kw - 1) : mk(0.0, 0.0);
         cplx* T = D;               // [AW][ALD]
