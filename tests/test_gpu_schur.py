@@ -1,0 +1,53 @@
+"""The eigensolver at the edges of its QR kernel: window and strip remainders,
+the smallest orders, the order from which deflation windows run, and entries
+whose squares leave the double range.  Residuals against numpy in FP64, with
+the bound of the other eigensolver tests (1e-12 n of the matrix's scale)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from varrcwa_b200.capi import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def _check(ctx, A):
+    lam, W = ctx.eig(A)
+    n = A.shape[-1]
+    for b in range(A.shape[0]):
+        scale = np.abs(A[b]).max()
+        assert np.abs(A[b] @ W[b] - W[b] * lam[b][None, :]).max() <= 1e-12 * scale * n
+        assert np.abs(np.linalg.norm(W[b], axis=0) - 1.0).max() < 1e-12
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 11, 12, 13, 31, 32, 33, 55, 56, 57, 58, 59, 61, 64, 97, 127, 128, 129, 131,
+                               165])
+def test_orders(ctx, n):
+    rng = np.random.default_rng(n)
+    _check(ctx, rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n)))
+
+
+@pytest.mark.parametrize("scale", [1e-120, 1e-75, 1e60])
+@pytest.mark.parametrize("n", [13, 140])
+def test_scaled(ctx, n, scale):
+    rng = np.random.default_rng(n)
+    _check(ctx, scale * (rng.standard_normal((2, n, n)) + 1j * rng.standard_normal((2, n, n))))
+
+
+@pytest.mark.parametrize("n", [30, 150])
+def test_structured(ctx, n):
+    """Graded rows, a diagonal matrix, exact zeros on the subdiagonal, a
+    cyclic shift (all eigenvalues of modulus one)."""
+    rng = np.random.default_rng(n)
+    G = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    graded = G * 10.0 ** (-8.0 * np.arange(n) / n)[:, None]
+    diag = np.diag(np.arange(n) + 1.0).astype(complex)
+    block = np.triu(G)
+    block[: n // 2, : n // 2] += np.tril(G[: n // 2, : n // 2], -1)
+    shift = np.roll(np.eye(n), 1, axis=0).astype(complex)
+    _check(ctx, np.stack([graded, diag, block, shift]))

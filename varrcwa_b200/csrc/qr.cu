@@ -6,18 +6,18 @@
 // trailing nb x nb block; one Wilkinson or exceptional shift when nb = 1):
 // bulge a (warp a) is introduced at round 3a and moves one position per
 // round, so in round r it performs step k = m + r - 3a.  Bulges three apart
-// use reflectors on disjoint index pairs.  In a round every entry receives at
-// most one row transform (L) and one column transform (R), and L (X R) =
-// (L X) R, so the warps need not wait for one another inside a round: the
-// only entries two warps share are the 2 x 2 blocks where a bulge's rows
-// cross a leading bulge's columns, and the row-transforming warp applies both
-// there (L first, then R, as a row phase followed by a column phase would),
-// while the leading bulge's column transform skips those rows.  Each warp
-// then forms its bulge's next reflector, and one CTA barrier ends the round.
-// Rounds run in chunks of QB inside a diagonal
-// window D held in shared memory; after a chunk the rest of the active
-// window is updated by one thread per row or column, which carries a value
-// down each bulge's chain of the chunk (carry_chain).  Rows above the
+// use rotations on disjoint index pairs, so in a round every entry receives
+// at most one row transform and one column transform.  Rounds run in chunks
+// of QB inside a diagonal window D held in shared memory, in three steps with
+// a CTA barrier after each: one warp forms all bulges' rotations (a lane per
+// bulge), every warp transforms its bulge's rows, every warp transforms its
+// bulge's columns.  (A barrier costs some 30 cycles; merging the steps, with
+// every warp forming its own rotation and the entries that two bulges share
+// handled apart, cost about 500 instructions per warp and round, and with
+// two CTAs per SM the instruction issue is what a round is bound by: 1,900
+// cycles per round at n = 242 then, 1,140 now.)  After a chunk the rest of
+// the active window is updated from strips staged in shared memory
+// (strip_rounds).  Rows above the
 // window, columns right of it and all of Z are not touched here: every
 // sweep's rotations are logged round-major and replayed afterwards, whole
 // rounds at a time from a sliding register ring (qr_replay_rows_kernel /
@@ -52,7 +52,11 @@ constexpr int QD = QB + 3 * (NBMAX - 1) + 3;     // diagonal window size (56)
 // leading dimension of the window: odd in 16-byte units, so that the lanes
 // of a row access (stride QLD) fall in distinct shared-memory banks
 constexpr int QLD = QD + 1;
-constexpr size_t QR_SMEM = (size_t)(QD * QLD + 2 * NBMAX * QB) * sizeof(cplx);
+// strips of the active window outside D: groups of FV vectors (rows or
+// columns) per warp, at most FE entries each, double buffered in D's room
+constexpr int FV = 4, FE = QB + 3 * (NBMAX - 1) + 1;
+constexpr int QR_D = QD * QLD > NBMAX * 2 * FV * FE ? QD * QLD : NBMAX * 2 * FV * FE;
+constexpr size_t QR_SMEM = (size_t)(QR_D + NBMAX * QB) * sizeof(cplx) + (size_t)NBMAX * QB * sizeof(double);
 
 struct QrLogHeader {
   int nsweeps, nrot;
@@ -89,152 +93,109 @@ __device__ __forceinline__ cplx* log_rot(char* logb, int sweep_cap) {
   return reinterpret_cast<cplx*>(logb + QR_HDR + (size_t)sweep_cap * sizeof(QrSweep));
 }
 
-// Eigenvalues of a small upper Hessenberg matrix A (nb x nb, column-major,
-// nb <= NBMAX, shared memory) by single-shift QR, used only to pick shifts
-// (on failure to converge the remaining diagonal entries are used).  One
-// warp (all lanes call it): the reflectors are formed redundantly by every
-// lane from the same shared-memory entries (identical results), and lanes own
-// the columns of each row transform and the rows of each column transform.
-__device__ void small_eigvals_warp(cplx* A, int nb, cplx* out, int lane) {
-  auto a = [&](int r, int c) -> cplx& { return A[c * nb + r]; };
-  int hi = nb - 1, it = 0;
-  while (hi >= 0) {
-    __syncwarp();
-    if (hi == 0) {
-      if (lane == 0) out[0] = a(0, 0);
-      break;
-    }
-    int lo = hi;
-    while (lo > 0 && cabs1(a(lo, lo - 1)) > EIG_ULP * (cabs1(a(lo - 1, lo - 1)) + cabs1(a(lo, lo)))) --lo;
-    if (lo == hi) {
-      if (lane == 0) out[hi] = a(hi, hi);
-      --hi;
-      it = 0;
-      continue;
-    }
-    if (++it > 40) {
-      if (lane == 0)
-        for (int k = 0; k <= hi; ++k) out[k] = a(k, k);
-      break;
-    }
-    const cplx p = a(hi - 1, hi - 1), q = a(hi - 1, hi), r = a(hi, hi - 1), d = a(hi, hi);
-    const cplx half = cscale(csub(p, d), 0.5);
-    const cplx disc = csqrt(cadd(cmul(half, half), cmul(q, r)));
-    const cplx e1 = cadd(cadd(d, half), disc), e2 = csub(cadd(d, half), disc);
-    cplx sh = (cabs2(csub(e1, d)) < cabs2(csub(e2, d))) ? e1 : e2;
-    if (it % 10 == 0) sh = cadd(d, mk(0.75 * fabs(a(hi, hi - 1).x), 0.0));
-    for (int k = lo; k < hi; ++k) {
-      cplx x, y, beta, tau, v2;
-      if (k == lo) {
-        x = csub(a(lo, lo), sh);
-        y = a(lo + 1, lo);
-      } else {
-        x = a(k, k - 1);
-        y = a(k + 1, k - 1);
-      }
-      refl2(x, y, &beta, &tau, &v2);
-      __syncwarp();  // every lane has read x, y
-      if (k > lo && lane == 0) {
-        a(k, k - 1) = beta;
-        a(k + 1, k - 1) = mk(0.0, 0.0);
-      }
-      const cplx tauc = cconj(tau), v2c = cconj(v2);
-      const int j = k + lane;
-      if (j <= hi) {
-        cplx u = a(k, j), w = a(k + 1, j);
-        cplx s = cmul(tauc, cadd(u, cmul(v2c, w)));
-        a(k, j) = csub(u, s);
-        a(k + 1, j) = csub(w, cmul(s, v2));
-      }
-      __syncwarp();
-      const int re = min(k + 2, hi), rr = lo + lane;
-      if (rr <= re) {
-        cplx u = a(rr, k), w = a(rr, k + 1);
-        cplx s = cmul(tau, cadd(u, cmul(v2, w)));
-        a(rr, k) = csub(u, s);
-        a(rr, k + 1) = csub(w, cmul(s, v2c));
-      }
-      __syncwarp();
+// Complex Givens rotation G = [c s; -conj(s) c], c real, with
+// G (f, g)^T = (r, 0)^T.  The whole rotation comes from one reciprocal square
+// root, u = 1 / (|f| sqrt(|f|^2 + |g|^2)): c = |f|^2 u, s = f conj(g) u,
+// r = f (|f|^2 + |g|^2) u.  A reflector (sqrt, two divisions, then seven
+// dependent FMAs per application against three here) is a longer serial
+// chain at every step.  Outside the range where the squares neither over- nor
+// underflow the pair is scaled first.
+// 1 / sqrt(x) for x well inside the normal range: the hardware's double
+// approximation, then one step of Halley's (cubic) iteration,
+// y (1 + e/2 + 3/8 e^2) with e = 1 - x y^2.
+__device__ __forceinline__ double rsqrt_inrange(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+struct Rot {
+  double c;
+  cplx s, r;
+};
+__device__ __forceinline__ Rot givens(cplx f, cplx g) {
+  Rot o;
+  const double f2 = cabs2(f), d2 = f2 + cabs2(g), u = rsqrt_inrange(f2 * d2);
+  o.c = f2 * u;
+  o.s = cscale(cmul(f, cconj(g)), u);
+  o.r = cscale(f, d2 * u);
+  if (!(f2 > 1e-140 && d2 < 1e140)) {  // f zero or far smaller than g, or squares out of range
+    const double m = fmax(cabs1(f), cabs1(g)), sc = 1.0 / fmax(m, 1e-300);
+    const cplx fs = cscale(f, sc), gs = cscale(g, sc);
+    const double a2 = cabs2(fs), g2 = cabs2(gs);
+    if (g2 < 1e-290) {
+      o.c = 1.0;
+      o.s = mk(0.0, 0.0);
+      o.r = f;
+    } else if (a2 < 1e-290) {
+      const double ug = rsqrt(g2);
+      o.c = 0.0;
+      o.s = mk(gs.x * ug, -gs.y * ug);
+      o.r = mk(g2 * ug * m, 0.0);
+    } else {
+      const double us = rsqrt(a2 * (a2 + g2));
+      o.c = a2 * us;
+      o.s = cscale(cmul(fs, cconj(gs)), us);
+      o.r = cscale(f, (a2 + g2) * us);
     }
   }
+  return o;
+}
+
+// The rotation on one pair (a, b): from the left (ROWOP, G) or, on a row of
+// two columns, from the right (G^H).  The product with the pair's first
+// entry, which a carried chain waits for, comes last.
+template <bool ROWOP>
+__device__ __forceinline__ void rotate2(cplx& a, cplx& b, double c, cplx s) {
+  if (!ROWOP) s.y = -s.y;  // (p, w) -> (c p + conj(s) w, c w - s p)
+  const cplx p = a, w = b;
+  a = mk(fma(c, p.x, fma(s.x, w.x, -s.y * w.y)), fma(c, p.y, fma(s.x, w.y, s.y * w.x)));
+  b = mk(fma(-s.y, p.y, fma(-s.x, p.x, c * w.x)), fma(s.y, p.x, fma(-s.x, p.y, c * w.y)));
+}
+
+// Principal square root of a value whose square is within range.
+__device__ __forceinline__ cplx csqrt_inrange(cplx a) {
+  const double a2 = cabs2(a);
+  const double q = 0.5 * fma(a2, rsqrt_inrange(a2), fabs(a.x)), iq = rsqrt_inrange(q), t = q * iq;
+  const double o = 0.5 * a.y * iq;
+  return a.x >= 0.0 ? mk(t, o) : mk(fabs(o), copysign(t, a.y));
+}
+
+// Wilkinson's shift of the 2x2 block [p q; r t]: its eigenvalue closer to t,
+// t - q r / (x +- sqrt(x^2 + q r)) with x = (p - t) / 2 and the sign that
+// enlarges the denominator.  Out of range the entries are scaled first; a
+// vanishing square root or denominator gives t.
+__device__ __forceinline__ cplx wilkinson(cplx p, cplx q, cplx r, cplx t) {
+  cplx x = cscale(csub(p, t), 0.5);
+  double big = 1.0;
+  cplx qr = cmul(q, r), z = cadd(cmul(x, x), qr);
+  double z2 = cabs2(z);
+  if (!(z2 > 1e-250 && z2 < 1e250)) {
+    big = fmax(cabs1(x), fmax(cabs1(q), cabs1(r)));
+    if (!(big > 1e-290)) return t;
+    const double inv = 1.0 / big;
+    x = cscale(x, inv);
+    qr = cmul(cscale(q, inv), cscale(r, inv));
+    z = cadd(cmul(x, x), qr);
+    z2 = cabs2(z);
+  }
+  cplx w = z2 > 1e-280 ? csqrt_inrange(z) : mk(0.0, 0.0);
+  if (x.x * w.x + x.y * w.y < 0.0) w = cneg(w);
+  const cplx den = cadd(x, w);
+  const double d2 = cabs2(den);
+  if (!(d2 > 1e-280)) return t;
+  const double rd = rsqrt_inrange(d2);
+  return csub(t, cscale(cmul(qr, cconj(den)), big * rd * rd));
 }
 
 // Single shift for window [l, i]: exceptional at iterations 10 and 20, else
-// Wilkinson's (the eigenvalue of the trailing 2x2 block closer to H[i][i],
-// computed in scaled form).
-__device__ cplx single_shift(const cplx* H, int n, int l, int i, int its) {
+// Wilkinson's of the trailing 2x2 block.
+__device__ __forceinline__ cplx single_shift(const cplx* H, int n, int l, int i, int its) {
   auto h = [&](int r, int c) { return H[(size_t)c * n + r]; };
-  if (its == 10) return cadd(mk(0.75 * fabs(h(l + 1, l).x), 0.0), h(l, l));
-  if (its == 20) return cadd(mk(0.75 * fabs(h(i, i - 1).x), 0.0), h(i, i));
-  cplx t = h(i, i);
-  cplx uu = cmul(csqrt(h(i - 1, i)), csqrt(h(i, i - 1)));
-  double s = cabs1(uu);
-  if (s != 0.0) {
-    cplx x = cscale(csub(h(i - 1, i - 1), t), 0.5);
-    double sx = cabs1(x);
-    s = fmax(s, sx);
-    cplx xs = cscale(x, 1.0 / s), us = cscale(uu, 1.0 / s);
-    cplx yv = cscale(csqrt(cadd(cmul(xs, xs), cmul(us, us))), s);
-    if (sx > 0.0) {
-      cplx xn = cscale(x, 1.0 / sx);
-      if (xn.x * yv.x + xn.y * yv.y < 0.0) yv = cneg(yv);
-    }
-    t = csub(t, cmul(uu, cdiv(uu, cadd(x, yv))));
-  }
-  return t;
-}
-
-// One reflector I - tau v v^H, v = (1, v2), on the pair (a, b): from the
-// left (ROWOP, conj(tau)) or from the right.
-template <bool ROWOP>
-__device__ __forceinline__ void rotate2(cplx& a, cplx& b, cplx tau, cplx v2) {
-  if (ROWOP) {
-    const cplx s = cmul(cconj(tau), cadd(a, cmul(cconj(v2), b)));
-    a = csub(a, s);
-    b = csub(b, cmul(s, v2));
-  } else {
-    const cplx s = cmul(tau, cadd(a, cmul(v2, b)));
-    a = csub(a, s);
-    b = csub(b, cmul(s, cconj(v2)));
-  }
-}
-
-// Carries one value down a chain of cnt rotations on consecutive index
-// pairs (k0, k0+1), (k0+1, k0+2), ...: row transforms on a column (rowop,
-// entries p0[t], stride 1) or column transforms on a row (stride n).  The
-// entries are fetched in groups of CG, double buffered: the loads of the
-// next group are issued before the current group's rotations, so their
-// latency overlaps the arithmetic.  Every entry a rotation writes lies below
-// the next group's (the chain moves forward), so the early loads read
-// values no rotation of this chain changes.
-template <int CG>
-__device__ __forceinline__ void carry_chain(cplx* p0, size_t stride, int cnt, const cplx* taus, const cplx* v2s,
-                                            bool rowop) {
-  cplx c = p0[0];
-  cplx q[CG], qn[CG];
-#pragma unroll
-  for (int u = 0; u < CG; ++u)
-    if (u < cnt) q[u] = p0[(size_t)(u + 1) * stride];
-  for (int t0 = 0; t0 < cnt; t0 += CG) {
-#pragma unroll
-    for (int u = 0; u < CG; ++u)
-      if (t0 + CG + u < cnt) qn[u] = p0[(size_t)(t0 + CG + u + 1) * stride];
-#pragma unroll
-    for (int u = 0; u < CG; ++u) {
-      if (t0 + u < cnt) {
-        cplx b = q[u];
-        if (rowop)
-          rotate2<true>(c, b, taus[t0 + u], v2s[t0 + u]);
-        else
-          rotate2<false>(c, b, taus[t0 + u], v2s[t0 + u]);
-        p0[(size_t)(t0 + u) * stride] = c;
-        c = b;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < CG; ++u) q[u] = qn[u];
-  }
-  p0[(size_t)cnt * stride] = c;
+  if (its == 10) return cadd(mk(0.75 * cabs1(h(l + 1, l)), 0.0), h(l, l));
+  if (its == 20) return cadd(mk(0.75 * cabs1(h(i, i - 1)), 0.0), h(i, i));
+  return wilkinson(h(i - 1, i - 1), h(i - 1, i), h(i, i - 1), h(i, i));
 }
 
 // cp.async copies of 16 bytes into shared memory, one commit group each.
@@ -246,6 +207,44 @@ __device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_gro
 template <int N>
 __device__ __forceinline__ void cpa_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
+// One chunk's rotations on FV vectors held in shared memory (entry e of vector
+// v at e * FV + v), 8 lanes per vector, one per bulge.  In a round the bulges
+// act on disjoint pairs, so the lanes work side by side: a lane carries its
+// pair's second entry over to the next round, takes in the entry above it
+// (left there by the leading bulge two rounds ago, so it is fetched a round
+// ahead) and puts back the one it has passed.  p: this lane's first entry;
+// rounds [ra0, ra1) of [r0, r1) are its own.  Bank conflict free: consecutive
+// bulges are 3 FV entries apart.
+//
+// Bounded by the FP64 pipe and issue (12 FP64 instructions of about 30 per
+// round and warp).  One thread per vector and bulge after bulge, straight from
+// global memory, took 234 cycles per rotation at n = 242: on a row transform
+// every lane walks a column of its own, so each access was 32 sectors, eight
+// times over.
+template <bool ROWOP>
+__device__ __forceinline__ void strip_rounds(cplx* p, int r0, int r1, int ra0, int ra1, const double* cs,
+                                             const cplx* ss) {
+  cplx x = mk(0.0, 0.0), y = x;
+  for (int r = r0; r < r1; ++r, cs += NBMAX, ss += NBMAX) {
+    if (r >= ra0 && r < ra1) {
+      if (r == ra0) {
+        x = p[0];
+        y = p[FV];
+      }
+      const bool more = r + 1 < ra1;
+      cplx nx = mk(0.0, 0.0);
+      if (more) nx = p[2 * FV];
+      rotate2<ROWOP>(x, y, cs[0], ss[0]);
+      p[0] = x;
+      if (!more) p[FV] = y;
+      x = y;
+      y = nx;
+      p += FV;
+    }
+    __syncwarp();
+  }
 }
 
 // A group of NBG bulges' rotations applied round by round to one vector x
@@ -292,7 +291,7 @@ struct RotRing {
     }
   }
 
-  // Rounds [t0, t1) (t0 a multiple of P); rot(t, g, tau, v2) gives bulge g's
+  // Rounds [t0, t1) (t0 a multiple of P); rot(t, g, c, s) gives bulge g's
   // rotation of round t, the identity where it is outside the window
   template <class ROT>
   __device__ __forceinline__ void run(int t0, int t1, ROT rot) {
@@ -312,9 +311,10 @@ struct RotRing {
           }
 #pragma unroll
           for (int g = 0; g < NBG; ++g) {  // straight-line: inactive pairs carry the identity
-            cplx tau, v2;
-            rot(t, g, tau, v2);
-            rotate2<ROWOP>(w[(tt - 3 * g + 2 * P) % P], w[(tt - 3 * g + 1 + 2 * P) % P], tau, v2);
+            double rc;
+            cplx rs;
+            rot(t, g, rc, rs);
+            rotate2<ROWOP>(w[(tt - 3 * g + 2 * P) % P], w[(tt - 3 * g + 1 + 2 * P) % P], rc, rs);
           }
           {
             const int q = t - L, c = cb - L;
@@ -351,55 +351,47 @@ struct RotRing {
 constexpr int AW = 32;       // largest deflation window
 constexpr int ALD = AW + 1;  // its leading dimension in shared memory (odd in 16-byte units)
 
-// Givens rotation [cs sn; -conj(sn) cs] (cs real) with cs f + sn g = r and
-// -conj(sn) f + cs g = 0.
-__device__ __forceinline__ void givens(cplx f, cplx g, double* cs, cplx* sn) {
-  const double ag = hypot(g.x, g.y);
-  if (ag == 0.0) {
-    *cs = 1.0;
-    *sn = mk(0.0, 0.0);
-    return;
-  }
-  const double af = hypot(f.x, f.y);
-  if (af == 0.0) {
-    *cs = 0.0;
-    *sn = cscale(cconj(g), 1.0 / ag);
-    return;
-  }
-  const double d = hypot(af, ag);
-  *cs = af / d;
-  *sn = cscale(cmul(cscale(f, 1.0 / af), cconj(g)), 1.0 / d);
-}
-
-// Negligible subdiagonal entry T[k][k-1] of a small window (the test of the
-// main iteration: Ahues-Tisseur, LAPACK xLAHQR).
-__device__ __forceinline__ bool small_negligible(const cplx* T, int nw, int k, double smlnum) {
-  auto t = [&](int r, int c) { return T[c * ALD + r]; };
-  const double cs = cabs1(t(k, k - 1));
+// Negligible subdiagonal entry sub = T[k][k-1] between the diagonal entries
+// dkm = T[k-1][k-1] and dk = T[k][k], with sup = T[k-1][k] and the
+// neighbouring subdiagonals below and above (Ahues-Tisseur, LAPACK xLAHQR).
+__device__ __forceinline__ bool negligible(cplx sub, cplx dkm, cplx dk, cplx sup, cplx sub_up, cplx sub_dn,
+                                           double smlnum) {
+  const double cs = cabs1(sub);
   if (cs <= smlnum) return true;
-  const cplx dkm = t(k - 1, k - 1), dk = t(k, k);
   double tst = cabs1(dkm) + cabs1(dk);
-  if (tst == 0.0) {
-    if (k - 2 >= 0) tst += fabs(t(k - 1, k - 2).x);
-    if (k + 1 <= nw - 1) tst += fabs(t(k + 1, k).x);
-  }
+  if (tst == 0.0) tst = cabs1(sub_up) + cabs1(sub_dn);
   if (cs > EIG_ULP * tst) return false;
-  const double a1 = cs, a2 = cabs1(t(k - 1, k));
-  const double ab = fmax(a1, a2), ba = fmin(a1, a2);
+  const double a2 = cabs1(sup);
+  const double ab = fmax(cs, a2), ba = fmin(cs, a2);
   const double b1 = cabs1(dk), b2 = cabs1(csub(dkm, dk));
   const double aa = fmax(b1, b2), bb = fmin(b1, b2);
-  const double s = aa + ab;
-  return ba * (ab / s) <= fmax(smlnum, EIG_ULP * (bb * (aa / s)));
+  return ba * ab <= fmax(smlnum * (aa + ab), EIG_ULP * (bb * aa));
+}
+__device__ __forceinline__ bool small_negligible(const cplx* T, int nw, int k, double smlnum) {
+  auto t = [&](int r, int c) { return T[c * ALD + r]; };
+  return negligible(t(k, k - 1), t(k - 1, k - 1), t(k, k), t(k - 1, k), k >= 2 ? t(k - 1, k - 2) : mk(0.0, 0.0),
+                    k + 1 < nw ? t(k + 1, k) : mk(0.0, 0.0), smlnum);
+}
+
+__device__ __forceinline__ cplx shfl_c(cplx v, int src) {
+  return mk(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
 // Schur form of the nw x nw upper Hessenberg T (shared memory, leading
-// dimension ALD) by single-shift QR with Wilkinson shifts (exceptional at
-// iterations 10 and 20), accumulating the rotations into U.  One warp; lanes
-// own the columns of a row transform and the rows of a column transform.
-// Returns false if an eigenvalue needs more than 30 * max(10, nw) iterations.
-__device__ bool small_schur_warp(cplx* T, cplx* U, int nw, int lane, double smlnum) {
+// dimension ALD, nw <= AW) by single-shift QR with Wilkinson shifts
+// (exceptional at iterations 10 and 20), accumulating the rotations into U
+// (may be null).  One warp.  A step is explicit, T - sh I = Q R, then
+// R Q + sh I (EISPACK's comqr), because its serial chain is the shortest: in
+// the first half lane j carries column j's running entry in a register, so a
+// rotation waits for one shuffle and one rotation of the step before; in the
+// second every row is a chain of its own with all rotations known.  The
+// implicit form hands two entries through shared memory twice per rotation
+// and took 260,000 cycles for a 12 x 12 window with U.  rc, rs: room for AW
+// rotations.  Returns false if an eigenvalue needs more than 30 * max(10, nw)
+// iterations.
+__device__ bool small_schur_warp(cplx* T, cplx* U, int nw, int lane, double smlnum, double* rc, cplx* rs) {
   auto t = [&](int r, int c) -> cplx& { return T[c * ALD + r]; };
-  auto u = [&](int r, int c) -> cplx& { return U[c * ALD + r]; };
+  const cplx zero = mk(0.0, 0.0);
   const int itmax = 30 * max(10, nw);
   int hi = nw - 1, its = 0;
   while (hi > 0) {
@@ -408,8 +400,7 @@ __device__ bool small_schur_warp(cplx* T, cplx* U, int nw, int lane, double smln
     const bool negl = lane + 1 <= hi && small_negligible(T, nw, lane + 1, smlnum);
     const unsigned bal = __ballot_sync(0xffffffffu, negl);
     const int lo = bal ? 32 - __clz(bal) : 0;
-    if (lo > 0 && lane == 0) t(lo, lo - 1) = mk(0.0, 0.0);
-    __syncwarp();
+    if (lo > 0 && lane == 0) t(lo, lo - 1) = zero;
     if (lo == hi) {
       --hi;
       its = 0;
@@ -417,27 +408,52 @@ __device__ bool small_schur_warp(cplx* T, cplx* U, int nw, int lane, double smln
     }
     if (++its > itmax) return false;
     const cplx sh = single_shift(T, ALD, lo, hi, its);
-    for (int k = lo; k < hi; ++k) {
-      cplx x, y, beta, tau, v2;
-      __syncwarp();
-      if (k == lo) {
-        x = csub(t(lo, lo), sh);
-        y = t(lo + 1, lo);
-      } else {
-        x = t(k, k - 1);
-        y = t(k + 1, k - 1);
+    __syncwarp();  // every lane has read T
+    {  // rows lo..hi, columns lo..nw-1; column j on lane j
+      const int j = lane;
+      const bool in = j < nw;
+      cplx cur = (in && j >= lo) ? t(lo, j) : zero;
+      if (j == lo) cur = csub(cur, sh);
+      cplx b = (in && j > lo) ? t(lo + 1, j) : zero, y = t(lo + 1, lo);
+      for (int k = lo; k < hi; ++k) {
+        if (j == k + 1) b = csub(b, sh);
+        cplx bn = zero, yn = zero;  // the next row's entries
+        if (k + 1 < hi) {
+          if (in && j > k + 1) bn = t(k + 2, j);
+          yn = t(k + 2, k + 1);
+        }
+        const Rot g = givens(shfl_c(cur, k), y);
+        rotate2<true>(cur, b, g.c, g.s);
+        if (in && j >= k) t(k, j) = j == k ? g.r : cur;
+        if (lane == 0) {
+          rc[k] = g.c;
+          rs[k] = g.s;
+        }
+        cur = b;
+        b = bn;
+        y = yn;
       }
-      refl2(x, y, &beta, &tau, &v2);
-      __syncwarp();  // every lane has read x, y
-      if (k > lo && lane == 0) {
-        t(k, k - 1) = beta;
-        t(k + 1, k - 1) = mk(0.0, 0.0);
+      if (in && j >= hi) t(hi, j) = cur;
+    }
+    __syncwarp();
+    // columns lo..hi of the rows of T and of U: row r of M as a chain
+    auto chain = [&](cplx* M, int r, bool tri) {
+      cplx p = (tri && r > lo) ? zero : M[lo * ALD + r];
+      for (int k = lo; k < hi; ++k) {
+        cplx w = (tri && r > k + 1) ? zero : M[(k + 1) * ALD + r];
+        rotate2<false>(p, w, rc[k], rs[k]);
+        M[k * ALD + r] = (tri && r == k) ? cadd(p, sh) : p;
+        p = w;
       }
-      const int j = k + lane;  // row transform over columns k..nw-1 (nw - k <= 32)
-      if (j < nw) rotate2<true>(t(k, j), t(k + 1, j), tau, v2);
-      __syncwarp();
-      if (lane <= min(k + 2, hi)) rotate2<false>(t(lane, k), t(lane, k + 1), tau, v2);
-      if (lane < nw) rotate2<false>(u(lane, k), u(lane, k + 1), tau, v2);
+      M[hi * ALD + r] = (tri && r == hi) ? cadd(p, sh) : p;
+    };
+    if (nw <= 16) {  // both at once, on half a warp each
+      const int r = lane & 15;
+      const bool tri = lane < 16;
+      if (tri ? r <= hi : (U != nullptr && r < nw)) chain(tri ? T : U, r, tri);
+    } else {
+      if (lane <= hi) chain(T, lane, true);
+      if (U != nullptr && lane < nw) chain(U, lane, false);
     }
   }
   __syncwarp();
@@ -449,33 +465,23 @@ __device__ bool small_schur_warp(cplx* T, cplx* U, int nw, int lane, double smln
 __device__ void schur_swap_warp(cplx* T, cplx* U, int nw, int k, int lane) {
   auto t = [&](int r, int c) -> cplx& { return T[c * ALD + r]; };
   auto u = [&](int r, int c) -> cplx& { return U[c * ALD + r]; };
-  const cplx t11 = t(k, k), t22 = t(k + 1, k + 1);
-  double cs;
-  cplx sn;
-  givens(t(k, k + 1), csub(t22, t11), &cs, &sn);
-  const cplx snc = cconj(sn);
-  __syncwarp();
+  const cplx t11 = t(k, k), t22 = t(k + 1, k + 1), zero = mk(0.0, 0.0);
   const int j = k + 2 + lane;
-  if (j < nw) {  // rows k, k+1 over columns k+2..nw-1
-    const cplx x = t(k, j), y = t(k + 1, j);
-    t(k, j) = cadd(cscale(x, cs), cmul(sn, y));
-    t(k + 1, j) = csub(cscale(y, cs), cmul(snc, x));
-  }
-  if (lane < k) {  // columns k, k+1 over rows 0..k-1
-    const cplx x = t(lane, k), y = t(lane, k + 1);
-    t(lane, k) = cadd(cscale(x, cs), cmul(snc, y));
-    t(lane, k + 1) = csub(cscale(y, cs), cmul(sn, x));
-  }
-  if (lane < nw) {
-    const cplx x = u(lane, k), y = u(lane, k + 1);
-    u(lane, k) = cadd(cscale(x, cs), cmul(snc, y));
-    u(lane, k + 1) = csub(cscale(y, cs), cmul(sn, x));
-  }
+  const bool row = j < nw, col = lane < k, uu = lane < nw;
+  cplx a0 = zero, a1 = zero, b0 = zero, b1 = zero, u0 = zero, u1 = zero;
+  if (row) a0 = t(k, j), a1 = t(k + 1, j);       // rows k, k+1 over columns k+2..nw-1
+  if (col) b0 = t(lane, k), b1 = t(lane, k + 1);  // columns k, k+1 over rows 0..k-1
+  if (uu) u0 = u(lane, k), u1 = u(lane, k + 1);
+  const Rot g = givens(t(k, k + 1), csub(t22, t11));
+  rotate2<true>(a0, a1, g.c, g.s);
+  rotate2<false>(b0, b1, g.c, g.s);
+  rotate2<false>(u0, u1, g.c, g.s);
   __syncwarp();
-  if (lane == 0) {
-    t(k, k) = t22;
-    t(k + 1, k + 1) = t11;
-  }
+  if (row) t(k, j) = a0, t(k + 1, j) = a1;
+  if (col) t(lane, k) = b0, t(lane, k + 1) = b1;
+  if (uu) u(lane, k) = u0, u(lane, k + 1) = u1;
+  if (lane == 0) t(k, k) = t22;
+  if (lane == 1) t(k + 1, k + 1) = t11;
   __syncwarp();
 }
 
@@ -571,18 +577,17 @@ __device__ int aed_deflate_warp(cplx* T, cplx* U, cplx* v, cplx* ev, int nw, cpl
   return ns;
 }
 
-// MINB: resident CTAs per SM the registers are sized for; with three the
-// carry chains prefetch two entries instead of four (no spills either way).
+// MINB: resident CTAs per SM the registers are sized for.
 template <int MINB>
 __global__ void __launch_bounds__(QR_THREADS, MINB)
     hqr_kernel(cplx* const* __restrict__ Hs, void* const* __restrict__ logs, cplx* const* __restrict__ Ws, int n,
                int sweep_cap, long long rot_cap, int* __restrict__ status, int aed_min, int aed_w) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* D = reinterpret_cast<cplx*>(smem_raw);  // [QD][QLD] column-major window
-  cplx* s_tau = D + QD * QLD;                   // [NBMAX][QB]
-  cplx* s_v2 = s_tau + NBMAX * QB;              // [NBMAX][QB]
+  cplx* s_s = D + QR_D;                                       // [QB][NBMAX] rotations: s
+  double* s_c = reinterpret_cast<double*>(s_s + NBMAX * QB);  // [QB][NBMAX] and c
   __shared__ cplx s_shift[NBMAX];
-  __shared__ cplx s_small[NBMAX * NBMAX];
+  __shared__ cplx s_small[NBMAX * ALD];
   __shared__ int s_red[QR_THREADS / 32];
   __shared__ int s_l, s_nb, s_nsw, s_nrot, s_over, s_nround, s_cur;
   // deflation window: reflector vector, undeflated eigenvalues, outcome
@@ -629,27 +634,9 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
       // Deflation search: largest k in (l, i] with a negligible H[k][k-1].
       int best = l;
       for (int k = l + 1 + tid; k <= i; k += QR_THREADS) {
-        const cplx sub = h(k, k - 1);
-        bool small = false;
-        const double cs = cabs1(sub);
-        if (cs <= smlnum) {
-          small = true;
-        } else {
-          const cplx dkm = h(k - 1, k - 1), dk = h(k, k);
-          double tst = cabs1(dkm) + cabs1(dk);
-          if (tst == 0.0) {
-            if (k - 2 >= 0) tst += fabs(h(k - 1, k - 2).x);
-            if (k + 1 <= n - 1) tst += fabs(h(k + 1, k).x);
-          }
-          if (cs <= EIG_ULP * tst) {
-            const double a1 = cs, a2 = cabs1(h(k - 1, k));
-            const double ab = fmax(a1, a2), ba = fmin(a1, a2);
-            const double b1 = cabs1(dk), b2 = cabs1(csub(dkm, dk));
-            const double aa = fmax(b1, b2), bb = fmin(b1, b2);
-            const double s = aa + ab;
-            if (ba * (ab / s) <= fmax(smlnum, EIG_ULP * (bb * (aa / s)))) small = true;
-          }
-        }
+        const bool small =
+            negligible(h(k, k - 1), h(k - 1, k - 1), h(k, k), h(k - 1, k), k >= 2 ? h(k - 1, k - 2) : mk(0.0, 0.0),
+                       k + 1 < n ? h(k + 1, k) : mk(0.0, 0.0), smlnum);
         if (small && k > best) best = k;
       }
 #pragma unroll
@@ -687,7 +674,7 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
         if (warp == 0) {
           int ns = -1;
           const long long c0 = clock64();
-          const bool conv = small_schur_warp(T, U, jw, lane, smlnum);
+          const bool conv = small_schur_warp(T, U, jw, lane, smlnum, s_c, s_s);
           const long long c1 = clock64();
           if (conv) ns = aed_deflate_warp(T, U, s_aedv, s_aedev, jw, s0, lane, smlnum);
           if (lane == 0) {
@@ -777,9 +764,13 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
           const int b0 = i - nb + 1;
           for (int idx = lane; idx < nb * nb; idx += 32) {
             const int c = idx / nb, r = idx - c * nb;
-            s_small[c * nb + r] = (r <= c + 1) ? h(b0 + r, b0 + c) : mk(0.0, 0.0);
+            s_small[c * ALD + r] = (r <= c + 1) ? h(b0 + r, b0 + c) : mk(0.0, 0.0);
           }
-          small_eigvals_warp(s_small, nb, s_shift, lane);
+          __syncwarp();
+          // (on failure to converge the diagonal entries reached are used)
+          small_schur_warp(s_small, nullptr, nb, lane, smlnum, s_c, s_s);
+          __syncwarp();
+          if (lane < nb) s_shift[lane] = s_small[lane * ALD + lane];
         }
         __syncwarp();  // every lane has read s_pend
         if (lane == 0) {
@@ -811,118 +802,161 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
         const int ds = (kmin > m) ? kmin - 1 : m;
         const int de = min(kmax + 2, i);
         const int dn = de - ds + 1;
-        for (int idx = tid; idx < dn * dn; idx += QR_THREADS) {
-          const int c = idx / dn, r = idx - c * dn;
-          D[c * QLD + r] = h(ds + r, ds + c);
+        for (int c = warp; c < dn; c += QR_THREADS / 32) {
+          const cplx* hc = &h(ds, ds + c);
+          for (int r = lane; r < dn; r += 32) D[c * QLD + r] = hc[r];
         }
         __syncthreads();
         if (s_over) break;
-        auto dd = [&](int r, int c) -> cplx& { return D[(c - ds) * QLD + (r - ds)]; };
-        auto reflect = [&](int r) {
-          const int k = m + r - 3 * a;
-          if (lane == 0 && mine && !(k >= m && k <= i - 1)) {  // outside the window: the identity
-            s_tau[a * QB + (r - r0)] = mk(0.0, 0.0);
-            s_v2[a * QB + (r - r0)] = mk(0.0, 0.0);
-          }
-          if (lane == 0 && mine && k >= m && k <= i - 1) {
-            cplx x, y, beta, tau, v2;
-            if (k == m) {
-              x = csub(dd(m, m), s_shift[a]);
-              y = dd(m + 1, m);
-            } else {
-              x = dd(k, k - 1);
-              y = dd(k + 1, k - 1);
-            }
-            refl2(x, y, &beta, &tau, &v2);
-            if (k > m) {
-              dd(k, k - 1) = beta;
-              dd(k + 1, k - 1) = mk(0.0, 0.0);
-            }
-            s_tau[a * QB + (r - r0)] = tau;
-            s_v2[a * QB + (r - r0)] = v2;
-          }
-        };
-        reflect(r0);
-        __syncthreads();
-        for (int r = r0; r < r1; ++r) {
-          const int k = m + r - 3 * a;
+        // A round in three steps, each ended by a CTA barrier: lane b of warp
+        // 0 forms bulge b's rotation (while every warp fetches the rows it
+        // will transform); each warp transforms its bulge's rows k, k+1 over
+        // columns k..de; each warp transforms columns k, k+1 over rows
+        // ds..min(k+2, i).  Both spans are at most QD, two entries per lane.
+        const int kr0 = m + r0 - 3 * a;
+        cplx* prow = D + (ptrdiff_t)(kr0 - ds) * (QLD + 1) + (ptrdiff_t)lane * QLD;
+        cplx* pcol = D + (ptrdiff_t)(kr0 - ds) * QLD + lane;
+        for (int r = r0; r < r1; ++r, prow += QLD + 1, pcol += QLD) {
+          const int k = m + r - 3 * a, u = r - r0;
           const bool act = mine && k >= m && k <= i - 1;
-          if (act) {
-            const cplx tau = s_tau[a * QB + (r - r0)], v2 = s_v2[a * QB + (r - r0)];
-            // row transform of rows k, k+1 over columns k..de
-            {
-              const cplx tauc = cconj(tau), v2c = cconj(v2);
-              for (int j = k + lane; j <= de; j += 32) {
-                const cplx x = dd(k, j), y = dd(k + 1, j);
-                const cplx s = cmul(tauc, cadd(x, cmul(v2c, y)));
-                dd(k, j) = csub(x, s);
-                dd(k + 1, j) = csub(y, cmul(s, v2));
-              }
-            }
-            __syncwarp();
-            // the leading bulges' column transforms on rows k, k+1: bulge
-            // b = a - 1 - lane acts on columns kb, kb + 1, kb = k + 3 (a - b)
-            {
-              const int b = a - 1 - lane, kb = k + 3 * (lane + 1);
-              if (b >= 0 && kb <= i - 1) {
-                const cplx tb = s_tau[b * QB + (r - r0)], vb = s_v2[b * QB + (r - r0)], vbc = cconj(vb);
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                  const cplx p = dd(k + q, kb), w = dd(k + q, kb + 1);
-                  const cplx s = cmul(tb, cadd(p, cmul(vb, w)));
-                  dd(k + q, kb) = csub(p, s);
-                  dd(k + q, kb + 1) = csub(w, cmul(s, vbc));
-                }
-              }
-            }
-            // column transform of columns k, k+1 over rows ds..min(k+2, i),
-            // except the rows of the trailing bulges (bulge a + q on rows
-            // k - 3q, k - 3q + 1), which their own warps transform
-            {
-              const cplx v2c = cconj(v2);
-              const int re = min(k + 2, i);
-              for (int rr = ds + lane; rr <= re; rr += 32) {
-                const int dk = k - rr, q = (dk + 1) / 3;
-                if (dk >= 2 && dk % 3 != 1 && a + q < nb && k - 3 * q >= m) continue;
-                const cplx p = dd(rr, k), w = dd(rr, k + 1);
-                const cplx s = cmul(tau, cadd(p, cmul(v2, w)));
-                dd(rr, k) = csub(p, s);
-                dd(rr, k + 1) = csub(w, cmul(s, v2c));
-              }
-            }
+          const bool row0 = act && lane <= de - k, row1 = act && lane + 32 <= de - k;
+          cplx x0, y0, x1, y1;
+          if (row0) {
+            x0 = prow[0];
+            y0 = prow[1];
           }
-          __syncwarp();
-          if (r + 1 < r1) reflect(r + 1);
+          if (row1) {
+            x1 = prow[32 * QLD];
+            y1 = prow[32 * QLD + 1];
+          }
+          if (tid < nb) {
+            const int kb = m + r - 3 * tid;
+            double c = 1.0;  // outside the window: the identity
+            cplx sn = mk(0.0, 0.0);
+            if (kb >= m && kb <= i - 1) {
+              cplx* pb = D + (ptrdiff_t)(kb - ds) * (QLD + 1);  // (kb, kb)
+              const bool first = kb == m;
+              const cplx x = first ? csub(pb[0], s_shift[tid]) : pb[-QLD];
+              const cplx y = first ? pb[1] : pb[1 - QLD];
+              const Rot g = givens(x, y);
+              if (!first) {
+                pb[-QLD] = g.r;
+                pb[1 - QLD] = mk(0.0, 0.0);
+              }
+              c = g.c;
+              sn = g.s;
+            }
+            s_c[u * NBMAX + tid] = c;
+            s_s[u * NBMAX + tid] = sn;
+          }
+          __syncthreads();
+          const double c = s_c[u * NBMAX + a];
+          const cplx sn = s_s[u * NBMAX + a];
+          if (row0) {
+            rotate2<true>(x0, y0, c, sn);
+            prow[0] = x0;
+            prow[1] = y0;
+          }
+          if (row1) {
+            rotate2<true>(x1, y1, c, sn);
+            prow[32 * QLD] = x1;
+            prow[32 * QLD + 1] = y1;
+          }
+          __syncthreads();
+          const int nc = min(k + 2, i) - ds;
+          const bool col0 = act && lane <= nc, col1 = act && lane + 32 <= nc;
+          if (col0) {
+            x0 = pcol[0];
+            y0 = pcol[QLD];
+          }
+          if (col1) {
+            x1 = pcol[32];
+            y1 = pcol[QLD + 32];
+          }
+          if (col0) {
+            rotate2<false>(x0, y0, c, sn);
+            pcol[0] = x0;
+            pcol[QLD] = y0;
+          }
+          if (col1) {
+            rotate2<false>(x1, y1, c, sn);
+            pcol[32] = x1;
+            pcol[QLD + 32] = y1;
+          }
           __syncthreads();
         }
         if (tid == 0) stamp(2);
         // Write the window back and log this chunk's rotations (round-major).
-        for (int idx = tid; idx < dn * dn; idx += QR_THREADS) {
-          const int c = idx / dn, r = idx - c * dn;
-          h(ds + r, ds + c) = D[c * QLD + r];
+        for (int c = warp; c < dn; c += QR_THREADS / 32) {
+          cplx* hc = &h(ds, ds + c);
+          for (int r = lane; r < dn; r += 32) hc[r] = D[c * QLD + r];
         }
         const int nr = r1 - r0;
         for (int idx = tid; idx < nb * nr; idx += QR_THREADS) {
           const int u = idx / nb, b = idx - u * nb;
           const size_t ri = (size_t)s_cur + (size_t)(r0 + u) * nb + b;
-          const int kk = m + r0 + u - 3 * b;  // slots of bulges outside the window hold the identity
-          const bool on = kk >= m && kk <= i - 1;
-          rot[2 * ri] = on ? s_tau[b * QB + u] : mk(0.0, 0.0);
-          rot[2 * ri + 1] = on ? s_v2[b * QB + u] : mk(0.0, 0.0);
+          rot[2 * ri] = mk(s_c[u * NBMAX + b], 0.0);  // (the identity where the bulge is outside the window)
+          rot[2 * ri + 1] = s_s[u * NBMAX + b];
         }
+        __syncthreads();  // D is free
         // Rest of the active window: columns de+1..i (row transforms) and rows
-        // m..ds-1 (column transforms), one bulge chain at a time, leading
-        // bulge first (the order of every pair of conflicting rotations).
-        const int nright = i - de, nabove = ds - m;
-        for (int task = tid; task < nright + nabove; task += QR_THREADS) {
-          const bool rowop = task < nright;
-          for (int b = 0; b < nb; ++b) {
-            const int ra0 = max(r0, 3 * b), ra1 = min(r1, 3 * b + (i - m));
-            if (ra1 <= ra0) continue;
-            const int k0 = m + ra0 - 3 * b;
-            cplx* p0 = rowop ? H + (size_t)(de + 1 + task) * n + k0 : H + (size_t)k0 * n + (m + task - nright);
-            carry_chain<(MINB >= 3 ? 2 : 4)>(p0, rowop ? 1 : (size_t)n, ra1 - ra0, s_tau + b * QB + (ra0 - r0), s_v2 + b * QB + (ra0 - r0),
-                        rowop);
+        // m..ds-1 (column transforms), FV vectors per warp at a time.
+        {
+          const int cnt = kmax + 2 - kmin;  // entries kmin..kmax+1 of each vector
+          const int nright = i - de, nabove = ds - m;
+          const int gr = (nright + FV - 1) / FV, ng = gr + (nabove + FV - 1) / FV;
+          cplx* buf = D + (size_t)warp * 2 * FV * FE;
+          auto where = [&](int g, cplx*& x, size_t& es, size_t& vs, int& nv) {
+            if (g < gr) {  // columns
+              const int c0 = de + 1 + g * FV;
+              x = H + (size_t)c0 * n + kmin;
+              es = 1;
+              vs = n;
+              nv = min(FV, i + 1 - c0);
+            } else {  // rows
+              const int q0 = m + (g - gr) * FV;
+              x = H + (size_t)kmin * n + q0;
+              es = n;
+              vs = 1;
+              nv = min(FV, ds - q0);
+            }
+          };
+          auto fetch = [&](int g, int half) {
+            cplx* x;
+            size_t es, vs;
+            int nv;
+            where(g, x, es, vs, nv);
+            const int v = lane % FV;
+            if (v < nv)
+              for (int e = lane / FV; e < cnt; e += 32 / FV)
+                cpa16(buf + half * FV * FE + e * FV + v, x + (size_t)e * es + (size_t)v * vs);
+            cpa_commit();
+          };
+          const int b = lane / FV;  // this lane's bulge
+          const int ra0 = max(r0, 3 * b), ra1 = b < nb ? min(r1, 3 * b + (i - m)) : r0;
+          const int off = (m + ra0 - 3 * b - kmin) * FV + lane % FV;
+          if (warp < ng) fetch(warp, 0);
+          for (int g = warp, half = 0; g < ng; g += NBMAX, half ^= 1) {
+            if (g + NBMAX < ng) {
+              fetch(g + NBMAX, half ^ 1);
+              cpa_wait<1>();
+            } else {
+              cpa_wait<0>();
+            }
+            __syncwarp();
+            cplx* vec = buf + half * FV * FE;
+            if (g < gr)
+              strip_rounds<true>(vec + off, r0, r1, ra0, ra1, s_c + b, s_s + b);
+            else
+              strip_rounds<false>(vec + off, r0, r1, ra0, ra1, s_c + b, s_s + b);
+            cplx* x;
+            size_t es, vs;
+            int nv;
+            where(g, x, es, vs, nv);
+            const int v = lane % FV;
+            if (v < nv)
+              for (int e = lane / FV; e < cnt; e += 32 / FV) x[(size_t)e * es + (size_t)v * vs] = vec[e * FV + v];
+            __syncwarp();  // the buffer is free for the group after next
           }
         }
         __syncthreads();
@@ -1032,15 +1066,15 @@ __device__ __forceinline__ void replay_sweeps(cplx* x, size_t stride, int sel, i
           const int u = e / RP_NBG, b = b0 + (e % RP_NBG);
           const bool on = b < nb;
           const cplx* q2 = src + 2 * ((size_t)(t0 + u) * nb + b);
-          s_rot[2 * e] = on ? ld(q2) : mk(0.0, 0.0);
+          s_rot[2 * e] = on ? ld(q2) : mk(1.0, 0.0);
           s_rot[2 * e + 1] = on ? ld(q2 + 1) : mk(0.0, 0.0);
         }
         __syncthreads();
         if (active)
-          ring.run(t0, t0 + nr, [&](int t, int g, cplx& tau, cplx& v2) {
+          ring.run(t0, t0 + nr, [&](int t, int g, double& c, cplx& sn) {
             const cplx* rr = s_rot + 2 * RP_NBG * (t - t0);
-            tau = rr[2 * g];
-            v2 = rr[2 * g + 1];
+            c = rr[2 * g].x;
+            sn = rr[2 * g + 1];
           });
       }
     }
@@ -1085,7 +1119,7 @@ void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* c
                    int* d_status, cudaStream_t st, int parts) {
   if (batch <= 0) return;
   // resident Schur CTAs per SM: 2 (default) or 3 (VRC_QR_CTAS=3); the
-  // arithmetic is the same, only the registers and the prefetch depth differ
+  // arithmetic is the same, only the registers differ
   static const int minb = [] {
     const char* e = std::getenv("VRC_QR_CTAS");
     return (e && std::atoi(e) == 3) ? 3 : 2;
