@@ -438,6 +438,17 @@ size_t Engine::batch_budget_bytes() const {
   return b;
 }
 
+// Items of `per` bytes to take at once.  What fits the budget's lower bound,
+// or the workspace already held, needs no look at the free memory:
+// cudaMemGetInfo is a call into the kernel driver, 64 us on an idle host and
+// far more while other processes allocate, and every stage of a solve asks.
+size_t Engine::batch_chunk(size_t count, size_t per, size_t most, bool in_workspace) const {
+  const size_t take = std::min(count, most);
+  const size_t held = std::max<size_t>((size_t)256 << 20, in_workspace ? ws_cap_ : 0);
+  if (take <= held / per) return std::max<size_t>(1, take);
+  return std::min(most, std::max<size_t>(1, batch_budget_bytes() / per));
+}
+
 // ---------------------------------------------------------------------------
 // Batched primitives
 // ---------------------------------------------------------------------------
@@ -912,9 +923,7 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
     const size_t o_fe33 = o_fe22 + (size_t)m * m;
     const size_t o_pml = o_fe33 + (size_t)m * m;
     const size_t per = (o_pml + (k.pml ? 6 * (size_t)m * m : 0) + 15) / 16 * 16;
-    const size_t budget = batch_budget_bytes();
-    size_t chunk = std::max<size_t>(1, budget / (per * 16));
-    chunk = std::min<size_t>(chunk, 8192);
+    const size_t chunk = batch_chunk(idx.size(), per * 16, 8192, true);
     for (size_t c0 = 0; c0 < idx.size(); c0 += chunk) {
       const size_t B = std::min(chunk, idx.size() - c0);
       cplx* ws = (cplx*)workspace(B * per * 16);
@@ -1161,8 +1170,7 @@ void Engine::eig(std::vector<EigReq>& reqs, int n, std::vector<int>* status) {
   if (reqs.empty()) return;
   const size_t logc = schur_log_bytes(n) / 16;  // rotation log, complex units
   const size_t per = (size_t)3 * n * n + 2 * (size_t)((n + 15) / 16 * 16) + logc;
-  size_t chunk = std::max<size_t>(1, batch_budget_bytes() / (per * 16));
-  chunk = std::min<size_t>(chunk, 16384);
+  const size_t chunk = batch_chunk(reqs.size(), per * 16, 16384, true);
   if (status && status->size() < reqs.size()) status->resize(reqs.size(), 0);
   for (size_t c0 = 0; c0 < reqs.size(); c0 += chunk) {
     const size_t B = std::min(chunk, reqs.size() - c0);
@@ -1344,8 +1352,7 @@ void Engine::segments(std::vector<SegReq>& reqs, int n) {
   if (reqs.empty()) return;
   const size_t nn = (size_t)n * n;
   const size_t per = 6 * nn;
-  size_t chunk = std::max<size_t>(1, batch_budget_bytes() / (per * 16));
-  chunk = std::min<size_t>(chunk, 16384);
+  const size_t chunk = batch_chunk(reqs.size(), per * 16, 16384, true);
   for (size_t c0 = 0; c0 < reqs.size(); c0 += chunk) {
     const size_t B = std::min(chunk, reqs.size() - c0);
     cplx* ws = (cplx*)workspace(B * per * 16);
@@ -1402,8 +1409,7 @@ void Engine::project_left(std::vector<ProjReq>& reqs, int n, std::vector<int>* s
   if (reqs.empty()) return;
   const size_t nn = (size_t)n * n;
   const size_t per = 6 * nn;
-  size_t chunk = std::max<size_t>(1, batch_budget_bytes() / (per * 16));
-  chunk = std::min<size_t>(chunk, 16384);
+  const size_t chunk = batch_chunk(reqs.size(), per * 16, 16384, true);
   if (status && status->size() < reqs.size()) status->resize(reqs.size(), 0);
   for (size_t c0 = 0; c0 < reqs.size(); c0 += chunk) {
     const size_t B = std::min(chunk, reqs.size() - c0);
@@ -1471,8 +1477,7 @@ void Engine::project_right(std::vector<ProjRReq>& reqs, int n, std::vector<int>*
   if (reqs.empty()) return;
   const size_t nn = (size_t)n * n;
   const size_t per = 6 * nn;
-  size_t chunk = std::max<size_t>(1, batch_budget_bytes() / (per * 16));
-  chunk = std::min<size_t>(chunk, 16384);
+  const size_t chunk = batch_chunk(reqs.size(), per * 16, 16384, true);
   if (status && status->size() < reqs.size()) status->resize(reqs.size(), 0);
   for (size_t c0 = 0; c0 < reqs.size(); c0 += chunk) {
     const size_t B = std::min(chunk, reqs.size() - c0);
@@ -1555,8 +1560,7 @@ void Engine::star(std::vector<StarReq>& reqs, int n, std::vector<int>* status) {
   if (reqs.empty()) return;
   const size_t nn = (size_t)n * n;
   const size_t per = 7 * nn;
-  size_t chunk = std::max<size_t>(1, batch_budget_bytes() / (per * 16));
-  chunk = std::min<size_t>(chunk, 16384);
+  const size_t chunk = batch_chunk(reqs.size(), per * 16, 16384, true);
   if (status && status->size() < reqs.size()) status->resize(reqs.size(), 0);
   for (size_t c0 = 0; c0 < reqs.size(); c0 += chunk) {
     const size_t B = std::min(chunk, reqs.size() - c0);
@@ -1658,8 +1662,7 @@ void Engine::rcwa_slabs(std::vector<SlabReq>& reqs, int n, std::vector<int>* sta
   // eigen outputs are pool-allocated per request; temps are pooled too
   if (status && status->size() < reqs.size()) status->resize(reqs.size(), 0);
   const size_t per_bytes = 16 * nn * 16;
-  size_t chunk = std::max<size_t>(1, batch_budget_bytes() / per_bytes);
-  chunk = std::min<size_t>(chunk, 4096);
+  const size_t chunk = batch_chunk(reqs.size(), per_bytes, 4096, false);
   for (size_t c0 = 0; c0 < reqs.size(); c0 += chunk) {
     const size_t B = std::min(chunk, reqs.size() - c0);
     std::vector<EigReq> er(B);
@@ -1737,8 +1740,7 @@ void Engine::diff_slices(std::vector<DiffReq>& reqs, int n, std::vector<int>* st
   if (reqs.empty()) return;
   if (status && status->size() < reqs.size()) status->resize(reqs.size(), 0);
   const size_t nn = (size_t)n * n;
-  size_t chunk = std::max<size_t>(1, batch_budget_bytes() / (24 * nn * 16));
-  chunk = std::min<size_t>(chunk, 4096);
+  const size_t chunk = batch_chunk(reqs.size(), 24 * nn * 16, 4096, false);
   for (size_t c0 = 0; c0 < reqs.size(); c0 += chunk) {
     const size_t B = std::min(chunk, reqs.size() - c0);
     const int NT = 20;

@@ -157,6 +157,7 @@ class Engine {
   // the pools handed out (not returned), summed over the pools
   void pool_report(size_t* held, size_t* out, size_t* npools, size_t* ws) const;
   size_t batch_budget_bytes() const;
+  size_t batch_chunk(size_t count, size_t per, size_t most, bool in_workspace) const;
 
   // batched primitives
   // opA / opB = 1: that operand enters as its conjugate transpose.
