@@ -19,9 +19,8 @@
 // the active window is updated from strips staged in shared memory
 // (strip_rounds).  Rows above the
 // window, columns right of it and all of Z are not touched here: every
-// sweep's rotations are logged round-major and replayed afterwards, whole
-// rounds at a time from a sliding register ring (qr_replay_rows_kernel /
-// qr_replay_cols_kernel).  For
+// sweep's rotations are logged round-major and replayed afterwards
+// (qr_replay_rows_kernel / qr_replay_cols_kernel).  For
 // any entry, eager in-window updates precede deferred column transforms,
 // which precede deferred row transforms (the window's bottom only moves up
 // and windows never straddle a zero subdiagonal), so the replay reproduces
@@ -246,93 +245,6 @@ __device__ __forceinline__ void strip_rounds(cplx* p, int r0, int r1, int ra0, i
     __syncwarp();
   }
 }
-
-// A group of NBG bulges' rotations applied round by round to one vector x
-// (entries x[c * stride]): in round t bulge g acts on the pair
-// (kb + t - 3g, kb + t - 3g + 1).  Entries arrive PFD rounds ahead through
-// 16-byte cp.async copies into this thread's shared-memory slots (THREADS
-// apart), then move into a ring of registers indexed by compile-time slots
-// (round loops are unrolled by the ring size): each round takes in the entry
-// the leading bulge reaches and retires the one the trailing bulge has
-// passed; the group's rotations within a round touch disjoint pairs and run
-// independently.  Entries outside [lo, hi] are neither read nor written.
-template <int NBG, int PFD, bool ROWOP, int THREADS>
-struct RotRing {
-  static constexpr int L = 3 * (NBG - 1);  // retire lag
-  static constexpr int P = L + 3;          // register ring: entries t-L .. t+1
-  static constexpr int S = PFD + 1;        // shared-memory slots per thread
-  cplx w[P];
-  cplx* x;
-  cplx* pf;  // this thread's slot 0; slot q at pf[q * THREADS]
-  size_t stride;
-  int kb, lo, hi, rmin, cnt;
-
-  __device__ __forceinline__ void begin(cplx* x_, size_t stride_, int kb_, int lo_, int hi_, int ng, int cnt_,
-                                        cplx* pf_) {
-    x = x_;
-    pf = pf_;
-    stride = stride_;
-    kb = kb_;
-    lo = lo_;
-    hi = hi_;
-    rmin = -3 * (ng - 1);
-    cnt = cnt_;
-    if (cnt <= 0) return;
-#pragma unroll
-    for (int q = -L; q <= 0; ++q) {
-      const int c = kb + q;
-      w[(q + P) % P] = (q >= rmin && c >= lo && c <= hi) ? x[(size_t)c * stride] : mk(0.0, 0.0);
-    }
-#pragma unroll
-    for (int d = 1; d <= PFD; ++d) {  // one commit group per entry
-      const int c = kb + d;
-      if (c >= lo && c <= hi) cpa16(pf + (d % S) * THREADS, x + (size_t)c * stride);
-      cpa_commit();
-    }
-  }
-
-  // Rounds [t0, t1) (t0 a multiple of P); rot(t, g, c, s) gives bulge g's
-  // rotation of round t, the identity where it is outside the window
-  template <class ROT>
-  __device__ __forceinline__ void run(int t0, int t1, ROT rot) {
-    t1 = min(t1, cnt);
-    for (int tb = t0; tb < t1; tb += P) {
-#pragma unroll
-      for (int tt = 0; tt < P; ++tt) {
-        const int t = tb + tt;
-        if (t < t1) {
-          const int cb = kb + t;
-          cpa_wait<PFD - 1>();  // the group of entry t+1 has landed
-          w[(tt + 1) % P] = (cb + 1 >= lo && cb + 1 <= hi) ? pf[((t + 1) % S) * THREADS] : mk(0.0, 0.0);
-          {
-            const int c = cb + 1 + PFD;  // into the slot of entry t, consumed last round
-            if (c >= lo && c <= hi) cpa16(pf + ((t + 1 + PFD) % S) * THREADS, x + (size_t)c * stride);
-            cpa_commit();
-          }
-#pragma unroll
-          for (int g = 0; g < NBG; ++g) {  // straight-line: inactive pairs carry the identity
-            double rc;
-            cplx rs;
-            rot(t, g, rc, rs);
-            rotate2<ROWOP>(w[(tt - 3 * g + 2 * P) % P], w[(tt - 3 * g + 1 + 2 * P) % P], rc, rs);
-          }
-          {
-            const int q = t - L, c = cb - L;
-            if (q >= rmin && c >= lo && c <= hi) x[(size_t)c * stride] = w[(tt - L + 2 * P) % P];
-          }
-          if (t == cnt - 1) {
-#pragma unroll
-            for (int d = 1; d <= L + 1; ++d) {  // entries t-L+1 .. t+1 still held
-              const int q = t - L + d, c = cb - L + d;
-              if (q >= rmin && c >= lo && c <= hi) x[(size_t)c * stride] = w[(tt - L + d + 2 * P) % P];
-            }
-            cpa_wait<0>();  // no copy may land in the slots after this vector is done
-          }
-        }
-      }
-    }
-  }
-};
 
 // ---------------------------------------------------------------------------
 // Aggressive early deflation (Braman, Byers & Mathias, "The multishift QR
@@ -991,126 +903,174 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
   }
 }
 
-// Replay kernels: one thread per row (column transforms: rows of Z for
-// every sweep, rows of H above the sweep's window) or per column (row
-// transforms: columns of H right of the window).  All threads of a block
-// belong to one matrix, so each sweep's rotations are staged through shared
-// memory in slabs of RS rounds and read as broadcasts.  A thread's entries
-// arrive PFD rounds ahead through 16-byte cp.async copies into its own
-// shared-memory slots (the rounds are short, so register prefetch cannot
-// cover the memory latency), then move into a ring of registers indexed by
-// compile-time slots (round loops are unrolled by the ring size): each round
-// takes in the entry the leading bulge reaches and retires the one the
-// trailing bulge has passed; the group's rotations within a round touch
-// disjoint pairs and run independently.
-constexpr int RP_THREADS = 128;
-constexpr int RP_NBG = 4;  // bulges per register ring
-constexpr int RP_PFD = 7;  // prefetch depth in rounds (ring of PFD + 1 = 8 slots)
+// Replay kernels: every vector (column transforms: rows of Z for every sweep,
+// rows of H above the sweep's window; row transforms: columns of H right of
+// the window) stays in shared memory from the first sweep to the last, FV
+// vectors per warp, and takes the log's rotations with eight lanes per vector
+// as strip_rounds does.  The log is one stream: it comes in through a ring of
+// four chunks, two ahead of the one in use, whatever sweep they belong to.
+//
+// Bounded by the FP64 pipe when several warps share a scheduler, by the
+// latency of a round (some 50 cycles) when the batch is small.  One thread
+// per vector with four bulges in a register ring, its entries streamed from
+// global memory once per four bulges and sweep, took 525 cycles per round and
+// four bulges, and two memory latencies at the start of every sweep.
+constexpr int RG_CHUNK = 128, RG_CHUNKS = 4;            // rotations per chunk, chunks of the ring
+constexpr int RG_SLOTS = RG_CHUNK * RG_CHUNKS;          // a power of two
+constexpr int RG_DENSE = 16;  // deflation-window blocks up to this order are read from the ring (two chunks at most)
+constexpr int RP_MAXW = 4;    // warps per block, at most
 
-constexpr int RS = 4 * RotRing<RP_NBG, RP_PFD, false, RP_THREADS>::P;  // rounds per slab (a multiple of the ring size)
-// staged rotations of a slab, or one deflation-window block (AW x AW)
-constexpr int RP_ROT = RS * NBMAX * 2 > AW * AW ? RS * NBMAX * 2 : AW * AW;
-constexpr size_t RP_SMEM = (size_t)RP_ROT * sizeof(cplx) + (size_t)(RP_PFD + 1) * RP_THREADS * sizeof(cplx);
-
-// A deflation-window block on one vector: x[kw..kw+jw-1] <- U^H x (row
-// transforms, ROWOP) or x U (column transforms); U in shared memory, AW x AW
-// column-major, zero outside jw x jw.
-template <bool ROWOP>
-__device__ __noinline__ void replay_block(cplx* x, size_t stride, int kw, int jw, const cplx* U) {
-  cplx v[AW];
-#pragma unroll
-  for (int k = 0; k < AW; ++k) v[k] = k < jw ? x[(size_t)(kw + k) * stride] : mk(0.0, 0.0);
-  for (int j = 0; j < jw; ++j) {
-    cplx acc = mk(0.0, 0.0);
-#pragma unroll
-    for (int k = 0; k < AW; ++k) {
-      const cplx u = U[j * AW + k];
-      acc = ROWOP ? cadd(acc, cmulc(u, v[k])) : cfma(v[k], u, acc);
-    }
-    x[(size_t)(kw + j) * stride] = acc;
-  }
+// Warps per block: the vectors of a warp take 64 n bytes.  Four warps let two
+// blocks share an SM up to n = 376; three keep two blocks there up to n = 500
+// and still fit one at n = 1024.
+int replay_warps(int n) { return n <= 376 ? RP_MAXW : 3; }
+size_t replay_smem(int n) {
+  return (size_t)RG_SLOTS * 2 * sizeof(cplx) + (size_t)replay_warps(n) * FV * n * sizeof(cplx);
 }
 
+struct LogRing {
+  const cplx* rot;  // the log's rotations (two complex numbers each)
+  cplx* ring;
+  int nrot, cur;  // rotations in the log, the chunk in use
+
+  __device__ __forceinline__ void load(int chunk) {
+    for (int e = threadIdx.x; e < RG_CHUNK * 2; e += blockDim.x)
+      if (chunk * RG_CHUNK + e / 2 < nrot)
+        cpa16(ring + (chunk % RG_CHUNKS) * RG_CHUNK * 2 + e, rot + (size_t)chunk * RG_CHUNK * 2 + e);
+    cpa_commit();
+  }
+  __device__ __forceinline__ void begin() {
+    cur = -1;
+    load(0);
+    load(1);
+  }
+  // every rotation up to `slot` is in the ring (and at least a chunk before
+  // it).  All threads of the block call it alike.
+  __device__ __forceinline__ void ensure(int slot) {
+    while (cur < slot / RG_CHUNK) {
+      ++cur;
+      cpa_wait<1>();    // chunk cur has landed
+      __syncthreads();  // for every thread; chunk cur - 2 is done with
+      load(cur + 2);
+    }
+  }
+};
+
 template <bool ROWOP>
-__device__ __forceinline__ void replay_sweeps(cplx* x, size_t stride, int sel, int idx, const QrSweep* sw,
-                                              int nsweeps, const cplx* rot, cplx* s_rot, cplx* s_pf) {
-  // sel: 0 = every sweep, 1 = sweeps with idx < m (rows of H above the
-  // window), 2 = sweeps with idx > i (columns of H right of the window);
-  // idx < 0 marks a thread without a vector (it still joins the barriers).
-  // Bulges are applied RP_NBG at a time, leading group first, each group
-  // over the whole sweep.
-  for (int s = 0; s < nsweeps; ++s) {
-    const QrSweep q = sw[s];
-    const int nb = q.nb;
-    const bool active = idx >= 0 && (sel == 0 || (sel == 1 && idx < q.m) || (sel == 2 && idx > q.i));
-    const cplx* src = rot + 2 * (size_t)q.start;
-    if (nb < 0) {  // deflation-window block
+__device__ __forceinline__ void replay(cplx* X, size_t es, size_t vs, int sel, int v0, int n, char* logb,
+                                       int sweep_cap, cplx* smem) {
+  // vectors v0 + 4 warp .. of X (entry e of vector v at e es + v vs); sel: 0 =
+  // every sweep, 1 = sweeps with v < m (rows of H above the window), 2 =
+  // sweeps with v > i (columns of H right of the window)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int b = lane / FV, vl = lane % FV, v = v0 + warp * FV + vl;
+  const QrLogHeader hdr = *reinterpret_cast<const QrLogHeader*>(logb);
+  const QrSweep* sw = log_sweeps(logb);
+  LogRing lr{log_rot(logb, sweep_cap), smem, hdr.nrot, -1};
+  cplx* vec = smem + RG_SLOTS * 2 + (size_t)warp * FV * n + vl;
+  lr.begin();
+  if (v < n)
+    for (int e = b; e < n; e += 32 / FV) vec[e * FV] = X[(size_t)e * es + (size_t)v * vs];
+  __syncwarp();
+  QrSweep next;
+  if (hdr.nsweeps > 0) next = sw[0];
+  for (int s = 0; s < hdr.nsweeps; ++s) {
+    const QrSweep q = next;
+    if (s + 1 < hdr.nsweeps) next = sw[s + 1];
+    const bool mine = v < n && (sel == 0 || (sel == 1 ? v < q.m : v > q.i));
+    const bool any = __any_sync(0xffffffffu, mine);
+    if (q.nb < 0) {  // deflation-window block: x <- U^H x (row transforms) or x U
       const int jw = q.R;
-      __syncthreads();  // the previous slab is consumed
-      for (int e = threadIdx.x; e < AW * AW; e += blockDim.x) {
-        const int c = e / AW, r = e - c * AW;
-        s_rot[e] = (r < jw && c < jw) ? ld(src + (size_t)c * jw + r) : mk(0.0, 0.0);
+      const bool ringed = jw <= RG_DENSE;
+      if (ringed) lr.ensure(q.start + (jw * jw - 1) / 2);
+      if (any) {
+        cplx out[AW / 8];
+#pragma unroll
+        for (int t = 0; t < AW / 8; ++t) {
+          const int j = b + 8 * t;
+          cplx acc = mk(0.0, 0.0);
+          if (j < jw)
+            for (int k = 0; k < jw; ++k) {
+              const int e = 2 * q.start + j * jw + k;
+              const cplx u = ringed ? lr.ring[e & (2 * RG_SLOTS - 1)] : ld(lr.rot + e);
+              const cplx x = vec[(q.pad0 + k) * FV];
+              acc = ROWOP ? cadd(acc, cmulc(u, x)) : cfma(x, u, acc);
+            }
+          out[t] = acc;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < AW / 8; ++t)
+          if (mine && b + 8 * t < jw) vec[(q.pad0 + b + 8 * t) * FV] = out[t];
+        __syncwarp();
       }
-      __syncthreads();
-      if (active) replay_block<ROWOP>(x, stride, q.pad0, jw, s_rot);
       continue;
     }
-    for (int b0 = 0; b0 < nb; b0 += RP_NBG) {
-      const int ng = min(RP_NBG, nb - b0);
-      RotRing<RP_NBG, RP_PFD, ROWOP, RP_THREADS> ring;
-      if (active) ring.begin(x, stride, q.m - 3 * b0, q.m, q.i, ng, q.R, s_pf + threadIdx.x);
-      for (int t0 = 0; t0 < q.R; t0 += RS) {
-        const int nr = min(RS, q.R - t0);
-        __syncthreads();  // the previous slab is consumed
-        for (int e = threadIdx.x; e < nr * RP_NBG; e += blockDim.x) {
-          const int u = e / RP_NBG, b = b0 + (e % RP_NBG);
-          const bool on = b < nb;
-          const cplx* q2 = src + 2 * ((size_t)(t0 + u) * nb + b);
-          s_rot[2 * e] = on ? ld(q2) : mk(1.0, 0.0);
-          s_rot[2 * e + 1] = on ? ld(q2 + 1) : mk(0.0, 0.0);
+    const int nb = q.nb;
+    const int ra0 = 3 * b, ra1 = (mine && b < nb) ? 3 * b + (q.i - q.m) : 0;
+    cplx* p = vec + (size_t)q.m * FV;
+    cplx x = mk(0.0, 0.0), y = x;
+    for (int t0 = 0; t0 < q.R;) {
+      lr.ensure(q.start + (t0 + 1) * nb - 1);
+      const int t1 = min(q.R, ((lr.cur + 1) * RG_CHUNK - q.start) / nb);  // rounds whose rotations are in the ring
+      if (any) {
+        int slot = q.start + t0 * nb + b;
+        auto rc = [&](int i) { return lr.ring[2 * (i & (RG_SLOTS - 1))].x; };
+        auto rs = [&](int i) { return lr.ring[2 * (i & (RG_SLOTS - 1)) + 1]; };
+        double c = rc(slot);
+        cplx sn = rs(slot);
+        for (int r = t0; r < t1; ++r) {
+          slot += nb;
+          const double cn = rc(slot);  // the next round's (stale past t1, then read again)
+          const cplx sn2 = rs(slot);
+          if (r >= ra0 && r < ra1) {
+            if (r == ra0) {
+              x = p[0];
+              y = p[FV];
+            }
+            const bool more = r + 1 < ra1;
+            cplx nx = mk(0.0, 0.0);
+            if (more) nx = p[2 * FV];
+            rotate2<ROWOP>(x, y, c, sn);
+            p[0] = x;
+            if (!more) p[FV] = y;
+            x = y;
+            y = nx;
+            p += FV;
+          }
+          c = cn;
+          sn = sn2;
+          __syncwarp();
         }
-        __syncthreads();
-        if (active)
-          ring.run(t0, t0 + nr, [&](int t, int g, double& c, cplx& sn) {
-            const cplx* rr = s_rot + 2 * RP_NBG * (t - t0);
-            c = rr[2 * g].x;
-            sn = rr[2 * g + 1];
-          });
       }
+      t0 = t1;
     }
   }
+  cpa_wait<0>();
+  if (v < n)
+    for (int e = b; e < n; e += 32 / FV) X[(size_t)e * es + (size_t)v * vs] = vec[e * FV];
 }
 
-__global__ void __launch_bounds__(RP_THREADS, 4)
+__global__ void __launch_bounds__(RP_MAXW * 32)
     qr_replay_rows_kernel(cplx* const* __restrict__ Hs, cplx* const* __restrict__ Zs,
                           void* const* __restrict__ logs, int n, int sweep_cap, int row_blocks) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx* s_rot = reinterpret_cast<cplx*>(smem_raw);
-  cplx* s_pf = s_rot + RP_ROT;
   const int mat = blockIdx.y;
   const bool isZ = blockIdx.x >= row_blocks;
-  const int r = (isZ ? blockIdx.x - row_blocks : blockIdx.x) * blockDim.x + threadIdx.x;
-  cplx* X = isZ ? Zs[mat] : Hs[mat];
-  char* logb = static_cast<char*>(logs[mat]);
-  const QrLogHeader hdr = *reinterpret_cast<const QrLogHeader*>(logb);
-  replay_sweeps<false>(X + min(r, n - 1), (size_t)n, isZ ? 0 : 1, r < n ? r : -1, log_sweeps(logb), hdr.nsweeps,
-                       log_rot(logb, sweep_cap), s_rot, s_pf);
+  const int per = blockDim.x / 32 * FV;
+  replay<false>(isZ ? Zs[mat] : Hs[mat], (size_t)n, 1, isZ ? 0 : 1,
+                (isZ ? blockIdx.x - row_blocks : blockIdx.x) * per, n, static_cast<char*>(logs[mat]), sweep_cap,
+                reinterpret_cast<cplx*>(smem_raw));
 }
 
 // Runs after qr_replay_rows_kernel: for any entry all column transforms
 // precede all row transforms.
-__global__ void __launch_bounds__(RP_THREADS, 4)
+__global__ void __launch_bounds__(RP_MAXW * 32)
     qr_replay_cols_kernel(cplx* const* __restrict__ Hs, void* const* __restrict__ logs, int n, int sweep_cap) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx* s_rot = reinterpret_cast<cplx*>(smem_raw);
-  cplx* s_pf = s_rot + RP_ROT;
   const int mat = blockIdx.y;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  cplx* H = Hs[mat];
-  char* logb = static_cast<char*>(logs[mat]);
-  const QrLogHeader hdr = *reinterpret_cast<const QrLogHeader*>(logb);
-  replay_sweeps<true>(H + (size_t)min(j, n - 1) * n, 1, 2, j < n ? j : -1, log_sweeps(logb), hdr.nsweeps,
-                      log_rot(logb, sweep_cap), s_rot, s_pf);
+  replay<true>(Hs[mat], 1, (size_t)n, 2, blockIdx.x * (blockDim.x / 32 * FV), n, static_cast<char*>(logs[mat]),
+               sweep_cap, reinterpret_cast<cplx*>(smem_raw));
 }
 
 }  // namespace
@@ -1141,21 +1101,22 @@ void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* c
   }();
   const int aed_min = aed_env >= 0 ? aed_env : (n <= 128 ? 0 : aed_w);
   ensure_smem((const void*)hqr, QR_SMEM);
-  ensure_smem((const void*)qr_replay_rows_kernel, RP_SMEM);
-  ensure_smem((const void*)qr_replay_cols_kernel, RP_SMEM);
+  const size_t rp_smem = replay_smem(n);
+  const int rp_threads = 32 * replay_warps(n);
+  ensure_smem((const void*)qr_replay_rows_kernel, rp_smem);
+  ensure_smem((const void*)qr_replay_cols_kernel, rp_smem);
   const int cc = schur_sweep_cap(n);
   const long long rc = schur_rot_cap(n);
-  const int row_blocks = (n + RP_THREADS - 1) / RP_THREADS;
-  const size_t rp_smem = RP_SMEM;
+  const int row_blocks = (n + rp_threads / 32 * FV - 1) / (rp_threads / 32 * FV);
   for (int b0 = 0; b0 < batch; b0 += 65535) {
     const int nb = min(65535, batch - b0);
     if (parts & SCHUR_ITERATE)
       hqr<<<nb, QR_THREADS, QR_SMEM, st>>>(d_H + b0, d_logs + b0, d_W + b0, n, cc, rc,
                                                   d_status ? d_status + b0 : nullptr, aed_min, aed_w);
     if (parts & SCHUR_REPLAY) {
-      qr_replay_rows_kernel<<<dim3(2 * row_blocks, nb), RP_THREADS, rp_smem, st>>>(d_H + b0, d_Z + b0, d_logs + b0,
+      qr_replay_rows_kernel<<<dim3(2 * row_blocks, nb), rp_threads, rp_smem, st>>>(d_H + b0, d_Z + b0, d_logs + b0,
                                                                                   n, cc, row_blocks);
-      qr_replay_cols_kernel<<<dim3(row_blocks, nb), RP_THREADS, rp_smem, st>>>(d_H + b0, d_logs + b0, n, cc);
+      qr_replay_cols_kernel<<<dim3(row_blocks, nb), rp_threads, rp_smem, st>>>(d_H + b0, d_logs + b0, n, cc);
     }
   }
   VRC_CUDA_CHECK(cudaGetLastError());
