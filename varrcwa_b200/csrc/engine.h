@@ -162,12 +162,8 @@ class Engine {
   // batched primitives
   // opA / opB = 1: that operand enters as its conjugate transpose.
   void gemm(std::vector<GemmDesc>& d, int n, cplx alpha, cplx beta, double delta, int opA = 0, int opB = 0);
-  // GEMM tile for order n and operand modes: timed once per shape on scratch
-  // operands (both tiles give identical results) and cached for the whole
-  // process; VRC_GEMM_TILE forces one.  0 from gemm_tile_cached when the
-  // shape was not tuned yet.
-  int gemm_tile(int n, int opA, int opB, size_t batch);
-  int gemm_tile_cached(int n, int opA, int opB) const;
+  // GEMM tile forced by VRC_GEMM_TILE (64 or 32), else 0: the launcher's choice
+  int gemm_tile() const;
   void inverse(const std::vector<cplx*>& mats, int n, std::vector<int>* status);
   void copy(const std::vector<cplx*>& src, const std::vector<cplx*>& dst, int n);
   void axpby(const std::vector<const cplx*>& A, const std::vector<const cplx*>& B, const std::vector<cplx*>& C,

@@ -9,12 +9,10 @@
 // leading dimensions (zgemm_rect_batched: the panel updates of the blocked
 // Hessenberg reduction).  Either operand may be taken as its conjugate
 // transpose (used by the adjoint and the Hessenberg reflectors).  One CTA
-// computes a 64 x 64 complex tile (eight warps of 32 x 16), or a 32 x 32
-// tile (four warps of 16 x 16) for small orders, where 64-wide tiles would
-// mostly compute padding (n = 82: 41% of a 128 x 128 cover is useful, 73% of
-// 96 x 96).  Every output element accumulates over k in the same order with
-// either tile, so the choice does not change results; the engine times both
-// once per shape and keeps the faster.  Operands are staged through shared
+// computes a 32 x 32 complex tile (four warps of 16 x 16), or a 64 x 64 tile
+// (eight warps of 32 x 16) where one is asked for.  Every output element
+// accumulates over k in the same order with either tile, so the choice does
+// not change results (launch() has both times).  Operands are staged through shared
 // memory by 16-byte cp.async copies in a 3-stage pipeline or, for the 64-wide
 // tile with VRC_GEMM_BULK set, by the TMA unit's bulk copies in a 4-stage
 // pipeline (zgemm_bulk_kernel).  The complex product
@@ -470,6 +468,12 @@ void launch_bulk(const GemmDesc* d_descs, int batch, const GemmShape& sh, cplx a
 
 void launch(const GemmDesc* d_descs, int batch, const GemmShape& sh, cplx alpha, cplx beta, double delta,
             cudaStream_t stream, int opA, int opB, int tile) {
+  // The 32-wide tile unless the bulk-staged 64-wide kernel is asked for: it
+  // has four times the CTAs for a small batch and at most as much padding for
+  // a large one.  Device us per launch, 64 / 32 (n, products): (98, 1) 24.5 /
+  // 12.7, (162, 4) 34.5 / 16.0, (162, 128) 220.6 / 222.4, (242, 512) 1928 /
+  // 1874, (450, 1) 80.3 / 38.7, (450, 96) 2529 / 2217, (882, 16) 2580 / 2484.
+  if (tile == 0) tile = bulk_mode() != 0 ? 64 : 32;
   if (tile != 32 && tile != 64) throw StatusError(ST_EINVAL, "GEMM tile must be 32 or 64");
   if (batch <= 0 || sh.M <= 0 || sh.N <= 0) return;
   if (tile == 64 && bulk_mode() != 0) {

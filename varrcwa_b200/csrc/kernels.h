@@ -21,18 +21,19 @@ struct GemmDesc {
   const cplx* cs;   // optional column scale (n)
 };
 // opA / opB = 1 takes that operand as its conjugate transpose (kdim == n).
-// tile: 64 (64 x 64 complex per CTA) or 32 (32 x 32); results are identical.
+// tile: 64 (64 x 64 complex per CTA), 32 (32 x 32) or 0, the launcher's choice;
+// results are identical.
 // throws ST_ETIMEOUT when a bulk-staged GEMM (VRC_GEMM_BULK) gave up waiting
 // for a stage since the last check; call after a stream synchronisation
 void gemm_bulk_check();
 void zgemm_batched(const GemmDesc* d_descs, int batch, int n, cplx alpha, cplx beta, double delta,
-                   cudaStream_t stream, int kdim = -1, int opA = 0, int opB = 0, int tile = 64);  // kdim < 0: n
+                   cudaStream_t stream, int kdim = -1, int opA = 0, int opB = 0, int tile = 0);  // kdim < 0: n
 // Rectangular form: C (M x N, leading dimension ldc) = alpha op(A) op(B)
 // (+ beta Cin, same ldc) with op(A) M x K and op(B) K x N; A is stored M x K
 // (lda) or, with opA, K x M; B is stored K x N (ldb) or, with opB, N x K.
 // The descriptors' rs / cs scale rows (M) / columns (N).
 void zgemm_rect_batched(const GemmDesc* d_descs, int batch, int M, int N, int K, int lda, int ldb, int ldc,
-                        cplx alpha, cplx beta, cudaStream_t stream, int opA = 0, int opB = 0, int tile = 64);
+                        cplx alpha, cplx beta, cudaStream_t stream, int opA = 0, int opB = 0, int tile = 0);
 
 // ---- inverse (in place) -------------------------------------------------------
 int zinv_panel_width(int n);

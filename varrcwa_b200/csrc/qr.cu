@@ -716,8 +716,10 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
         const int dn = de - ds + 1;
         for (int c = warp; c < dn; c += QR_THREADS / 32) {
           const cplx* hc = &h(ds, ds + c);
-          for (int r = lane; r < dn; r += 32) D[c * QLD + r] = hc[r];
+          for (int r = lane; r < dn; r += 32) cpa16(D + c * QLD + r, hc + r);
         }
+        cpa_commit();
+        cpa_wait<0>();
         __syncthreads();
         if (s_over) break;
         // A round in three steps, each ended by a CTA barrier: lane b of warp
