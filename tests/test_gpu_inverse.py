@@ -1,0 +1,48 @@
+"""The blocked inversion at the edges of its panels (16 columns up to n = 512, 8
+above, one or two rows per thread) against the identity, and matrices whose
+pivots lie far from the diagonal.  Residual bound: eps n cond, with room of 50."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from varrcwa_b200.capi import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def _check(ctx, A):
+    X, st = ctx.zinv(A)
+    n = A.shape[-1]
+    assert not np.any(st)
+    for b in range(A.shape[0]):
+        bound = 50 * 2.2e-16 * n * np.linalg.cond(A[b])
+        assert np.abs(A[b] @ X[b] - np.eye(n)).max() < bound
+
+
+@pytest.mark.parametrize("n", [31, 32, 33, 47, 48, 49, 64, 65, 255, 256, 257, 272, 511, 512, 513, 520, 527])
+def test_orders(ctx, n):
+    rng = np.random.default_rng(n)
+    _check(ctx, rng.standard_normal((2, n, n)) + 1j * rng.standard_normal((2, n, n)))
+
+
+@pytest.mark.parametrize("n", [40, 70, 300, 530])
+def test_far_pivots(ctx, n):
+    """A scaled permutation (every pivot off the diagonal), and rows of very
+    different size."""
+    rng = np.random.default_rng(n)
+    P = np.eye(n)[rng.permutation(n)] * rng.uniform(0.5, 2.0, n)[:, None] + 0j
+    G = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    _check(ctx, np.stack([P, P + 1e-3 * G, G * 10.0 ** rng.uniform(-3, 3, n)[:, None]]))
+
+
+@pytest.mark.parametrize("n", [40, 300, 530])
+def test_singular(ctx, n):
+    A = np.ones((2, n, n), dtype=complex)
+    A[1] = np.eye(n)
+    A[1, 5, 5] = 0.0
+    assert list(ctx.zinv(A)[1]) == [4, 4]

@@ -179,329 +179,149 @@ __global__ void __launch_bounds__(INV_THREADS)
 }
 
 // ---------------------------------------------------------------------------
-// Blocked form with the rank-w updates on the tensor cores.  Per panel of w
-// columns: zinv_panel_kernel reduces the panel in shared memory (as above),
-// writes it back, stores the update factor M = Tp - E (n x w) and, for every
-// other column, applies the panel's row interchanges and extracts
-// X = a[k:k+w, :] (w x n, zero in the panel's columns); the batched GEMM then
-// performs a += M X for all columns at once (the panel's columns get + 0).
-// zinv_colswap_kernel finally undoes the row interchanges as column
-// interchanges.  Scratch per matrix: M, X and the pivots.
-constexpr int PANEL_THREADS = 256;
-
-__global__ void __launch_bounds__(PANEL_THREADS)
+// Blocked form with the rank-w updates on the tensor cores.  Rows are never
+// exchanged: step t takes as pivot row p_t the largest entry of column t among
+// the rows not yet used, and the permutation comes out once at the end,
+// inverse(t, p_u) = a(p_t, u).  Per panel of w columns zinv_panel_kernel
+// reduces the panel, stores the update factor M = Tp - E (n x w; E the unit
+// columns at the pivot rows) and extracts the pivot rows of the other columns,
+// X (w x n, zero in the panel's columns); the batched GEMM then performs
+// a += M X for all columns at once.
+//
+// The panel kernel holds a row (or RPT rows) per thread, so the multiplier of
+// a step is the thread's own register and a pivot passes two barriers: the
+// candidates are compared by their upper 32 bits (a pivot within 1e-6 of the
+// largest is as good) with one warp reduction each side of the first, and the
+// pivot row is scaled by the one thread that has it before the second.  Bound
+// by that chain for few matrices and by the FP64 issue of the update for many.
+// With rows split over two threads, exchanges, and every thread reducing the
+// candidates and forming the reciprocal, a pivot took 4,700 cycles at n = 162,
+// the row moves 25,000 cycles per panel and the final column exchanges one
+// global round trip per column; above n = 256 the panel was in shared memory
+// (n = 450: 4.0 ms per inversion of four matrices).
+template <int THREADS, int RPT, int W>
+__global__ void __launch_bounds__(THREADS, 1)
     zinv_panel_kernel(cplx* const* __restrict__ mats, cplx* __restrict__ scratch, size_t per, int n, int k, int w,
-                      int W, int* __restrict__ status) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx* panel = reinterpret_cast<cplx*>(smem_raw);  // [w][n]
-  cplx* fcol = panel + (size_t)w * n;                // [n]
-  int* src = reinterpret_cast<int*>(fcol + n);       // [n]: row r of P a is row src[r] of a
-  int* rows = src + n;                               // [2 W]: rows that move
-  __shared__ PivotCand red[PANEL_THREADS / 32];
-  __shared__ cplx s_inv;
-  __shared__ int s_p, s_bad, s_nrows;
+                      int* __restrict__ status) {
+  __shared__ cplx s_prow[W];
+  __shared__ unsigned s_key[16];
+  __shared__ int s_row[16], s_piv[W], s_bad;
 
   cplx* a = mats[blockIdx.x];
   cplx* M = scratch + (size_t)blockIdx.x * per;  // [w][n] (room for W)
   cplx* X = M + (size_t)n * W;                   // [n][w]: X(s, j) at X[j * w + s]
-  int* piv = reinterpret_cast<int*>(M + 2 * (size_t)n * W);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int nwarps = PANEL_THREADS / 32;
-  if (tid == 0) {
-    s_bad = 0;
-    s_nrows = 0;
-  }
-  for (int c2 = 0; c2 < w; ++c2)
-    for (int i = tid; i < n; i += PANEL_THREADS) panel[c2 * n + i] = a[(size_t)(k + c2) * n + i];
-  for (int i = tid; i < n; i += PANEL_THREADS) src[i] = i;
-  __syncthreads();
-  for (int s = 0; s < w; ++s) {
-    const int r0 = k + s;
-    cplx* col = panel + (size_t)s * n;
-    PivotCand c{-1.0, n};
-    for (int i = r0 + tid; i < n; i += PANEL_THREADS) {
-      const double v = cabs1(col[i]);
-      if (v > c.v) {
-        c.v = v;
-        c.i = i;
-      }
-    }
-    c = warp_argmax(c);
-    if (lane == 0) red[warp] = c;
-    __syncthreads();
-    if (warp == 0) {
-      PivotCand cc = lane < nwarps ? red[lane] : PivotCand{-1.0, n};
-      cc = warp_argmax(cc);
-      if (lane == 0) {
-        int p = cc.i;
-        cplx pv = col[p < n ? p : r0];
-        if (!(cc.v > 0.0) || !isfinite(cc.v)) {
-          s_bad = 1;
-          pv = mk(1.0, 0.0);
-          p = r0;
-        }
-        s_p = p;
-        s_inv = cinv(pv);
-        piv[r0] = p;
-        const int t = src[r0];
-        src[r0] = src[p];
-        src[p] = t;
-      }
-    }
-    __syncthreads();
-    const int p = s_p;
-    const cplx ip = s_inv;
-    if (p != r0 && tid < w) {
-      const cplx t = panel[tid * n + r0];
-      panel[tid * n + r0] = panel[tid * n + p];
-      panel[tid * n + p] = t;
-    }
-    __syncthreads();
-    // multipliers, then the scaled pivot row (fcol[r0] is never used)
-    for (int i = tid; i < n; i += PANEL_THREADS) fcol[i] = col[i];
-    if (tid < w) panel[tid * n + r0] = cmul(tid == s ? mk(1.0, 0.0) : panel[tid * n + r0], ip);
-    __syncthreads();
-    for (int c2 = 0; c2 < w; ++c2) {
-      const cplx prow = panel[c2 * n + r0];
-      cplx* pc = panel + (size_t)c2 * n;
-      for (int i = tid; i < n; i += PANEL_THREADS) {
-        if (i == r0) continue;
-        const cplx v = (c2 == s) ? mk(0.0, 0.0) : pc[i];
-        pc[i] = csub(v, cmul(fcol[i], prow));
-      }
-    }
-    __syncthreads();
-  }
-  for (int c2 = 0; c2 < w; ++c2)
-    for (int i = tid; i < n; i += PANEL_THREADS) {
-      const cplx v = panel[c2 * n + i];
-      a[(size_t)(k + c2) * n + i] = v;
-      M[(size_t)c2 * n + i] = (i == k + c2) ? mk(v.x - 1.0, v.y) : v;
-    }
-  // rows moved by the panel's interchanges (at most 2w)
-  for (int i = tid; i < n; i += PANEL_THREADS)
-    if (src[i] != i) rows[atomicAdd(&s_nrows, 1)] = i;
-  __syncthreads();
-  const int nrows = s_nrows;
-  // other columns: permute the moved rows, staged through the panel's shared
-  // memory (all reads of a group of columns before any write; a warp per
-  // column, a lane per moved row), then x_s = (P a)[k+s]
-  const int cw = max(1, (int)((size_t)w * n / max(nrows, 1)));  // columns per group
-  for (int g0 = 0; g0 < n && nrows > 0; g0 += cw) {
-    const int g1 = min(n, g0 + cw);
-    for (int j = g0 + warp; j < g1; j += nwarps) {
-      if (j >= k && j < k + w) continue;
-      for (int q = lane; q < nrows; q += 32) panel[(size_t)(j - g0) * nrows + q] = a[(size_t)j * n + src[rows[q]]];
-    }
-    __syncthreads();
-    for (int j = g0 + warp; j < g1; j += nwarps) {
-      if (j >= k && j < k + w) continue;
-      for (int q = lane; q < nrows; q += 32) a[(size_t)j * n + rows[q]] = panel[(size_t)(j - g0) * nrows + q];
-    }
-    __syncthreads();
-  }
-  for (int j = warp; j < n; j += nwarps) {
-    const bool pc = j >= k && j < k + w;
-    for (int s2 = lane; s2 < w; s2 += 32) X[(size_t)j * w + s2] = pc ? mk(0.0, 0.0) : a[(size_t)j * n + k + s2];
-  }
-  if (tid == 0 && status && s_bad) status[blockIdx.x] = ST_ESINGULAR;
-}
+  int* piv = reinterpret_cast<int*>(M + 2 * (size_t)n * W);  // [n]: pivot row of each column
+  int* used = piv + n;                                       // [n]: rows that have been pivots
+  const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nth >> 5;
 
-// The same panel step with the panel held in registers (n <= 256): thread
-// (h, i) of 512 keeps row i of panel columns [16h, 16h+16); per pivot only
-// the pivot candidates, the exchanged rows, the multipliers and the scaled
-// pivot row pass through shared memory.
-constexpr int RPN_THREADS = 512;
-constexpr int RPN_STAGE = 32 * 1024;  // bytes for the row moves of the other columns
-
-__global__ void __launch_bounds__(RPN_THREADS, 1)
-    zinv_panel_reg_kernel(cplx* const* __restrict__ mats, cplx* __restrict__ scratch, size_t per, int n, int k,
-                          int w, int W, int* __restrict__ status) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx* stage = reinterpret_cast<cplx*>(smem_raw);                 // [RPN_STAGE bytes]
-  int* src = reinterpret_cast<int*>(smem_raw + RPN_STAGE);         // [256]
-  int* rows = src + 256;                                           // [64]
-  __shared__ PivotCand red[8];
-  __shared__ cplx prow[32];
-  __shared__ cplx fcol[256];
-  __shared__ int s_bad, s_nrows;
-
-  cplx* a = mats[blockIdx.x];
-  cplx* M = scratch + (size_t)blockIdx.x * per;
-  cplx* X = M + (size_t)n * W;
-  int* piv = reinterpret_cast<int*>(M + 2 * (size_t)n * W);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int h = tid >> 8, i = tid & 255;
-  const bool row = i < n;
-
-#ifdef ZP_TIMING
-  long long zt0 = clock64(), zt1 = 0, zt2 = 0, zt3 = 0, zt4 = 0, zs[4] = {0, 0, 0, 0};
-#endif
-  cplx r[16];
+  cplx r[RPT][W];
+  bool open[RPT];
+  int step[RPT];  // the step of this panel whose pivot the row was
 #pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    const int gc = 16 * h + c;
-    r[c] = (row && gc < w) ? a[(size_t)(k + gc) * n + i] : mk(0.0, 0.0);
-  }
-  for (int q = tid; q < n; q += RPN_THREADS) src[q] = q;
-  if (tid == 0) {
-    s_bad = 0;
-    s_nrows = 0;
-  }
-  // Rows stay in their threads; the interchanges only relabel them: lpos is
-  // the row index this thread's row has after the interchanges so far.
-  int lpos = i;
-  __syncthreads();
-#ifdef ZP_TIMING
-  zt1 = clock64();
-#endif
-  // the step loop is not unrolled (its body is large); a thread's entry of
-  // column s is picked from the register row by an unrolled select
-  auto pick = [&](int cs) {
-    cplx v = r[0];
+  for (int q = 0; q < RPT; ++q) {
+    const int i = tid + q * nth;
+    step[q] = -1;
+    open[q] = i < n && (k == 0 || used[i] == 0);
 #pragma unroll
-    for (int c = 1; c < 16; ++c)
-      if (c == cs) v = r[c];
-    return v;
-  };
-#pragma unroll 1
-  for (int s = 0; s < 32; ++s) {
+    for (int c = 0; c < W; ++c) r[q][c] = (i < n && c < w) ? a[(size_t)(k + c) * n + i] : mk(0.0, 0.0);
+  }
+  if (tid == 0) s_bad = 0;
+#pragma unroll
+  for (int s = 0; s < W; ++s) {
     if (s < w) {
-      const int r0 = k + s;
-      const int hs = s >> 4, cs = s & 15;
-      if (h == hs) {
-        PivotCand c{-1.0, n};
-        if (row && lpos >= r0) {
-          c.v = cabs1(pick(cs));
-          c.i = lpos;
+      unsigned key = 0;  // rows that may be pivots have keys from 1 up
+      int row = 0;
+#pragma unroll
+      for (int q = 0; q < RPT; ++q)
+        if (open[q]) {
+          const unsigned kq = max(1u, (unsigned)__double2hiint(cabs1(r[q][s])));
+          if (kq > key) {
+            key = kq;
+            row = tid + q * nth;
+          }
         }
-        c = warp_argmax(c);
-        if (lane == 0) red[warp & 7] = c;
+      const unsigned wmax = __reduce_max_sync(0xffffffffu, key);
+      const unsigned eq = __ballot_sync(0xffffffffu, key == wmax);
+      if (lane == __ffs(eq) - 1) {
+        s_key[warp] = key;
+        s_row[warp] = row;
       }
-#ifdef ZP_TIMING
-      long long ta = clock64();
-#endif
       __syncthreads();
-#ifdef ZP_TIMING
-      long long tb = clock64();
-      zs[0] += tb - ta;
-#endif
-      // every thread reduces the eight candidates itself (same order, same result)
-      PivotCand cc = red[0];
+      const unsigned kw = lane < nwarps ? s_key[lane] : 0u;
+      const unsigned top = __reduce_max_sync(0xffffffffu, kw);
+      const int p = s_row[__ffs(__ballot_sync(0xffffffffu, kw == top)) - 1];
+      const bool bad = top <= 1u || top >= 0x7ff00000u;
 #pragma unroll
-      for (int q = 1; q < 8; ++q) {
-        const PivotCand o = red[q];
-        if (o.v > cc.v || (o.v == cc.v && o.i < cc.i)) cc = o;
-      }
-      const bool bad = !(cc.v > 0.0) || !isfinite(cc.v) || cc.i >= n;
-      const int p = bad ? r0 : cc.i;
-      if (tid == 0) {
-        if (bad) s_bad = 1;
-        piv[r0] = p;
-        const int t = src[r0];
-        src[r0] = src[p];
-        src[p] = t;
-      }
-      if (lpos == p) lpos = r0;
-      else if (lpos == r0) lpos = p;
-      // the pivot row (now labelled r0) and the multipliers of column s
-      const bool prow_thread = row && lpos == r0;
-      if (prow_thread) {
+      for (int q = 0; q < RPT; ++q)
+        if (p == tid + q * nth) {
+          const cplx ip = bad ? mk(1.0, 0.0) : cinv_fast(r[q][s]);
 #pragma unroll
-        for (int c = 0; c < 16; ++c) prow[16 * h + c] = r[c];
-      }
-      if (h == hs && row) fcol[i] = pick(cs);
-#ifdef ZP_TIMING
-      long long tc = clock64();
-      zs[1] += tc - tb;
-#endif
+          for (int c = 0; c < W; ++c) {
+            r[q][c] = c == s ? ip : cmul(r[q][c], ip);
+            s_prow[c] = r[q][c];
+          }
+          step[q] = s;
+          open[q] = false;
+          s_piv[s] = p;
+          if (bad) s_bad = 1;
+        }
       __syncthreads();
-#ifdef ZP_TIMING
-      long long td = clock64();
-      zs[2] += td - tc;
-#endif
-      const cplx ip = bad ? mk(1.0, 0.0) : cinv_fast(prow[s]);
-      if (prow_thread) {
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          const int gc = 16 * h + c;
-          r[c] = cmul(gc == s ? mk(1.0, 0.0) : r[c], ip);
-        }
-      } else if (row) {
-        const cplx f = cmul(fcol[i], ip);
+      for (int q = 0; q < RPT; ++q)
+        if (step[q] != s) {
+          const cplx f = mk(-r[q][s].x, -r[q][s].y);
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          const int gc = 16 * h + c;
-          // column s: -a(i, s) / pivot; others: a(i, c) - a(i, s) / pivot * a(r0, c)
-          if (gc < w) r[c] = (gc == s) ? cneg(f) : csub(r[c], cmul(f, prow[gc]));
+          for (int c = 0; c < W; ++c) r[q][c] = c == s ? cmul(f, s_prow[c]) : cfma(f, s_prow[c], r[q][c]);
         }
-      }
-#ifdef ZP_TIMING
-      zs[3] += clock64() - td;
-#endif
     }
   }
 #pragma unroll
-  for (int c = 0; c < 16; ++c) {
-    const int gc = 16 * h + c;
-    if (row && gc < w) {
-      const cplx v = r[c];
-      a[(size_t)(k + gc) * n + lpos] = v;
-      M[(size_t)gc * n + lpos] = (lpos == k + gc) ? mk(v.x - 1.0, v.y) : v;
+  for (int q = 0; q < RPT; ++q) {
+    const int i = tid + q * nth;
+    if (i < n) {
+#pragma unroll
+      for (int c = 0; c < W; ++c)
+        if (c < w) {
+          const cplx v = r[q][c];
+          a[(size_t)(k + c) * n + i] = v;
+          M[(size_t)c * n + i] = step[q] == c ? mk(v.x - 1.0, v.y) : v;
+        }
+      if (k == 0 || step[q] >= 0) used[i] = step[q] >= 0 ? 1 : 0;
     }
   }
-#ifdef ZP_TIMING
-  zt2 = clock64();
-#endif
-  for (int q = tid; q < n; q += RPN_THREADS)
-    if (src[q] != q) rows[atomicAdd(&s_nrows, 1)] = q;
   __syncthreads();
-  const int nrows = s_nrows;
-  constexpr int nwarps = RPN_THREADS / 32;
-  const int cw = max(1, (int)(RPN_STAGE / 16 / max(nrows, 1)));
-  for (int g0 = 0; g0 < n && nrows > 0; g0 += cw) {
-    const int g1 = min(n, g0 + cw);
-    for (int j = g0 + warp; j < g1; j += nwarps) {
-      if (j >= k && j < k + w) continue;
-      for (int q = lane; q < nrows; q += 32) stage[(size_t)(j - g0) * nrows + q] = a[(size_t)j * n + src[rows[q]]];
-    }
-    __syncthreads();
-    for (int j = g0 + warp; j < g1; j += nwarps) {
-      if (j >= k && j < k + w) continue;
-      for (int q = lane; q < nrows; q += 32) a[(size_t)j * n + rows[q]] = stage[(size_t)(j - g0) * nrows + q];
-    }
-    __syncthreads();
-  }
-#ifdef ZP_TIMING
-  zt3 = clock64();
-#endif
-  for (int j = warp; j < n; j += nwarps) {
-    const bool pc = j >= k && j < k + w;
-    for (int s2 = lane; s2 < w; s2 += 32) X[(size_t)j * w + s2] = pc ? mk(0.0, 0.0) : a[(size_t)j * n + k + s2];
+  if (tid < w) piv[k + tid] = s_piv[tid];
+  for (int e = tid; e < n * w; e += nth) {
+    const int j = e / w, s = e - j * w;
+    X[e] = (j >= k && j < k + w) ? mk(0.0, 0.0) : a[(size_t)j * n + s_piv[s]];
   }
   if (tid == 0 && status && s_bad) status[blockIdx.x] = ST_ESINGULAR;
-#ifdef ZP_TIMING
-  __syncthreads();
-  zt4 = clock64();
-  if (tid == 0 && blockIdx.x == 0)
-    printf("zp k=%d load %lld pivots %lld [sync1 %lld reduce %lld sync2 %lld elim %lld] permute %lld extract %lld\n", k,
-           zt1 - zt0, zt2 - zt1, zs[0], zs[1], zs[2], zs[3], zt3 - zt2, zt4 - zt3);
-#endif
 }
 
-__global__ void __launch_bounds__(256)
-    zinv_colswap_kernel(cplx* const* __restrict__ mats, const cplx* __restrict__ scratch, size_t per, int n, int w) {
-  cplx* a = mats[blockIdx.x];
-  const int* piv = reinterpret_cast<const int*>(scratch + (size_t)blockIdx.x * per + 2 * (size_t)n * w);
-  for (int k = n - 1; k >= 0; --k) {
-    const int p = piv[k];
-    if (p != k)
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const cplx t = a[(size_t)k * n + i];
-        a[(size_t)k * n + i] = a[(size_t)p * n + i];
-        a[(size_t)p * n + i] = t;
-      }
+// The permutation at the end, in two passes that are each in place within a
+// block's shared memory: entry t of a column is its entry p_t (four columns
+// per block), then column u becomes column p_u (four rows per block).
+constexpr int PERM_THREADS = 128;
+template <bool COLS>
+__global__ void __launch_bounds__(PERM_THREADS)
+    zinv_permute_kernel(cplx* const* __restrict__ mats, const cplx* __restrict__ scratch, size_t per, int n, int W) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx* buf = reinterpret_cast<cplx*>(smem_raw);  // [4 n]
+  cplx* a = mats[blockIdx.y];
+  const int* piv = reinterpret_cast<const int*>(scratch + (size_t)blockIdx.y * per + 2 * (size_t)n * W);
+  const int v0 = blockIdx.x * 4, nv = min(4, n - v0), tid = threadIdx.x;
+  if (COLS) {
+    const int v = tid & 3;
+    if (v < nv)
+      for (int e = tid >> 2; e < n; e += PERM_THREADS / 4) buf[e * 4 + v] = a[(size_t)e * n + v0 + v];
     __syncthreads();
+    if (v < nv)
+      for (int e = tid >> 2; e < n; e += PERM_THREADS / 4) a[(size_t)piv[e] * n + v0 + v] = buf[e * 4 + v];
+  } else {
+    for (int e = tid; e < nv * n; e += PERM_THREADS) buf[e] = a[(size_t)v0 * n + e];
+    __syncthreads();
+    for (int v = 0; v < nv; ++v)
+      for (int e = tid; e < n; e += PERM_THREADS) a[(size_t)(v0 + v) * n + e] = buf[v * n + piv[e]];
   }
 }
 
@@ -514,45 +334,44 @@ int zinv_panel_width(int n) {
   return nb;
 }
 
-int zinv_blocked_width(int n) {
-  int w = 32;
-  while (w > 4 && ((size_t)(w + 1) * n * 16 + (size_t)n * 4 + 2 * w * 4 > 200 * 1024)) w >>= 1;
-  return w;
-}
+// Panel columns: what a thread's registers hold with a row per thread up to
+// n = 512 and two above (512 threads, 128 registers each).
+int zinv_blocked_width(int n) { return n <= 512 ? 16 : 8; }
 
 size_t zinv_blocked_scratch(int n) {
   const int w = zinv_blocked_width(n);
-  return (2 * (size_t)n * w + ((size_t)n * 4 + 15) / 16) * 16;  // M, X, pivots
+  return (2 * (size_t)n * w + (2 * (size_t)n * 4 + 15) / 16) * 16;  // M, X, pivots, used rows
 }
 
 void zinv_blocked_batched(cplx* const* d_mats, int batch, int n, int* d_status, void* scratch,
                           const GemmDesc* d_descs, cudaStream_t stream) {
   if (batch <= 0) return;
+  if (n > 1024) throw StatusError(ST_EINVAL, "blocked inversion: n <= 1024");
   const int W = zinv_blocked_width(n);
   const size_t per = zinv_blocked_scratch(n) / 16;
-  const size_t smem = (size_t)(W + 1) * n * 16 + (size_t)n * 4 + 2 * W * 4;
-  ensure_smem((const void*)zinv_panel_kernel, smem);
-  // registers hold the panel when every row has a thread of each half
-  const bool use_reg = n <= 256 && W == 32 && !std::getenv("VRC_ZINV_SMEM_PANEL");
-  const size_t reg_smem = RPN_STAGE + (256 + 64) * sizeof(int);
-  if (use_reg) ensure_smem((const void*)zinv_panel_reg_kernel, reg_smem);
+  const size_t psm = (size_t)4 * n * sizeof(cplx);
+  ensure_smem((const void*)zinv_permute_kernel<false>, psm);
+  ensure_smem((const void*)zinv_permute_kernel<true>, psm);
   cplx* scr = static_cast<cplx*>(scratch);
   for (int b0 = 0; b0 < batch; b0 += 65535) {
     const int nb = min(65535, batch - b0);
+    cplx* sb = scr + (size_t)b0 * per;
     for (int k = 0; k < n; k += W) {
       const int w = min(W, n - k);
-      if (use_reg)
-        zinv_panel_reg_kernel<<<nb, RPN_THREADS, reg_smem, stream>>>(
-            d_mats + b0, scr + (size_t)b0 * per, per, n, k, w, W, d_status ? d_status + b0 : nullptr);
-      else
-        zinv_panel_kernel<<<nb, PANEL_THREADS, smem, stream>>>(d_mats + b0, scr + (size_t)b0 * per, per, n, k, w, W,
-                                                               d_status ? d_status + b0 : nullptr);
+      int* st = d_status ? d_status + b0 : nullptr;
+      const int threads = (n <= 512 ? n + 31 : (n + 1) / 2 + 31) / 32 * 32;
+      auto panel = n <= 256   ? zinv_panel_kernel<256, 1, 16>
+                   : n <= 512 ? zinv_panel_kernel<512, 1, 16>
+                              : zinv_panel_kernel<512, 2, 8>;
+      panel<<<nb, threads, 0, stream>>>(d_mats + b0, sb, per, n, k, w, st);
       VRC_CUDA_CHECK(cudaGetLastError());
       // descriptor b: A = M (n x w, leading dimension n), B = X (w x n,
       // leading dimension w) at M + n W, C = Cin = the matrix
       zgemm_batched(d_descs + b0, nb, n, mk(1.0, 0.0), mk(1.0, 0.0), 0.0, stream, w);
     }
-    zinv_colswap_kernel<<<nb, 256, 0, stream>>>(d_mats + b0, scr + (size_t)b0 * per, per, n, W);
+    const dim3 grid((n + 3) / 4, nb);
+    zinv_permute_kernel<false><<<grid, PERM_THREADS, psm, stream>>>(d_mats + b0, sb, per, n, W);
+    zinv_permute_kernel<true><<<grid, PERM_THREADS, psm, stream>>>(d_mats + b0, sb, per, n, W);
   }
   VRC_CUDA_CHECK(cudaGetLastError());
 }
