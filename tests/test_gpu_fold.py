@@ -1,0 +1,97 @@
+"""Order powers of mirror-symmetric cells through their parity classes against
+the general way (VRC_NO_FOLD), to 1e-9 of the largest power as the other
+order-power tests: every method, both sides, odd and equal harmonic counts,
+single-row truncations, lossy media, odd rasters, mixed calls; same statuses
+and the same trees (rectangular lattices: no degenerate modes)."""
+import numpy as np
+import pytest
+
+from varrcwa_b200 import structures as st
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from varrcwa_b200.capi import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def _pillar(seed, nx, ny, npx=64, npy=64, **kw):
+    d = st.pillar_cell(seed, norders=3, npix=npx, lam=0.55)
+    d.update(nx=nx, ny=ny, npy=npy, Lx=0.41, Ly=0.46, **kw)
+    return d
+
+
+def _both(ctx, monkeypatch, cells, **kw):
+    monkeypatch.delenv("VRC_NO_FOLD", raising=False)
+    a = ctx.order_powers(cells, **kw)
+    ta = [ctx.tree(c) for c in range(len(cells))]
+    monkeypatch.setenv("VRC_NO_FOLD", "1")
+    b = ctx.order_powers(cells, **kw)
+    tb = [ctx.tree(c) for c in range(len(cells))]
+    for c in range(len(cells)):
+        assert a[c]["status"] == b[c]["status"] == 0
+        for k in ("R", "T"):
+            assert np.abs(a[c][k] - b[c][k]).max() <= 1e-9 * max(b[c]["R"].max(), b[c]["T"].max())
+        assert [(x[0], x[1], x[3]) for x in ta[c]] == [(x[0], x[1], x[3]) for x in tb[c]]
+    return a
+
+
+@pytest.mark.parametrize("nx,ny", [(3, 3), (9, 1), (1, 9), (5, 3), (3, 7), (7, 5), (9, 9)])
+@pytest.mark.parametrize("side", [0, 1])
+def test_adaptive(ctx, monkeypatch, nx, ny, side):
+    _both(ctx, monkeypatch, [_pillar(7, nx, ny)], method="redheffer", pe=1e-2, side=side)
+
+
+@pytest.mark.parametrize("method", ["rcwa", "differential"])
+@pytest.mark.parametrize("nx,ny", [(5, 3), (7, 7)])
+def test_fixed_slices(ctx, monkeypatch, method, nx, ny):
+    n = 4 if method == "rcwa" else 16
+    for flux in (True, False):
+        _both(ctx, monkeypatch, [_pillar(8, nx, ny, z1=0.1)], method=method, nslices=n, side=1, flux_norm=flux)
+
+
+def test_lossy_and_odd_rasters(ctx, monkeypatch):
+    _both(ctx, monkeypatch, [_pillar(9, 7, 5, npx=33, npy=64, eps_in=5.8 + 0.4j),
+                             _pillar(10, 5, 7, npx=64, npy=31, eps_out=1.7 + 0.01j)], method="redheffer", pe=1e-2)
+
+
+def test_mixed_call(ctx, monkeypatch):
+    """Pillars of several truncations beside a grid cell, over the lanes."""
+    g = dict(kind="grid", lam=1.3, nx=5, ny=3, pml=False, x=np.array([0.0, 0.13, 0.41, 1.0]),
+             y=np.array([0.0, 0.3, 0.8]), eps=np.array([[2.0, 9.0, 2.0], [2.0, 2.0, 2.0]], dtype=complex),
+             z0=0.0, z1=0.3, end0=2.085, end1=1.0)
+    cells = [_pillar(20, 3, 3), g, _pillar(21, 5, 5), _pillar(22, 1, 1), _pillar(23, 7, 3), g, _pillar(24, 5, 3)]
+    _both(ctx, monkeypatch, cells, method="redheffer", pe=1e-2)
+
+
+def test_energy(ctx):
+    a = ctx.order_powers([_pillar(11, 9, 7)], method="rcwa", nslices=6)[0]
+    assert np.abs(a["R"].sum(1) + a["T"].sum(1) - 1.0).max() < 1e-10
+
+
+@pytest.mark.parametrize("ends", [True, False])
+@pytest.mark.parametrize("call", ["redheffer", "rcwa", "differential"])
+@pytest.mark.parametrize("nx,ny", [(5, 3), (1, 9), (7, 7)])
+def test_blocks(ctx, monkeypatch, call, ends, nx, ny):
+    """Blocks in the full-order end modes: the same modes in the same order,
+    the blocks to 1e-9 of their largest entry in the Fourier basis."""
+    from tests.conftest import fourier_blocks
+    ds = [_pillar(31, nx, ny, z1=0.12), _pillar(32, nx, ny, z1=0.15)]
+    if not ends:
+        for d in ds:
+            d["end0"] = d["end1"] = None
+    out = []
+    for env in (None, "1"):
+        monkeypatch.delenv("VRC_NO_FOLD", raising=False) if env is None else monkeypatch.setenv("VRC_NO_FOLD", env)
+        out.append(ctx.redheffer(ds, pe=1e-2) if call == "redheffer" else getattr(ctx, call)(ds, 8))
+    for a, b in zip(*out):
+        for k in ("status", "n", "N", "n_eig", "n_samples", "n_nodes"):
+            assert a[k] == b[k], k
+        assert np.array_equal(a["gam0"], b["gam0"]) and np.array_equal(a["W1"], b["W1"])
+        F, G = fourier_blocks(a), fourier_blocks(b)
+        for k in F:
+            assert np.abs(F[k] - G[k]).max() <= 1e-9 * max(np.abs(G[k]).max(), 1e-3), k

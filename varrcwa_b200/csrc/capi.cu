@@ -557,7 +557,7 @@ int vrc_redheffer(vrc_context* ctx, int ncells, const vrc_cell* cells, double pe
                   std::vector<vrc::CellResult>& r) {
                 vrc::Engine::RedhefferOpts lo = o;
                 lo.rotate = g;
-                E.redheffer(sp, lo, r);
+                E.solve_cells(sp, 0, lo, 0, r);
               });
     tm.done();
     export_results(ctx, res, owner, results);
@@ -616,7 +616,7 @@ int vrc_redheffer_forward(vrc_context* ctx, int ncells, const vrc_cell* cells, d
                   std::vector<vrc::CellResult>& r) {
                 vrc::Engine::RedhefferOpts lo = o;
                 lo.rotate = g;
-                E.redheffer(sp, lo, r);
+                E.solve_cells(sp, 0, lo, 0, r);
               });
     tm.done();
     export_results(ctx, res, owner, results, &ctx->grad_ends);
@@ -757,7 +757,7 @@ int vrc_rcwa(vrc_context* ctx, int ncells, const vrc_cell* cells, int N, vrc_res
     Timed tm(ctx);
     run_lanes(ctx, specs, res, owner,
               [&](int, vrc::Engine& E, const std::vector<vrc::CellSpec>& sp, const std::vector<int>&,
-                  std::vector<vrc::CellResult>& r) { E.rcwa(sp, N, r); });
+                  std::vector<vrc::CellResult>& r) { E.solve_cells(sp, 1, {}, N, r); });
     tm.done();
     export_results(ctx, res, owner, results);
   });
@@ -771,7 +771,7 @@ int vrc_differential(vrc_context* ctx, int ncells, const vrc_cell* cells, int N,
     Timed tm(ctx);
     run_lanes(ctx, specs, res, owner,
               [&](int, vrc::Engine& E, const std::vector<vrc::CellSpec>& sp, const std::vector<int>&,
-                  std::vector<vrc::CellResult>& r) { E.differential(sp, N, r); });
+                  std::vector<vrc::CellResult>& r) { E.solve_cells(sp, 2, {}, N, r); });
     tm.done();
     export_results(ctx, res, owner, results);
   });
@@ -791,19 +791,12 @@ int vrc_order_powers(vrc_context* ctx, int ncells, const vrc_cell* cells, int me
     run_lanes(ctx, specs, res, owner,
               [&](int g, vrc::Engine& E, const std::vector<vrc::CellSpec>& sp, const std::vector<int>& ids,
                   std::vector<vrc::CellResult>& r) {
-                if (method == 0) {
-                  vrc::Engine::RedhefferOpts o;
-                  o.pe = pe;
-                  o.max_depth = max_depth;
-                  o.rotate = g;
-                  E.redheffer(sp, o, r);
-                } else if (method == 1) {
-                  E.rcwa(sp, nslices, r);
-                } else {
-                  E.differential(sp, nslices, r);
-                }
+                vrc::Engine::RedhefferOpts o;
+                o.pe = pe;
+                o.max_depth = max_depth;
+                o.rotate = g;
                 std::vector<std::vector<double>> lr, lt;
-                E.order_powers(sp, r, side, flux_norm, lr, lt);
+                E.solve_powers(sp, method, o, nslices, side, flux_norm, r, lr, lt);
                 for (size_t k = 0; k < ids.size(); ++k) {
                   Rv[ids[k]] = std::move(lr[k]);
                   Tv[ids[k]] = std::move(lt[k]);

@@ -85,6 +85,7 @@ enum {
   ST_ETIMEOUT = 7,
   ST_EDEPTH = 8,
   ST_ENODEV = 9,
+  ST_ASYMMETRIC = 64,  // internal: a raster without the mirror planes its cell promised
 };
 
 }  // namespace vrc

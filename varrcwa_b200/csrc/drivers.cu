@@ -17,7 +17,9 @@
 #include <algorithm>
 #include <cmath>
 #include <list>
+#include <cstdlib>
 #include <map>
+#include <tuple>
 
 namespace vrc {
 
@@ -54,6 +56,9 @@ struct Book {
   std::vector<int> pend_samples, pend_refs;
   std::vector<int> cell_status;
   std::vector<CellResult>* out;
+  // cells come four at a time, the parity classes of one mirror-symmetric
+  // cell: n is the folded order, a sample is assembled once for all four
+  bool folded = false;
 
   Book(Engine& e, int n_, const std::vector<CellSpec>& c, std::vector<Engine::CellDev*>& cd)
       : E(e), n(n_), cells(c), cds(cd) {}
@@ -86,18 +91,77 @@ struct Book {
       R[r].W = R[r].V = R[r].Winv = R[r].Vinv = R[r].gam = nullptr;
     }
   }
-  // Assemble all pending samples and decompose all pending references.
-  void flush() {
-    std::vector<Engine::SampleReq> sr;
+  // Folded samples: each distinct (structure, medium, z) is assembled at full
+  // order and every class that asked for it gets its part.
+  void flush_folded() {
+    std::map<std::tuple<int, bool, double>, std::vector<int>> want;
     for (int s : pend_samples) {
       const SampleB& b = S[s];
-      sr.push_back({&cells[b.cell], cds[b.cell], b.z, b.homog, b.eps_h, b.P, b.Q});
+      want[{b.cell / 4, b.homog, b.z}].push_back(s);
       (*out)[b.cell].n_samples++;
     }
+    std::vector<std::vector<int>> groups;
+    for (auto& kv : want) {  // same z, other half-space medium: a group of its own
+      std::vector<std::vector<int>> part;
+      for (int s : kv.second) {
+        bool put = false;
+        for (auto& p : part)
+          if (S[p[0]].eps_h.x == S[s].eps_h.x && S[p[0]].eps_h.y == S[s].eps_h.y) {
+            p.push_back(s);
+            put = true;
+            break;
+          }
+        if (!put) part.push_back({s});
+      }
+      for (auto& p : part) groups.push_back(std::move(p));
+    }
+    for (size_t g0 = 0; g0 < groups.size();) {
+      const int nf = cells[S[groups[g0][0]].cell].n();  // one full order per call of a driver
+      const size_t most = std::max<size_t>(1, ((size_t)512 << 20) / (32 * (size_t)nf * nf));
+      const size_t g1 = std::min(groups.size(), g0 + most);
+      std::vector<Engine::SampleReq> sr;
+      for (size_t g = g0; g < g1; ++g) {
+        const SampleB& b = S[groups[g][0]];
+        sr.push_back({&cells[b.cell], cds[b.cell], b.z, b.homog, b.eps_h, E.mat(nf), E.mat(nf), nullptr, !b.homog});
+      }
+      std::vector<int> st;
+      E.assemble(sr, &st);
+      std::map<std::pair<int, int>, std::vector<FoldDesc>> fd;  // by harmonic counts
+      for (size_t g = g0; g < g1; ++g)
+        for (int s : groups[g]) {
+          const SampleB& b = S[s];
+          const CellSpec& c = cells[b.cell];
+          fd[{c.nx, c.ny}].push_back({sr[g - g0].P, sr[g - g0].Q, b.P, b.Q, c.k0() * c.k0(), b.cell % 4});
+          if (st[g - g0]) cell_status[b.cell] = st[g - g0];
+        }
+      for (auto& kv : fd) {
+        const FoldDesc* d = E.upload(kv.second);
+        Engine::Prof pr(E, "assembly", 0.0, 160.0 * n * (double)n * kv.second.size());
+        fold_batched(d, (int)kv.second.size(), kv.first.first, kv.first.second, E.stream());
+      }
+      for (auto& r : sr) {
+        E.free_mat(r.P, nf);
+        E.free_mat(r.Q, nf);
+      }
+      g0 = g1;
+    }
+  }
+  // Assemble all pending samples and decompose all pending references.
+  void flush() {
     std::vector<int> st;
-    E.assemble(sr, &st);
-    for (size_t i = 0; i < st.size(); ++i)
-      if (st[i]) cell_status[S[pend_samples[i]].cell] = st[i];
+    if (folded) {
+      flush_folded();
+    } else {
+      std::vector<Engine::SampleReq> sr;
+      for (int s : pend_samples) {
+        const SampleB& b = S[s];
+        sr.push_back({&cells[b.cell], cds[b.cell], b.z, b.homog, b.eps_h, b.P, b.Q});
+        (*out)[b.cell].n_samples++;
+      }
+      E.assemble(sr, &st);
+      for (size_t i = 0; i < st.size(); ++i)
+        if (st[i]) cell_status[S[pend_samples[i]].cell] = st[i];
+    }
     std::vector<Engine::EigReq> er;
     for (int r : pend_refs) {
       const RefB& b = R[r];
@@ -132,6 +196,26 @@ struct Book {
 void start_results(const std::vector<CellSpec>& cells, std::vector<CellResult>& out) {
   out.assign(cells.size(), CellResult());
   for (size_t c = 0; c < cells.size(); ++c) out[c].n = cells[c].n();
+}
+
+// Order of the problems solved for cells of order n.
+int solved_order(int n, int folded) { return folded ? (n / 2 + 1) / 2 : n; }
+
+// Cells whose S-matrix is wanted.  FOLD_EXCITED: the classes that a normally
+// incident plane wave excites, (even, even) by x polarisation and (odd, odd) by
+// y polarisation.
+bool excited(int c, int folded) { return folded != Engine::FOLD_EXCITED || c % 4 == 0 || c % 4 == 3; }
+
+// The four classes of a cell share its CellDev.
+std::vector<Engine::CellDev*> prepare_cells(Engine& E, const std::vector<CellSpec>& cells, int folded) {
+  std::vector<Engine::CellDev*> cds;
+  for (size_t c = 0; c < cells.size(); ++c)
+    cds.push_back(folded && c % 4 ? cds.back() : E.prepare_cell(cells[c]));
+  return cds;
+}
+void release_cells(Engine& E, const std::vector<Engine::CellDev*>& cds, int folded) {
+  for (size_t c = 0; c < cds.size(); ++c)
+    if (!folded || c % 4 == 0) E.release_cell(cds[c]);
 }
 
 void validate(const CellSpec& c) {
@@ -186,6 +270,7 @@ void Engine::release_result(CellResult& r) {
 // Adaptive varRCWA
 // ---------------------------------------------------------------------------
 void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& o, std::vector<CellResult>& out) {
+  const int folded = o.folded;
   for (const auto& c : cells) validate(c);
   start_results(cells, out);
   std::map<int, std::vector<int>> by_n;
@@ -194,16 +279,16 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
   if (!classes.empty())
     std::rotate(classes.begin(), classes.begin() + (size_t)std::max(0, o.rotate) % classes.size(), classes.end());
   for (auto& kv : classes) {
-    const int n = kv.first;
+    const int n = solved_order(kv.first, folded);
     const std::vector<int>& ids = kv.second;
     std::vector<CellSpec> sub;
     for (int c : ids) sub.push_back(cells[c]);
-    std::vector<CellDev*> cds;
-    for (auto& c : sub) cds.push_back(prepare_cell(c));
+    std::vector<CellDev*> cds = prepare_cells(*this, sub, folded);
     std::vector<CellResult> res(sub.size());
     for (size_t c = 0; c < sub.size(); ++c) res[c].n = n;
     Book bk(*this, n, sub, cds);
     bk.out = &res;
+    bk.folded = folded != 0;
     bk.cell_status.assign(sub.size(), ST_OK);
     const int C = (int)sub.size();
     std::vector<NodeB> N;
@@ -269,6 +354,15 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
       VRC_CUDA_CHECK(cudaMemcpyAsync(herr.data(), derr, herr.size() * sizeof(double), cudaMemcpyDeviceToHost, stream_));
       sync();
       free_bytes(derr, active.size() * sizeof(double));
+      if (folded) {  // a node's error is the largest of its four classes
+        std::map<std::pair<int, double>, double> worst;
+        for (size_t i = 0; i < active.size(); ++i) {
+          const NodeB& nd = N[active[i]];
+          auto it = worst.emplace(std::make_pair(nd.cell / 4, nd.a), herr[i]).first;
+          if (!(herr[i] <= it->second) && !std::isnan(it->second)) it->second = herr[i];
+        }
+        for (size_t i = 0; i < active.size(); ++i) herr[i] = worst[{N[active[i]].cell / 4, N[active[i]].a}];
+      }
       std::vector<int> next;
       for (size_t i = 0; i < active.size(); ++i) {
         const int id = active[i];
@@ -333,6 +427,14 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
     std::vector<ProjReq> pr;
     std::vector<int> pr_cell;
     for (int c = 0; c < C; ++c) {
+      if (!excited(c, folded)) {  // only its errors were needed
+        for (int id : order[c]) {
+          free_mat(N[id].tdd, n); free_mat(N[id].tuu, n); free_mat(N[id].rud, n); free_mat(N[id].rdu, n);
+          bk.release_ref(N[id].ref);
+        }
+        order[c].clear();
+        continue;
+      }
       int prev = e0[c];
       for (int id : order[c]) {
         const NodeB& nd = N[id];
@@ -349,6 +451,7 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
     std::vector<std::vector<SBlocks>> lists(C);
     std::vector<int> last(C);
     for (int c = 0; c < C; ++c) {
+      if (order[c].empty()) continue;
       for (int id : order[c]) lists[c].push_back({N[id].tdd, N[id].tuu, N[id].rud, N[id].rdu});
       last[c] = N[order[c].back()].ref;
       for (int id : order[c])
@@ -356,23 +459,29 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
     }
     star_reduce(lists, n, &bk.cell_status);
     std::vector<ProjRReq> rr;
+    std::vector<int> rr_cell;
     for (int c = 0; c < C; ++c) {
+      if (lists[c].empty()) continue;
+      rr_cell.push_back(c);
       const SBlocks& s = lists[c][0];
       rr.push_back({bk.R[last[c]].Winv, bk.R[last[c]].Vinv, bk.R[e1[c]].W, bk.R[e1[c]].V, s.tdd, s.tuu, s.rud, s.rdu});
     }
     std::vector<int> rst;
     project_right(rr, n, &rst);
     sync();
+    for (size_t i = 0; i < rst.size(); ++i)
+      if (rst[i]) bk.cell_status[rr_cell[i]] = rst[i];
     for (int c = 0; c < C; ++c) {
-      if (rst.size() > (size_t)c && rst[c]) bk.cell_status[c] = rst[c];
       // release the remaining holds of the last leaf's reference
       for (int id : order[c])
         if (N[id].ref == last[c]) bk.release_ref(last[c]);
       CellResult& r = res[c];
-      r.Tdd = lists[c][0].tdd;
-      r.Tuu = lists[c][0].tuu;
-      r.Rud = lists[c][0].rud;
-      r.Rdu = lists[c][0].rdu;
+      if (!lists[c].empty()) {
+        r.Tdd = lists[c][0].tdd;
+        r.Tuu = lists[c][0].tuu;
+        r.Rud = lists[c][0].rud;
+        r.Rdu = lists[c][0].rdu;
+      }
       bk.export_basis(e0[c], r.W0, r.V0, r.gam0, r.W0inv);
       bk.export_basis(e1[c], r.W1, r.V1, r.gam1, r.W1inv);
       r.status = bk.cell_status[c];
@@ -383,7 +492,7 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
         free_mat(bk.S[s].P, n);
         free_mat(bk.S[s].Q, n);
       }
-    for (auto* cd : cds) release_cell(cd);
+    release_cells(*this, cds, folded);
     for (size_t c = 0; c < ids.size(); ++c) out[ids[c]] = res[c];
   }
 }
@@ -392,28 +501,29 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
 // Plain RCWA: N midpoint slices (RCWAIntegrator::compute,
 // src/core/RCWAIntegrator.cpp:20-87).
 // ---------------------------------------------------------------------------
-void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellResult>& out) {
+void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellResult>& out, int folded) {
   if (Nsl < 1) throw StatusError(ST_EINVAL, "N must be >= 1");
   for (const auto& c : cells) validate(c);
   start_results(cells, out);
   std::map<int, std::vector<int>> by_n;
   for (size_t c = 0; c < cells.size(); ++c) by_n[cells[c].n()].push_back((int)c);
   for (auto& kv : by_n) {
-    const int n = kv.first;
+    const int n = solved_order(kv.first, folded);
     const std::vector<int>& ids = kv.second;
     std::vector<CellSpec> sub;
     for (int c : ids) sub.push_back(cells[c]);
-    std::vector<CellDev*> cds;
-    for (auto& c : sub) cds.push_back(prepare_cell(c));
+    std::vector<CellDev*> cds = prepare_cells(*this, sub, folded);
     std::vector<CellResult> res(sub.size());
     for (auto& r : res) r.n = n;
     Book bk(*this, n, sub, cds);
     bk.out = &res;
+    bk.folded = folded != 0;
     const int C = (int)sub.size();
     bk.cell_status.assign(C, ST_OK);
     std::vector<int> e0(C), e1(C);
     std::vector<std::vector<int>> slices(C);
     for (int c = 0; c < C; ++c) {
+      if (!excited(c, folded)) continue;
       const CellSpec& s = sub[c];
       const int s1 = bk.sample(c, s.z1);
       e1[c] = bk.end_basis(c, s1, s.has_end1, s.eps_end1);
@@ -431,6 +541,7 @@ void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellR
     std::vector<std::vector<SBlocks>> lists(C);
     std::vector<int> sl_cell;
     for (int c = 0; c < C; ++c) {
+      if (!excited(c, folded)) continue;
       const CellSpec& s = sub[c];
       const double dz = (s.z1 - s.z0) / (double)Nsl;
       for (int si : slices[c]) {
@@ -458,16 +569,21 @@ void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellR
       for (int si : slices[c]) bk.release_sample(si);
     star_reduce(lists, n, &bk.cell_status);
     std::vector<ProjLEReq> pl;
+    std::vector<int> pl_cell;
     for (int c = 0; c < C; ++c) {
+      if (lists[c].empty()) continue;
+      pl_cell.push_back(c);
       const SBlocks& s = lists[c][0];
       pl.push_back({bk.R[e1[c]].Winv, bk.R[e1[c]].Vinv, bk.R[e0[c]].W, bk.R[e0[c]].V, s.tdd, s.tuu, s.rud, s.rdu});
     }
     std::vector<int> pst;
     project_left_end(pl, n, &pst);
     sync();
+    for (size_t i = 0; i < pst.size(); ++i)
+      if (pst[i]) bk.cell_status[pl_cell[i]] = pst[i];
     for (int c = 0; c < C; ++c) {
-      if (pst.size() > (size_t)c && pst[c]) bk.cell_status[c] = pst[c];
       CellResult& r = res[c];
+      if (lists[c].empty()) continue;
       r.Tdd = lists[c][0].tdd; r.Tuu = lists[c][0].tuu; r.Rud = lists[c][0].rud; r.Rdu = lists[c][0].rdu;
       bk.export_basis(e0[c], r.W0, r.V0, r.gam0, r.W0inv);
       bk.export_basis(e1[c], r.W1, r.V1, r.gam1, r.W1inv);
@@ -475,7 +591,7 @@ void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellR
     }
     for (size_t s = 0; s < bk.S.size(); ++s)
       if (bk.S[s].P) { free_mat(bk.S[s].P, n); free_mat(bk.S[s].Q, n); }
-    for (auto* cd : cds) release_cell(cd);
+    release_cells(*this, cds, folded);
     for (size_t c = 0; c < ids.size(); ++c) out[ids[c]] = res[c];
   }
 }
@@ -484,28 +600,29 @@ void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellR
 // Differential method (DifferentialIntegrator::compute,
 // src/core/DifferentialIntegrator.cpp:21-134).
 // ---------------------------------------------------------------------------
-void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellResult>& out) {
+void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellResult>& out, int folded) {
   if (Nsl < 1) throw StatusError(ST_EINVAL, "N must be >= 1");
   for (const auto& c : cells) validate(c);
   start_results(cells, out);
   std::map<int, std::vector<int>> by_n;
   for (size_t c = 0; c < cells.size(); ++c) by_n[cells[c].n()].push_back((int)c);
   for (auto& kv : by_n) {
-    const int n = kv.first;
+    const int n = solved_order(kv.first, folded);
     const std::vector<int>& ids = kv.second;
     std::vector<CellSpec> sub;
     for (int c : ids) sub.push_back(cells[c]);
-    std::vector<CellDev*> cds;
-    for (auto& c : sub) cds.push_back(prepare_cell(c));
+    std::vector<CellDev*> cds = prepare_cells(*this, sub, folded);
     std::vector<CellResult> res(sub.size());
     for (auto& r : res) r.n = n;
     Book bk(*this, n, sub, cds);
     bk.out = &res;
+    bk.folded = folded != 0;
     const int C = (int)sub.size();
     bk.cell_status.assign(C, ST_OK);
     std::vector<int> e0(C), e1(C);
     std::vector<std::vector<int>> pts(C);  // samples at z0, zm_0, zr_0, zm_1, zr_1, ...
     for (int c = 0; c < C; ++c) {
+      if (!excited(c, folded)) continue;
       const CellSpec& s = sub[c];
       const int s1 = bk.sample(c, s.z1);
       e1[c] = bk.end_basis(c, s1, s.has_end1, s.eps_end1);
@@ -530,6 +647,7 @@ void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vect
     std::vector<std::vector<SBlocks>> lists(C);
     std::vector<int> dr_cell;
     for (int c = 0; c < C; ++c) {
+      if (!excited(c, folded)) continue;
       const CellSpec& s = sub[c];
       const double dz = (s.z1 - s.z0) / (double)Nsl;
       const RefB& b1 = bk.R[e1[c]];
@@ -550,16 +668,21 @@ void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vect
       for (int p : pts[c]) bk.release_sample(p);
     star_reduce(lists, n, &bk.cell_status);
     std::vector<ProjLEReq> pl;
+    std::vector<int> pl_cell;
     for (int c = 0; c < C; ++c) {
+      if (lists[c].empty()) continue;
+      pl_cell.push_back(c);
       const SBlocks& s = lists[c][0];
       pl.push_back({bk.R[e1[c]].Winv, bk.R[e1[c]].Vinv, bk.R[e0[c]].W, bk.R[e0[c]].V, s.tdd, s.tuu, s.rud, s.rdu});
     }
     std::vector<int> pst;
     project_left_end(pl, n, &pst);
     sync();
+    for (size_t i = 0; i < pst.size(); ++i)
+      if (pst[i]) bk.cell_status[pl_cell[i]] = pst[i];
     for (int c = 0; c < C; ++c) {
-      if (pst.size() > (size_t)c && pst[c]) bk.cell_status[c] = pst[c];
       CellResult& r = res[c];
+      if (lists[c].empty()) continue;
       r.Tdd = lists[c][0].tdd; r.Tuu = lists[c][0].tuu; r.Rud = lists[c][0].rud; r.Rdu = lists[c][0].rdu;
       bk.export_basis(e0[c], r.W0, r.V0, r.gam0, r.W0inv);
       bk.export_basis(e1[c], r.W1, r.V1, r.gam1, r.W1inv);
@@ -567,7 +690,7 @@ void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vect
     }
     for (size_t s = 0; s < bk.S.size(); ++s)
       if (bk.S[s].P) { free_mat(bk.S[s].P, n); free_mat(bk.S[s].Q, n); }
-    for (auto* cd : cds) release_cell(cd);
+    release_cells(*this, cds, folded);
     for (size_t c = 0; c < ids.size(); ++c) out[ids[c]] = res[c];
   }
 }
@@ -577,7 +700,7 @@ void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vect
 // ---------------------------------------------------------------------------
 void Engine::order_powers(const std::vector<CellSpec>& cells, const std::vector<CellResult>& res, int side,
                           int flux_norm, std::vector<std::vector<double>>& Rout,
-                          std::vector<std::vector<double>>& Tout) {
+                          std::vector<std::vector<double>>& Tout, int folded) {
   const size_t C = cells.size();
   Rout.assign(C, {});
   Tout.assign(C, {});
@@ -597,34 +720,49 @@ void Engine::order_powers(const std::vector<CellSpec>& cells, const std::vector<
     std::vector<MatVecDesc> mv1, mv2;
     std::vector<double*> Rd(2 * B), Td(2 * B);
     std::vector<double*> ab(B);
+    const int ns = solved_order(n, folded);
+    std::vector<cplx*> cls;  // folded: the classes' harmonics
+    std::map<std::pair<int, int>, std::vector<UnfoldDesc>> ud;
     for (size_t b = 0; b < B; ++b) {
       const CellSpec& s = cells[ids[b]];
-      const CellResult& r = res[ids[b]];
       const int nx = s.nx, ny = s.ny;
-      const int c0 = (ny * (nx - 1)) / 2 + (ny - 1) / 2;
-      const cplx* Win = side == 0 ? r.W0 : r.W1;
-      const cplx* Wininv = side == 0 ? r.W0inv : r.W1inv;
-      const cplx* Wout = side == 0 ? r.W1 : r.W0;
-      const cplx* Rm = side == 0 ? r.Rdu : r.Rud;
-      const cplx* Tm = side == 0 ? r.Tuu : r.Tdd;
       for (int p = 0; p < 2; ++p) {
         const size_t k = 2 * b + p;
+        // the class of this polarisation, and its zero order's place there
+        const CellResult& r = folded ? res[4 * ids[b] + (p == 0 ? 0 : 3)] : res[ids[b]];
+        const int c0 = folded ? (p == 0 ? 0 : (nx - 1) / 2 * ((ny - 1) / 2))
+                              : (p == 0 ? 0 : m) + (ny * (nx - 1)) / 2 + (ny - 1) / 2;
+        const cplx* Win = side == 0 ? r.W0 : r.W1;
+        const cplx* Wininv = side == 0 ? r.W0inv : r.W1inv;
+        const cplx* Wout = side == 0 ? r.W1 : r.W0;
+        const cplx* Rm = side == 0 ? r.Rdu : r.Rud;
+        const cplx* Tm = side == 0 ? r.Tuu : r.Tdd;
         // c = Win^-1 s with s the unit vector of the zero order (px or py)
-        cvec[k] = const_cast<cplx*>(Wininv) + (size_t)(p == 0 ? c0 : m + c0) * n;
+        cvec[k] = const_cast<cplx*>(Wininv) + (size_t)c0 * ns;
         rc[k] = vec(n); rf[k] = vec(n); tc[k] = vec(n); tf[k] = vec(n);
+        cplx *rk = rf[k], *tk = tf[k];
+        if (folded) {
+          cls.push_back(rk = vec(n));
+          cls.push_back(tk = vec(n));
+          ud[{nx, ny}].push_back({rk, rf[k], p == 0 ? 0 : 3});
+          ud[{nx, ny}].push_back({tk, tf[k], p == 0 ? 0 : 3});
+        }
         mv1.push_back({Rm, cvec[k], rc[k]});
         mv1.push_back({Tm, cvec[k], tc[k]});
-        mv2.push_back({Win, rc[k], rf[k]});
-        mv2.push_back({Wout, tc[k], tf[k]});
+        mv2.push_back({Win, rc[k], rk});
+        mv2.push_back({Wout, tc[k], tk});
         Rd[k] = (double*)bytes(m * sizeof(double));
         Td[k] = (double*)bytes(m * sizeof(double));
       }
       ab[b] = (double*)bytes(2 * m * sizeof(double));
     }
     {
-      Prof pr(*this, "powers", 16.0 * n * (double)n * (mv1.size() + mv2.size()), 16.0 * n * (double)n * (mv1.size() + mv2.size()), 2);
-      matvec_batched(upload(mv1), (int)mv1.size(), n, stream_);
-      matvec_batched(upload(mv2), (int)mv2.size(), n, stream_);
+      const double work = 16.0 * ns * (double)ns * (mv1.size() + mv2.size());
+      Prof pr(*this, "powers", work, work, 2 + (int)ud.size());
+      matvec_batched(upload(mv1), (int)mv1.size(), ns, stream_);
+      matvec_batched(upload(mv2), (int)mv2.size(), ns, stream_);
+      for (auto& kv : ud)
+        unfold_batched(upload(kv.second), (int)kv.second.size(), kv.first.first, kv.first.second, stream_);
     }
     std::vector<PowerDesc> pd;
     std::vector<std::vector<double>> hab(B);
@@ -672,6 +810,240 @@ void Engine::order_powers(const std::vector<CellSpec>& cells, const std::vector<
       free_bytes(Td[k], m * sizeof(double));
     }
     for (size_t b = 0; b < B; ++b) free_bytes(ab[b], 2 * m * sizeof(double));
+    for (cplx* p : cls) free_vec(p, n);
+  }
+}
+
+// A pillar's raster is its own mirror image along x and y, so its solve splits
+// into four parity classes of a quarter of the order each (fold.cu): an
+// eigen-decomposition costs a sixteenth of the operations.  Every other
+// structure, and a pillar whose raster turns out not to be symmetric (a pixel
+// centre within rounding of the rim), takes the general way.  Below nine
+// harmonics there is nothing to split.  Order powers: one 7 x 7-order pillar
+// 38 -> 12 ms, 16 at 11 x 11 orders 348 -> 72, 16 slices of two at 13 x 9
+// orders 59 -> 9.  On a square lattice the modes of two classes are degenerate
+// in pairs; apart in their classes, the adaptive tree no longer depends on how a
+// solver's rounding mixes them.
+static bool mirror_symmetric(const CellSpec& c) {
+  return c.kind == GEOM_PILLAR && !c.pml && c.m() >= 9 && !std::getenv("VRC_NO_FOLD");
+}
+
+namespace {
+struct Held {  // device blocks of solves, given back also on errors
+  Engine& E;
+  std::vector<CellResult> r;
+  ~Held() {
+    for (auto& x : r) E.release_result(x);
+  }
+};
+// Status of a cell from those of its classes; false: not symmetric after all.
+bool class_status(const std::vector<CellResult>& r, size_t i, int* status) {
+  *status = ST_OK;
+  for (int k = 0; k < 4; ++k) {
+    const int s = r[4 * i + k].status;
+    if (s == ST_ASYMMETRIC) return false;
+    if (s && !*status) *status = s;
+  }
+  return true;
+}
+void copy_counts(CellResult& r, const CellResult& from, int status) {
+  r.status = status;
+  r.N = from.N;
+  r.n_eig = from.n_eig;
+  r.n_samples = from.n_samples;
+  r.n_nodes = from.n_nodes;
+  r.nodes = from.nodes;
+}
+}  // namespace
+
+void Engine::solve(const std::vector<CellSpec>& cells, int method, const RedhefferOpts& o, int nslices,
+                   std::vector<CellResult>& out, int folded) {
+  if (method == 0) {
+    RedhefferOpts ro = o;
+    ro.folded = folded;
+    redheffer(cells, ro, out);
+  } else if (method == 1) {
+    rcwa(cells, nslices, out, folded);
+  } else {
+    differential(cells, nslices, out, folded);
+  }
+}
+
+// The classes' S-matrices in the modes of the full-order end media, which are
+// solved as ever, so that modes keep their order and phases: each class's
+// blocks go over to its Fourier basis (W1 Tuu W0^-1 ...), those add up to the
+// full one, and that goes over to the end modes.
+void Engine::unfold_results(const std::vector<CellSpec>& cells, const std::vector<CellResult>& sub,
+                            const std::vector<int>& pick, std::vector<CellResult>& out) {
+  std::map<std::pair<int, int>, std::vector<int>> by_shape;
+  for (int i : pick) by_shape[{cells[i].nx, cells[i].ny}].push_back(i);
+  for (auto& kv : by_shape) {
+    const int nx = kv.first.first, ny = kv.first.second, n = 2 * nx * ny, d = solved_order(n, FOLD_ALL);
+    const std::vector<int>& ids = kv.second;
+    const size_t B = ids.size();
+    // end media at full order
+    std::vector<CellDev*> cds;
+    std::vector<SampleReq> sr;
+    std::vector<EigReq> er;
+    for (int i : ids) {
+      const CellSpec& s = cells[i];
+      CellResult& r = out[i];
+      r.n = n;
+      cds.push_back(prepare_cell(s));
+      for (cplx** p : {&r.W0, &r.V0, &r.W0inv, &r.W1, &r.V1, &r.W1inv, &r.Tdd, &r.Tuu, &r.Rud, &r.Rdu}) *p = mat(n);
+      r.gam0 = vec(n);
+      r.gam1 = vec(n);
+      for (int e = 0; e < 2; ++e) {
+        const bool has = e ? s.has_end1 : s.has_end0;
+        sr.push_back({&s, cds.back(), has ? s.z0 : (e ? s.z1 : s.z0), has, e ? s.eps_end1 : s.eps_end0, mat(n), mat(n)});
+        er.push_back({sr.back().P, sr.back().Q, e ? r.W1 : r.W0, e ? r.V1 : r.V0, e ? r.W1inv : r.W0inv, nullptr,
+                      e ? r.gam1 : r.gam0});
+      }
+    }
+    std::vector<int> ast, est;
+    assemble(sr, &ast);
+    eig(er, n, &est);
+    for (size_t q = 0; q < 2 * B; ++q) {
+      const int s = q < ast.size() && ast[q] ? ast[q] : (q < est.size() ? est[q] : 0);
+      if (s && !out[ids[q / 2]].status) out[ids[q / 2]].status = s;
+    }
+    for (auto& r : sr) {
+      free_mat(r.P, n);
+      free_mat(r.Q, n);
+    }
+    for (auto* cd : cds) release_cell(cd);
+    // per block (Tdd, Tuu, Rud, Rdu): out-side and in-side ends
+    const int oe[4] = {0, 1, 1, 0}, ie[4] = {1, 0, 1, 0};
+    std::vector<cplx*> tmp, F, T;  // d x d products, n x n Fourier blocks and products
+    std::vector<GemmDesc> g1, g2, h1, h2;
+    std::vector<UnfoldMatDesc> ud;
+    for (size_t b = 0; b < B; ++b) {
+      const CellResult* c = &sub[4 * ids[b]];
+      CellResult& r = out[ids[b]];
+      cplx* const full[4] = {r.Tdd, r.Tuu, r.Rud, r.Rdu};
+      for (int q = 0; q < 4; ++q) {
+        UnfoldMatDesc u;
+        for (int k = 0; k < 4; ++k) {
+          const cplx* blk = q == 0 ? c[k].Tdd : q == 1 ? c[k].Tuu : q == 2 ? c[k].Rud : c[k].Rdu;
+          cplx *t = mat(d), *f = mat(d);
+          tmp.push_back(t);
+          tmp.push_back(f);
+          g1.push_back({oe[q] ? c[k].W1 : c[k].W0, blk, t, nullptr, nullptr, nullptr});
+          g2.push_back({t, ie[q] ? c[k].W1inv : c[k].W0inv, f, nullptr, nullptr, nullptr});
+          u.in[k] = f;
+        }
+        F.push_back(mat(n));
+        T.push_back(mat(n));
+        u.out = F.back();
+        ud.push_back(u);
+        h1.push_back({oe[q] ? r.W1inv : r.W0inv, F.back(), T.back(), nullptr, nullptr, nullptr});
+        h2.push_back({T.back(), ie[q] ? r.W1 : r.W0, full[q], nullptr, nullptr, nullptr});
+      }
+    }
+    gemm(g1, d, mk(1, 0), mk(0, 0), 0.0);
+    gemm(g2, d, mk(1, 0), mk(0, 0), 0.0);
+    {
+      Prof pr(*this, "elementwise", 0.0, 80.0 * n * (double)n * ud.size());
+      unfold_matrices(upload(ud), (int)ud.size(), nx, ny, stream_);
+    }
+    gemm(h1, n, mk(1, 0), mk(0, 0), 0.0);
+    gemm(h2, n, mk(1, 0), mk(0, 0), 0.0);
+    sync();
+    for (auto* p : tmp) free_mat(p, d);
+    for (auto* p : F) free_mat(p, n);
+    for (auto* p : T) free_mat(p, n);
+  }
+}
+
+void Engine::solve_cells(const std::vector<CellSpec>& cells, int method, const RedhefferOpts& o, int nslices,
+                         std::vector<CellResult>& out) {
+  for (const auto& c : cells) validate(c);
+  std::vector<int> general, mirrored;
+  for (size_t c = 0; c < cells.size(); ++c) (mirror_symmetric(cells[c]) ? mirrored : general).push_back((int)c);
+  if (mirrored.empty()) {
+    solve(cells, method, o, nslices, out, FOLD_NONE);
+    return;
+  }
+  start_results(cells, out);
+  {
+    std::vector<CellSpec> one, four;
+    for (int c : mirrored) {
+      one.push_back(cells[c]);
+      four.insert(four.end(), 4, cells[c]);
+    }
+    Held h{*this, {}}, full{*this, {}};
+    solve(four, method, o, nslices, h.r, FOLD_ALL);
+    start_results(one, full.r);
+    std::vector<int> pick;
+    for (size_t i = 0; i < mirrored.size(); ++i) {
+      int status;
+      if (class_status(h.r, i, &status)) {
+        copy_counts(full.r[i], h.r[4 * i], status);
+        pick.push_back((int)i);
+      } else {
+        general.push_back(mirrored[i]);
+      }
+    }
+    unfold_results(one, h.r, pick, full.r);
+    for (int i : pick) {
+      out[mirrored[i]] = full.r[i];
+      full.r[i] = CellResult();
+    }
+  }
+  if (general.empty()) return;
+  std::sort(general.begin(), general.end());
+  std::vector<CellSpec> cs;
+  for (int c : general) cs.push_back(cells[c]);
+  std::vector<CellResult> g;
+  solve(cs, method, o, nslices, g, FOLD_NONE);
+  for (size_t i = 0; i < general.size(); ++i) out[general[i]] = g[i];
+}
+
+void Engine::solve_powers(const std::vector<CellSpec>& cells, int method, const RedhefferOpts& o, int nslices,
+                          int side, int flux_norm, std::vector<CellResult>& res, std::vector<std::vector<double>>& R,
+                          std::vector<std::vector<double>>& T) {
+  for (const auto& c : cells) validate(c);
+  start_results(cells, res);
+  R.assign(cells.size(), {});
+  T.assign(cells.size(), {});
+  std::vector<int> general, mirrored;
+  for (size_t c = 0; c < cells.size(); ++c)
+    (mirror_symmetric(cells[c]) && cells[c].has_end0 && cells[c].has_end1 ? mirrored : general).push_back((int)c);
+  if (!mirrored.empty()) {
+    std::vector<CellSpec> one, four;
+    for (int c : mirrored) {
+      one.push_back(cells[c]);
+      four.insert(four.end(), 4, cells[c]);
+    }
+    Held h{*this, {}};
+    solve(four, method, o, nslices, h.r, FOLD_EXCITED);
+    std::vector<std::vector<double>> Rm, Tm;
+    order_powers(one, h.r, side, flux_norm, Rm, Tm, FOLD_EXCITED);
+    for (size_t i = 0; i < mirrored.size(); ++i) {
+      const int c = mirrored[i];
+      int status;
+      if (!class_status(h.r, i, &status)) {
+        general.push_back(c);
+        continue;
+      }
+      R[c] = std::move(Rm[i]);
+      T[c] = std::move(Tm[i]);
+      copy_counts(res[c], h.r[4 * i], status);
+    }
+  }
+  if (general.empty()) return;
+  std::sort(general.begin(), general.end());
+  std::vector<CellSpec> cs;
+  for (int c : general) cs.push_back(cells[c]);
+  Held h{*this, {}};
+  solve(cs, method, o, nslices, h.r, FOLD_NONE);
+  std::vector<std::vector<double>> Rg, Tg;
+  order_powers(cs, h.r, side, flux_norm, Rg, Tg);
+  for (size_t i = 0; i < general.size(); ++i) {
+    const int c = general[i];
+    R[c] = std::move(Rg[i]);
+    T[c] = std::move(Tg[i]);
+    copy_counts(res[c], h.r[i], h.r[i].status);
   }
 }
 

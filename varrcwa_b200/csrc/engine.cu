@@ -740,10 +740,10 @@ void Engine::release_cell(CellDev* cd) {
 // ---------------------------------------------------------------------------
 namespace {
 struct AsmKey {
-  int nx, ny, ncx, ncy, pml, pillar, devgeom;
+  int nx, ny, ncx, ncy, pml, pillar, devgeom, mirrored;
   bool operator<(const AsmKey& o) const {
-    return std::tie(nx, ny, ncx, ncy, pml, pillar, devgeom) <
-           std::tie(o.nx, o.ny, o.ncx, o.ncy, o.pml, o.pillar, o.devgeom);
+    return std::tie(nx, ny, ncx, ncy, pml, pillar, devgeom, mirrored) <
+           std::tie(o.nx, o.ny, o.ncx, o.ncy, o.pml, o.pillar, o.devgeom, o.mirrored);
   }
 };
 }  // namespace
@@ -828,6 +828,7 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
     k.nx = r.spec->nx;
     k.ny = r.spec->ny;
     k.pml = r.spec->pml ? 1 : 0;
+    k.mirrored = r.mirrored ? 1 : 0;
     // a perturbed copy (the geometric adjoint's, with a host callback) shares
     // its structure's CellDev but not its rules: it stays on the host path
     k.devgeom = (!r.homogeneous && r.cd && r.cd->dev_geom && r.spec->kind == GEOM_GRID && !r.spec->geom_cb) ? 1 : 0;
@@ -989,6 +990,12 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
           }
         }
       }
+      int* dstat = nullptr;
+      if (status) {
+        dstat = (int*)bytes(B * sizeof(int));
+        VRC_CUDA_CHECK(cudaMemsetAsync(dstat, 0, B * sizeof(int), stream_));
+      }
+      if (k.pillar && k.mirrored && dstat) mirror_check(d_eps, (int)B, nc, nr, dstat, stream_);
       auto ex = ptrs(o_ex), exs = ptrs(o_exs), ey = ptrs(o_ey);
       twiddles(upload(xp), upload(ex), (int)B, ncx, P, stream_);
       twiddles(upload(xsp), upload(exs), (int)B, ncx, P, stream_);
@@ -1006,11 +1013,6 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
       // F2 = BX * Ey^T (P x Q)
       small_gemm(P, Q, nr, upload(cst(bx)), P, upload(cst(ey)), Q, 1, upload(f2), P, (int)B, stream_);
       auto ti = ptrs(o_ti), tj = ptrs(o_tj);
-      int* dstat = nullptr;
-      if (status) {
-        dstat = (int*)bytes(B * sizeof(int));
-        VRC_CUDA_CHECK(cudaMemsetAsync(dstat, 0, B * sizeof(int), stream_));
-      }
       toeplitz_inverses(upload(cst(ax)), upload(ti), nx, nr, (int)B, dstat, stream_);
       toeplitz_inverses(upload(cst(ay)), upload(tj), ny, nc, (int)B, dstat, stream_);
       auto g11 = ptrs(o_g11), g22 = ptrs(o_g22);

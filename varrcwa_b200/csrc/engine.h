@@ -201,6 +201,7 @@ class Engine {
     cplx* P;
     cplx* Q;
     cplx* keep_fe33inv = nullptr;  // optional copy of fe33^-1 (m x m; periodic cells)
+    bool mirrored = false;  // the raster has to be its own mirror image (else status ST_ASYMMETRIC)
   };
   void assemble(std::vector<SampleReq>& reqs, std::vector<int>* status);
   // samples of caller-sampler cells (GEOM_SAMPLER): the callbacks fill P, Q
@@ -281,6 +282,9 @@ class Engine {
   void diff_slices(std::vector<DiffReq>& reqs, int n, std::vector<int>* status);
 
   // ---- drivers ----
+  // FOLD_ALL / FOLD_EXCITED: the cells are parity classes, four per cell, and
+  // every one's S-matrix is wanted, or those a normally incident wave excites
+  enum { FOLD_NONE = 0, FOLD_ALL = 1, FOLD_EXCITED = 2 };
   struct RedhefferOpts {
     double pe = 1e-2;
     int max_depth = 40;
@@ -289,6 +293,9 @@ class Engine {
     // the class order starts at class `rotate` (mod the class count), so that
     // concurrent engines given the same mix work on different sizes at once
     int rotate = 0;
+    // cells come four at a time, the parity classes of one mirror-symmetric
+    // cell (fold.cu): results are in the classes' own bases
+    int folded = FOLD_NONE;
   };
   void redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& o, std::vector<CellResult>& out);
   // Gradient with respect to the rule knots of grid cells of one truncation,
@@ -302,14 +309,32 @@ class Engine {
   void cell_backward(const std::vector<CellSpec>& cells, const std::vector<std::vector<double>>& cuts,
                      const std::vector<const cplx*>& gS, const std::vector<const cplx*>& gB,
                      const std::vector<const cplx*>& ends, int every, std::vector<std::vector<double>>& grad);
-  void rcwa(const std::vector<CellSpec>& cells, int N, std::vector<CellResult>& out);
-  void differential(const std::vector<CellSpec>& cells, int N, std::vector<CellResult>& out);
+  void rcwa(const std::vector<CellSpec>& cells, int N, std::vector<CellResult>& out, int folded = FOLD_NONE);
+  void differential(const std::vector<CellSpec>& cells, int N, std::vector<CellResult>& out, int folded = FOLD_NONE);
+  // redheffer (method 0), rcwa (1) or differential (2) of the cells as given ...
+  void solve(const std::vector<CellSpec>& cells, int method, const RedhefferOpts& o, int nslices,
+             std::vector<CellResult>& out, int folded);
+  // ... and of whole cells, mirror-symmetric ones through their parity classes
+  void solve_cells(const std::vector<CellSpec>& cells, int method, const RedhefferOpts& o, int nslices,
+                   std::vector<CellResult>& out);
+  // full-order results of the picked cells from their classes' (four per cell)
+  void unfold_results(const std::vector<CellSpec>& cells, const std::vector<CellResult>& sub,
+                      const std::vector<int>& pick, std::vector<CellResult>& out);
   void release_result(CellResult& r);
 
   // Per-order powers for the two polarisations (px,py) = (1,0), (0,1).
   // side 0: incidence from z0 (Rdu, Tuu), 1: from z1 (Rud, Tdd).
+  // folded: res holds four parity classes per cell.
   void order_powers(const std::vector<CellSpec>& cells, const std::vector<CellResult>& res, int side,
-                    int flux_norm, std::vector<std::vector<double>>& R, std::vector<std::vector<double>>& T);
+                    int flux_norm, std::vector<std::vector<double>>& R, std::vector<std::vector<double>>& T,
+                    int folded = FOLD_NONE);
+
+  // order_powers of cells solved by the given method (0 adaptive, 1 RCWA, 2
+  // differential), mirror-symmetric ones through their parity classes; res
+  // receives statuses and trees (no device blocks).
+  void solve_powers(const std::vector<CellSpec>& cells, int method, const RedhefferOpts& o, int nslices, int side,
+                    int flux_norm, std::vector<CellResult>& res, std::vector<std::vector<double>>& R,
+                    std::vector<std::vector<double>>& T);
 
   // ---- layer stacks of z-uniform pixel rasters: forward and adjoint ----
   // Layer l (0 nearest z0) holds an npy x npx raster of real permittivity on a

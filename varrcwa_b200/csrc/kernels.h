@@ -149,6 +149,33 @@ void axpby_batched(const cplx* const* A, const cplx* const* B, cplx* const* C, c
 void order_power_batched(const PowerDesc* d, int batch, int m, cudaStream_t st);
 void matvec_batched(const MatVecDesc* d, int batch, int n, cudaStream_t st);
 
+// ---- mirror-symmetric cells (fold.cu) ------------------------------------------------
+// Order of the four parity classes of a cell with nx x ny harmonics.
+inline int fold_order(int nx, int ny) { return (nx * ny + 1) / 2; }
+// One class's P, Q (fold_order x fold_order) from the full matrices of a sample.
+struct FoldDesc {
+  const cplx *Pfull, *Qfull;
+  cplx *P, *Q;
+  double k0sq;
+  int cls;
+};
+void fold_batched(const FoldDesc* d, int batch, int nx, int ny, cudaStream_t st);
+// All harmonics (2 nx ny) of a class's E vector.
+struct UnfoldDesc {
+  const cplx* in;
+  cplx* out;
+  int cls;
+};
+void unfold_batched(const UnfoldDesc* d, int batch, int nx, int ny, cudaStream_t st);
+// All harmonics (2 nx ny square) of an operator on E from its four classes.
+struct UnfoldMatDesc {
+  const cplx* in[4];
+  cplx* out;
+};
+void unfold_matrices(const UnfoldMatDesc* d, int batch, int nx, int ny, cudaStream_t st);
+// status[s] = ST_ASYMMETRIC where raster s is not its own mirror image along x and y.
+void mirror_check(const cplx* const* d_eps, int batch, int npx, int npy, int* d_status, cudaStream_t st);
+
 // ---- layer-stack forward / adjoint (adjoint.cu) ------------------------------------
 // out = diag(rs) A diag(cs); rs / cs (or an entry of them) may be null.
 void scale_batched(const cplx* const* A, const cplx* const* rs, const cplx* const* cs, cplx* const* out, int batch,
