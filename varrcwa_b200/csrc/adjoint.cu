@@ -251,219 +251,146 @@ __device__ bool warp_inverse(cplx* a, cplx* fcol, int* piv, int t, int lane) {
 
 constexpr int PX_THREADS = 256, PX_WARPS = PX_THREADS / 32;
 
-// Per-warp scratch (complex elements) of pixel_adjoint_kernel.
-__host__ __device__ inline int px_warp_scratch(int t) { return 3 * t * t + 2 * (2 * t - 1) + t; }
-
-// One CTA per (stack, layer): dL/d(pixel) from dL/dfe11, dL/dfe22, dL/dfe33 on a
-// uniform npy x npx grid (FourierSolver2D::solve, src/rcwa/FourierSolver2D.cpp:
-// 43-349: Laurent rule for fe33, Li's inverse rule for fe11 (y strips) and
-// fe22 (x columns)).  The per-strip Toeplitz inverses are recomputed here.
-// The Toeplitz-diagonal sums of dL/dfe11 and dL/dfe22 (K11, K22: read by every
-// strip) go to a global scratch of the layer (L2 resident), so that 15 x 15
-// orders fit; the CTA has as many warps as its shared memory allows.
-__global__ void __launch_bounds__(PX_THREADS)
-    pixel_adjoint_kernel(const PixAdjDesc* __restrict__ ds, int nx, int ny, int npx, int npy) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const PixAdjDesc d = ds[blockIdx.x];
-  const int P = 2 * nx - 1, Q = 2 * ny - 1, m = nx * ny, t = nx > ny ? nx : ny;
-  const int NW = blockDim.x >> 5;
-  cplx* Ex = reinterpret_cast<cplx*>(smem_raw);  // [npx][P]
-  cplx* Ey = Ex + (size_t)P * npx;               // [npy][Q]
-  cplx* gf = Ey + (size_t)Q * npy;               // [Q][P]
-  cplx* H1 = gf + (size_t)P * Q;                 // [Q][npx]
-  cplx* wsc = H1 + (size_t)Q * npx;              // per-warp scratch
-  double* acc = reinterpret_cast<double*>(wsc + (size_t)NW * px_warp_scratch(t));  // [npy][npx]
-  int* pivs = reinterpret_cast<int*>(acc + (size_t)npy * npx);
-  cplx* K11 = d.kscr;                            // [Q][nx][nx]
-  cplx* K22 = d.kscr + (size_t)Q * nx * nx;      // [P][ny][ny]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int NT = blockDim.x;
-
-  for (int idx = tid; idx < P * npx; idx += NT) {
-    const int c = idx / P, p = idx - c * P;
-    Ex[idx] = twiddle(p, nx - 1, d.Lx * c / npx, d.Lx * (c + 1) / npx, d.Lx);
-  }
-  for (int idx = tid; idx < Q * npy; idx += NT) {
-    const int r = idx / Q, q = idx - r * Q;
-    Ey[idx] = twiddle(q, ny - 1, d.Ly * r / npy, d.Ly * (r + 1) / npy, d.Ly);
-  }
+// dL/d(pixel) from dL/dfe11, dL/dfe22, dL/dfe33 on a uniform npy x npx grid
+// (FourierSolver2D::solve, src/rcwa/FourierSolver2D.cpp:43-349: Laurent rule
+// for fe33, Li's inverse rule for fe11 (y strips) and fe22 (x columns)).  First
+// the Toeplitz-diagonal sums of the three (K11, K22, gf, in the layer's
+// scratch), then one warp per strip: all rows of all layers, each row's pixels
+// written (fe33 and fe11), then all columns, added to (fe22).  The per-strip
+// Toeplitz inverses are recomputed.  Bound by the strips' serial inversions, so
+// they are spread over the GPU: with one CTA per layer doing all its strips, a
+// layer after the other, the four layers of one 9 x 9-order stack of 64 x 64
+// pixels took 4.5 ms.
+__global__ void pixel_sums_kernel(const PixAdjDesc* __restrict__ ds, int nx, int ny) {
+  const PixAdjDesc d = ds[blockIdx.y];
+  const int P = 2 * nx - 1, Q = 2 * ny - 1, m = nx * ny;
+  cplx* K11 = d.kscr;                        // [Q][nx][nx]
+  cplx* K22 = K11 + (size_t)Q * nx * nx;     // [P][ny][ny]
+  cplx* gf = K22 + (size_t)P * ny * ny;      // [Q][P]
   auto G = [&](const cplx* M, int a, int c, int b, int dd) { return M[(size_t)(b * ny + dd) * m + a * ny + c]; };
-  // Toeplitz-diagonal sums of the three Fourier-block adjoints
-  for (int idx = tid; idx < Q * nx * nx; idx += NT) {
-    const int q = idx / (nx * nx), rem = idx - q * nx * nx, b = rem / nx, a = rem - b * nx;
-    const int qq = q - (ny - 1);
+  const int n1 = Q * nx * nx, n2 = P * ny * ny, n3 = P * Q;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n1 + n2 + n3; e += gridDim.x * blockDim.x) {
     cplx s = mk(0.0, 0.0);
-    for (int c = 0; c < ny; ++c) {
-      const int dd = c - qq;
-      if (dd >= 0 && dd < ny) s = cadd(s, G(d.g11, a, c, b, dd));
+    if (e < n1) {
+      const int q = e / (nx * nx), rem = e - q * nx * nx, b = rem / nx, a = rem - b * nx;
+      const int qq = q - (ny - 1);
+      for (int c = max(0, qq); c < min(ny, ny + qq); ++c) s = cadd(s, G(d.g11, a, c, b, c - qq));
+      K11[e] = s;
+    } else if (e < n1 + n2) {
+      const int idx = e - n1, p = idx / (ny * ny), rem = idx - p * ny * ny, dd = rem / ny, c = rem - dd * ny;
+      const int pp = p - (nx - 1);
+      for (int a = max(0, pp); a < min(nx, nx + pp); ++a) s = cadd(s, G(d.g22, a, c, a - pp, dd));
+      K22[idx] = s;
+    } else {
+      const int idx = e - n1 - n2, q = idx / P, p = idx - q * P;
+      const int pp = p - (nx - 1), qq = q - (ny - 1);
+      for (int a = max(0, pp); a < min(nx, nx + pp); ++a)
+        for (int c = max(0, qq); c < min(ny, ny + qq); ++c) s = cadd(s, G(d.g33, a, c, a - pp, c - qq));
+      gf[idx] = s;
     }
-    K11[idx] = s;
   }
-  for (int idx = tid; idx < P * ny * ny; idx += NT) {
-    const int p = idx / (ny * ny), rem = idx - p * ny * ny, dd = rem / ny, c = rem - dd * ny;
-    const int pp = p - (nx - 1);
-    cplx s = mk(0.0, 0.0);
-    for (int a = 0; a < nx; ++a) {
-      const int b = a - pp;
-      if (b >= 0 && b < nx) s = cadd(s, G(d.g22, a, c, b, dd));
-    }
-    K22[idx] = s;
-  }
-  for (int idx = tid; idx < P * Q; idx += NT) {
-    const int q = idx / P, p = idx - q * P;
-    const int pp = p - (nx - 1), qq = q - (ny - 1);
-    cplx s = mk(0.0, 0.0);
-    for (int a = 0; a < nx; ++a) {
-      const int b = a - pp;
-      if (b < 0 || b >= nx) continue;
-      for (int c = 0; c < ny; ++c) {
-        const int dd = c - qq;
-        if (dd >= 0 && dd < ny) s = cadd(s, G(d.g33, a, c, b, dd));
-      }
-    }
-    gf[idx] = s;
-  }
-  __syncthreads();
-  // fe33 (Laurent rule): four = Ex f^T Ey^T  ->  df = Ey^H-weighted sums
-  for (int idx = tid; idx < Q * npx; idx += NT) {
-    const int q = idx / npx, c = idx - q * npx;
-    cplx s = mk(0.0, 0.0);
-    for (int p = 0; p < P; ++p) s = cadd(s, cmulc(Ex[c * P + p], gf[q * P + p]));
-    H1[idx] = s;
-  }
-  __syncthreads();
-  for (int idx = tid; idx < npy * npx; idx += NT) {
-    const int r = idx / npx, c = idx - r * npx;
-    double s = 0.0;
-    for (int q = 0; q < Q; ++q) {
-      const cplx h = H1[q * npx + c], e = Ey[r * Q + q];  // h * conj(e)
-      s += h.x * e.x + h.y * e.y;
-    }
-    acc[idx] = s;
-  }
-  __syncthreads();
-  cplx* T = wsc + (size_t)warp * px_warp_scratch(t);
+}
+
+// Per-warp shared memory (complex elements) of a strip of `len` pixels with t
+// harmonics along it and ho Fourier coefficients across it.
+__host__ __device__ inline int px_strip_scratch(int t, int len, int ho) {
+  return 3 * t * t + 3 * (2 * t - 1) + t + len + ho;
+}
+
+template <bool ROWS>
+__global__ void __launch_bounds__(PX_THREADS)
+    pixel_strip_kernel(const PixAdjDesc* __restrict__ ds, int nx, int ny, int npx, int npy) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const PixAdjDesc d = ds[blockIdx.y];
+  const int P = 2 * nx - 1, Q = 2 * ny - 1, NW = blockDim.x >> 5;
+  // along the strip: t harmonics, H coefficients, len pixels; across: HO
+  const int t = ROWS ? nx : ny, H = 2 * t - 1, HO = ROWS ? Q : P, len = ROWS ? npx : npy;
+  const int strips = ROWS ? npy : npx, to = ROWS ? ny : nx;
+  const double D = ROWS ? d.Lx : d.Ly, DO = ROWS ? d.Ly : d.Lx;
+  const cplx* K = d.kscr + (ROWS ? 0 : (size_t)Q * nx * nx);  // [HO][t][t]
+  const cplx* gf = d.kscr + (size_t)Q * nx * nx + (size_t)P * ny * ny;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  cplx* E = reinterpret_cast<cplx*>(smem_raw);  // [len][H]
+  cplx* T = E + (size_t)len * H + (size_t)warp * px_strip_scratch(t, len, HO);
   cplx* gT = T + t * t;
   cplx* tmp = gT + t * t;
-  cplx* gvec = tmp + t * t;        // 2t-1: Fourier coefficients of 1/eps
-  cplx* gv = gvec + (2 * t - 1);   // 2t-1: Toeplitz-diagonal adjoint
-  cplx* fcol = gv + (2 * t - 1);   // t
-  int* piv = pivs + warp * 32;
-  // fe11: one y strip r per warp pass; T_r = inv(Toep(Ex (1/eps[r, :])))
-  for (int r = warp; r < npy; r += NW) {
-    const cplx* er = d.eps + (size_t)r * npx;
-    for (int p = lane; p < P; p += 32) {
-      cplx s = mk(0.0, 0.0);
-      for (int c = 0; c < npx; ++c) s = cadd(s, cmul(Ex[c * P + p], cinv(er[c])));
-      gvec[p] = s;
-    }
-    __syncwarp();
-    for (int idx = lane; idx < nx * nx; idx += 32) {
-      const int k = idx / nx, i = idx - k * nx;
-      T[k * nx + i] = gvec[nx - 1 + i - k];
-    }
-    __syncwarp();
-    warp_inverse(T, fcol, piv, nx, lane);
-    // gT[a,b] = sum_q conj(Ey[q, r]) K11[q, b, a]
-    for (int idx = lane; idx < nx * nx; idx += 32) {
-      const int b = idx / nx, a = idx - b * nx;
-      cplx s = mk(0.0, 0.0);
-      for (int q = 0; q < Q; ++q) s = cadd(s, cmulc(Ey[r * Q + q], K11[(q * nx + b) * nx + a]));
-      gT[b * nx + a] = s;
-    }
-    __syncwarp();
-    // tmp = T^H gT ; gT <- -tmp T^H
-    for (int idx = lane; idx < nx * nx; idx += 32) {
-      const int b = idx / nx, a = idx - b * nx;
-      cplx s = mk(0.0, 0.0);
-      for (int k = 0; k < nx; ++k) s = cadd(s, cmulc(T[a * nx + k], gT[b * nx + k]));
-      tmp[b * nx + a] = s;
-    }
-    __syncwarp();
-    for (int idx = lane; idx < nx * nx; idx += 32) {
-      const int b = idx / nx, a = idx - b * nx;
-      cplx s = mk(0.0, 0.0);
-      for (int k = 0; k < nx; ++k) s = cadd(s, cmul(tmp[k * nx + a], cconj(T[k * nx + b])));
-      gT[b * nx + a] = cneg(s);
-    }
-    __syncwarp();
-    for (int k = lane; k < P; k += 32) {
-      const int off = k - (nx - 1);  // a - b
-      cplx s = mk(0.0, 0.0);
-      for (int b = 0; b < nx; ++b) {
-        const int a = b + off;
-        if (a >= 0 && a < nx) s = cadd(s, gT[b * nx + a]);
-      }
-      gv[k] = s;
-    }
-    __syncwarp();
-    for (int c = lane; c < npx; c += 32) {
-      cplx s = mk(0.0, 0.0);
-      for (int k = 0; k < P; ++k) s = cadd(s, cmulc(Ex[c * P + k], gv[k]));
-      const cplx w = cinv(er[c]);
-      const cplx w2 = cmul(w, w);
-      // conj(-w^2) * s, real part
-      acc[r * npx + c] += -(w2.x * s.x + w2.y * s.y);
-    }
-    __syncwarp();
+  cplx* gvec = tmp + t * t;  // H: Fourier coefficients of 1/eps
+  cplx* gv = gvec + H;       // H: Toeplitz-diagonal adjoint
+  cplx* v33 = gv + H;        // H: this row of dL/dfe33
+  cplx* fcol = v33 + H;      // t
+  cplx* w = fcol + t;        // len: 1/eps
+  cplx* eo = w + len;        // HO: twiddles across the strip
+  int* piv = reinterpret_cast<int*>(E + (size_t)len * H + (size_t)NW * px_strip_scratch(t, len, HO)) + warp * 32;
+  for (int idx = tid; idx < len * H; idx += blockDim.x) {
+    const int c = idx / H, p = idx - c * H;
+    E[idx] = twiddle(p, t - 1, D * c / len, D * (c + 1) / len, D);
   }
   __syncthreads();
-  // fe22: one x column i per warp pass; T_i = inv(Toep(Ey (1/eps[:, i])))
-  for (int i = warp; i < npx; i += NW) {
-    for (int q = lane; q < Q; q += 32) {
-      cplx s = mk(0.0, 0.0);
-      for (int r = 0; r < npy; ++r) s = cadd(s, cmul(Ey[r * Q + q], cinv(d.eps[(size_t)r * npx + i])));
-      gvec[q] = s;
+  const int r = blockIdx.x * NW + warp;  // this warp's strip
+  if (r >= strips) return;
+  const cplx* er = d.eps + (ROWS ? (size_t)r * npx : r);
+  double* gr = d.grad + (ROWS ? (size_t)r * npx : r);
+  const int st = ROWS ? 1 : npx;
+  for (int c = lane; c < len; c += 32) w[c] = cinv(er[(size_t)c * st]);
+  for (int q = lane; q < HO; q += 32) eo[q] = twiddle(q, to - 1, DO * r / strips, DO * (r + 1) / strips, DO);
+  __syncwarp();
+  for (int p = lane; p < H; p += 32) {
+    cplx s = mk(0.0, 0.0), u = s;
+    for (int c = 0; c < len; ++c) s = cadd(s, cmul(E[c * H + p], w[c]));
+    gvec[p] = s;
+    if (ROWS) {
+      for (int q = 0; q < HO; ++q) u = cadd(u, cmulc(eo[q], gf[q * H + p]));
+      v33[p] = u;
     }
-    __syncwarp();
-    for (int idx = lane; idx < ny * ny; idx += 32) {
-      const int k = idx / ny, ii = idx - k * ny;
-      T[k * ny + ii] = gvec[ny - 1 + ii - k];
-    }
-    __syncwarp();
-    warp_inverse(T, fcol, piv, ny, lane);
-    for (int idx = lane; idx < ny * ny; idx += 32) {
-      const int dd = idx / ny, c = idx - dd * ny;
-      cplx s = mk(0.0, 0.0);
-      for (int p = 0; p < P; ++p) s = cadd(s, cmulc(Ex[i * P + p], K22[(p * ny + dd) * ny + c]));
-      gT[dd * ny + c] = s;
-    }
-    __syncwarp();
-    for (int idx = lane; idx < ny * ny; idx += 32) {
-      const int b = idx / ny, a = idx - b * ny;
-      cplx s = mk(0.0, 0.0);
-      for (int k = 0; k < ny; ++k) s = cadd(s, cmulc(T[a * ny + k], gT[b * ny + k]));
-      tmp[b * ny + a] = s;
-    }
-    __syncwarp();
-    for (int idx = lane; idx < ny * ny; idx += 32) {
-      const int b = idx / ny, a = idx - b * ny;
-      cplx s = mk(0.0, 0.0);
-      for (int k = 0; k < ny; ++k) s = cadd(s, cmul(tmp[k * ny + a], cconj(T[k * ny + b])));
-      gT[b * ny + a] = cneg(s);
-    }
-    __syncwarp();
-    for (int k = lane; k < Q; k += 32) {
-      const int off = k - (ny - 1);
-      cplx s = mk(0.0, 0.0);
-      for (int b = 0; b < ny; ++b) {
-        const int a = b + off;
-        if (a >= 0 && a < ny) s = cadd(s, gT[b * ny + a]);
-      }
-      gv[k] = s;
-    }
-    __syncwarp();
-    for (int r = lane; r < npy; r += 32) {
-      cplx s = mk(0.0, 0.0);
-      for (int k = 0; k < Q; ++k) s = cadd(s, cmulc(Ey[r * Q + k], gv[k]));
-      const cplx w = cinv(d.eps[(size_t)r * npx + i]);
-      const cplx w2 = cmul(w, w);
-      acc[r * npx + i] += -(w2.x * s.x + w2.y * s.y);
-    }
-    __syncwarp();
   }
-  __syncthreads();
-  for (int idx = tid; idx < npy * npx; idx += NT) d.grad[idx] = acc[idx];
+  __syncwarp();
+  for (int idx = lane; idx < t * t; idx += 32) {
+    const int k = idx / t, i = idx - k * t;
+    T[k * t + i] = gvec[t - 1 + i - k];
+  }
+  __syncwarp();
+  warp_inverse(T, fcol, piv, t, lane);
+  // gT[a,b] = sum_q conj(eo[q]) K[q, b, a]
+  for (int idx = lane; idx < t * t; idx += 32) {
+    cplx s = mk(0.0, 0.0);
+    for (int q = 0; q < HO; ++q) s = cadd(s, cmulc(eo[q], K[(size_t)q * t * t + idx]));
+    gT[idx] = s;
+  }
+  __syncwarp();
+  // tmp = T^H gT ; gT <- -tmp T^H
+  for (int idx = lane; idx < t * t; idx += 32) {
+    const int b = idx / t, a = idx - b * t;
+    cplx s = mk(0.0, 0.0);
+    for (int k = 0; k < t; ++k) s = cadd(s, cmulc(T[a * t + k], gT[b * t + k]));
+    tmp[b * t + a] = s;
+  }
+  __syncwarp();
+  for (int idx = lane; idx < t * t; idx += 32) {
+    const int b = idx / t, a = idx - b * t;
+    cplx s = mk(0.0, 0.0);
+    for (int k = 0; k < t; ++k) s = cadd(s, cmul(tmp[k * t + a], cconj(T[k * t + b])));
+    gT[b * t + a] = cneg(s);
+  }
+  __syncwarp();
+  for (int k = lane; k < H; k += 32) {
+    const int off = k - (t - 1);  // a - b
+    cplx s = mk(0.0, 0.0);
+    for (int b = max(0, -off); b < min(t, t - off); ++b) s = cadd(s, gT[b * t + b + off]);
+    gv[k] = s;
+  }
+  __syncwarp();
+  for (int c = lane; c < len; c += 32) {
+    cplx s = mk(0.0, 0.0);
+    double s33 = 0.0;
+    for (int k = 0; k < H; ++k) {
+      const cplx e = E[c * H + k];
+      s = cadd(s, cmulc(e, gv[k]));
+      if (ROWS) s33 += e.x * v33[k].x + e.y * v33[k].y;
+    }
+    const cplx w2 = cmul(w[c], w[c]);
+    const double g = -(w2.x * s.x + w2.y * s.y);  // Re conj(-w^2) s
+    gr[(size_t)c * st] = ROWS ? s33 + g : gr[(size_t)c * st] + g;
+  }
 }
 
 // Per-order powers of a stack (RCWASolver::scatterPlaneWave,
@@ -606,33 +533,45 @@ void thick_adjoint_batched(const ThickAdjDesc* d, int batch, int n, cudaStream_t
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 
-size_t pixel_adjoint_smem(int nx, int ny, int npx, int npy, int nw) {
+// Rasters accepted: both directions' twiddle tables, the coefficients and one
+// strip's matrices within a CTA's shared memory, at most 32 harmonics an axis.
+bool pixel_adjoint_fits(int nx, int ny, int npx, int npy) {
+  if (nx > 32 || ny > 32) return false;
   const int P = 2 * nx - 1, Q = 2 * ny - 1, t = nx > ny ? nx : ny;
-  size_t c = (size_t)P * npx + (size_t)Q * npy + (size_t)P * Q + (size_t)Q * npx + (size_t)nw * px_warp_scratch(t);
-  return c * 16 + (size_t)npy * npx * 8 + (size_t)nw * 32 * sizeof(int);
+  const size_t c = (size_t)P * npx + (size_t)Q * npy + (size_t)P * Q + (size_t)Q * npx +
+                   (size_t)(3 * t * t + 2 * (2 * t - 1) + t);
+  return c * 16 + (size_t)npy * npx * 8 + 32 * sizeof(int) <= 227 * 1024;
 }
-
-// warps per CTA: the most (up to eight) whose shared memory fits; 0 if none
-int pixel_adjoint_warps(int nx, int ny, int npx, int npy) {
-  if (nx > 32 || ny > 32) return 0;
-  for (int nw = PX_WARPS; nw >= 1; nw /= 2)
-    if (pixel_adjoint_smem(nx, ny, npx, npy, nw) <= 227 * 1024) return nw;
-  return 0;
-}
-
-bool pixel_adjoint_fits(int nx, int ny, int npx, int npy) { return pixel_adjoint_warps(nx, ny, npx, npy) > 0; }
 
 size_t pixel_adjoint_scratch(int nx, int ny) {
-  return ((size_t)(2 * ny - 1) * nx * nx + (size_t)(2 * nx - 1) * ny * ny) * 16;
+  const int P = 2 * nx - 1, Q = 2 * ny - 1;
+  return ((size_t)Q * nx * nx + (size_t)P * ny * ny + (size_t)P * Q) * 16;
 }
 
 void pixel_adjoint_batched(const PixAdjDesc* d, int batch, int nx, int ny, int npx, int npy, cudaStream_t st) {
   if (batch <= 0) return;
-  const int nw = pixel_adjoint_warps(nx, ny, npx, npy);
-  if (!nw) throw StatusError(ST_EINVAL, "pixel adjoint: raster and harmonics exceed the shared-memory tile");
-  const size_t smem = pixel_adjoint_smem(nx, ny, npx, npy, nw);
-  ensure_smem((const void*)pixel_adjoint_kernel, smem);
-  pixel_adjoint_kernel<<<batch, nw * 32, smem, st>>>(d, nx, ny, npx, npy);
+  if (!pixel_adjoint_fits(nx, ny, npx, npy))
+    throw StatusError(ST_EINVAL, "pixel adjoint: raster and harmonics exceed the shared-memory tile");
+  // strips per CTA: the most (up to eight) that leave room
+  auto smem = [&](bool rows, int nw) {
+    const int t = rows ? nx : ny, len = rows ? npx : npy, ho = 2 * (rows ? ny : nx) - 1;
+    return ((size_t)len * (2 * t - 1) + (size_t)nw * px_strip_scratch(t, len, ho)) * 16 + nw * 32 * sizeof(int);
+  };
+  auto warps = [&](bool rows) {
+    int nw = PX_WARPS;
+    while (nw > 1 && smem(rows, nw) > 227 * 1024) nw /= 2;
+    return nw;
+  };
+  const int wr = warps(true), wc = warps(false);
+  ensure_smem((const void*)pixel_strip_kernel<true>, smem(true, wr));
+  ensure_smem((const void*)pixel_strip_kernel<false>, smem(false, wc));
+  for (int b0 = 0; b0 < batch; b0 += 65535) {
+    const int nb = batch - b0 < 65535 ? batch - b0 : 65535;
+    pixel_sums_kernel<<<dim3(8, nb), 256, 0, st>>>(d + b0, nx, ny);
+    pixel_strip_kernel<true><<<dim3((npy + wr - 1) / wr, nb), wr * 32, smem(true, wr), st>>>(d + b0, nx, ny, npx, npy);
+    pixel_strip_kernel<false><<<dim3((npx + wc - 1) / wc, nb), wc * 32, smem(false, wc), st>>>(d + b0, nx, ny, npx,
+                                                                                            npy);
+  }
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 
