@@ -165,28 +165,83 @@ __global__ void reciprocal_kernel(cplx* const* __restrict__ in, cplx* const* __r
 }
 
 // ---------------------------------------------------------------------------
-// Small batched contraction C[M x N] = A[M x K] * op(B), column-major,
-// one thread per output element (the operands are L1/L2 resident).
-// transB = 0: B is K x N (ldb); transB = 1: B is N x K (ldb), use B^T.
+// Batched contraction C[M x N] = A[M x K] * op(B), column-major, of the Fourier
+// stages (M harmonics, N strips, K pixels: 13..29 x 256 x 256 for a pillar's
+// raster).  transB = 0: B is K x N (ldb); transB = 1: B is N x K (ldb), use B^T.
+// A CTA computes SG_M x SG_N, a row and four columns per thread, its operands
+// staged through shared memory in slices of SG_K, three in flight.  Per slice
+// entry a warp has 16 FP64 instructions to five shared loads, so the FP64 pipe
+// and the shared-memory port are about level.  One thread per output, its
+// operands from global memory one k at a time, waited for memory at every step:
+// 94 us for three samples of 256 x 256 pixels at 7 orders.
 // ---------------------------------------------------------------------------
-__global__ void small_gemm_kernel(int M, int N, int K, const cplx* const* __restrict__ As, int lda,
-                                  const cplx* const* __restrict__ Bs, int ldb, int transB,
-                                  cplx* const* __restrict__ Cs, int ldc) {
-  const int s = blockIdx.y;
-  const cplx* A = As[s];
-  const cplx* B = Bs[s];
-  cplx* C = Cs[s];
-  const int total = M * N;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    int j = idx / M, i = idx - j * M;
-    cplx acc = mk(0.0, 0.0);
-    if (!transB) {
-      const cplx* b = B + (size_t)j * ldb;
-      for (int k = 0; k < K; ++k) acc = cfma(A[(size_t)k * lda + i], b[k], acc);
-    } else {
-      for (int k = 0; k < K; ++k) acc = cfma(A[(size_t)k * lda + i], B[(size_t)k * ldb + j], acc);
+constexpr int SG_M = 16, SG_N = 64, SG_K = 16, SG_ST = 3, SG_THREADS = 256;
+constexpr int SG_LDB = SG_N + 1;
+constexpr size_t SG_SMEM = (size_t)SG_ST * SG_K * (SG_M + SG_LDB) * sizeof(cplx);
+
+__device__ __forceinline__ void sg_copy(cplx* s, const cplx* g, bool on) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(s);
+  const int sz = on ? 16 : 0;  // zero-filled outside the operand
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(a), "l"(g), "r"(sz) : "memory");
+}
+
+template <int TRANSB>
+__global__ void __launch_bounds__(SG_THREADS)
+    small_gemm_kernel(int M, int N, int K, const cplx* const* __restrict__ As, int lda,
+                      const cplx* const* __restrict__ Bs, int ldb, cplx* const* __restrict__ Cs, int ldc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx* sa = reinterpret_cast<cplx*>(smem_raw);  // [SG_ST][SG_K][SG_M]
+  cplx* sb = sa + SG_ST * SG_K * SG_M;           // [SG_ST][SG_K][SG_LDB]
+  const cplx* A = As[blockIdx.y];
+  const cplx* B = Bs[blockIdx.y];
+  cplx* C = Cs[blockIdx.y];
+  const int tm = (M + SG_M - 1) / SG_M, m0 = (blockIdx.x % tm) * SG_M, n0 = (blockIdx.x / tm) * SG_N;
+  const int tid = threadIdx.x, i = tid % SG_M, jg = tid / SG_M;  // row, column group (columns jg + 16 q)
+  const int KT = (K + SG_K - 1) / SG_K;
+  auto load = [&](int kt) {
+    const int k0 = kt * SG_K, st = kt % SG_ST;
+    {
+      const int k = tid / SG_M, r = tid % SG_M;
+      const bool on = m0 + r < M && k0 + k < K;
+      sg_copy(sa + (st * SG_K + k) * SG_M + r, on ? A + (size_t)(k0 + k) * lda + m0 + r : A, on);
     }
-    C[(size_t)j * ldc + i] = acc;
+#pragma unroll
+    for (int q = 0; q < SG_K * SG_N / SG_THREADS; ++q) {
+      const int e = tid + q * SG_THREADS;
+      const int k = TRANSB ? e / SG_N : e % SG_K, c = TRANSB ? e % SG_N : e / SG_K;
+      const bool on = n0 + c < N && k0 + k < K;
+      const size_t at = TRANSB ? (size_t)(k0 + k) * ldb + n0 + c : (size_t)(n0 + c) * ldb + k0 + k;
+      sg_copy(sb + (st * SG_K + k) * SG_LDB + c, on ? B + at : B, on);
+    }
+  };
+  cplx acc[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) acc[q] = mk(0.0, 0.0);
+#pragma unroll
+  for (int s = 0; s < SG_ST - 1; ++s) {
+    if (s < KT) load(s);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  for (int kt = 0; kt < KT; ++kt) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(SG_ST - 2) : "memory");
+    __syncthreads();
+    if (kt + SG_ST - 1 < KT) load(kt + SG_ST - 1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const cplx* a = sa + (kt % SG_ST) * SG_K * SG_M;
+    const cplx* b = sb + (kt % SG_ST) * SG_K * SG_LDB;
+    const int kn = min(SG_K, K - kt * SG_K);
+#pragma unroll 4
+    for (int k = 0; k < kn; ++k) {
+      const cplx x = a[k * SG_M + i];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = cfma(x, b[k * SG_LDB + jg + 16 * q], acc[q]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int j = n0 + jg + 16 * q;
+    if (m0 + i < M && j < N) C[(size_t)j * ldc + m0 + i] = acc[q];
   }
 }
 
@@ -423,7 +478,10 @@ void reciprocal(cplx* const* d_in, cplx* const* d_out, int batch, int total, cud
 void small_gemm(int M, int N, int K, const cplx* const* d_A, int lda, const cplx* const* d_B, int ldb, int transB,
                 cplx* const* d_C, int ldc, int batch, cudaStream_t st) {
   if (batch <= 0) return;
-  small_gemm_kernel<<<grid_for(M * N, batch), 256, 0, st>>>(M, N, K, d_A, lda, d_B, ldb, transB, d_C, ldc);
+  auto kern = transB ? small_gemm_kernel<1> : small_gemm_kernel<0>;
+  ensure_smem((const void*)kern, SG_SMEM);
+  const int tiles = ((M + SG_M - 1) / SG_M) * ((N + SG_N - 1) / SG_N);
+  kern<<<dim3(tiles, batch), SG_THREADS, SG_SMEM, st>>>(M, N, K, d_A, lda, d_B, ldb, d_C, ldc);
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 
