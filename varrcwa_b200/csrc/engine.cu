@@ -1717,7 +1717,6 @@ void Engine::diff_slices(std::vector<DiffReq>& reqs, int n, std::vector<int>* st
     // L11 = I - a2 (P1Q0 + P1Q1 + P2Q1 - b2 P2Q1 P1Q0)
     // L22 = I - a2 (Q1P0 + Q1P1 + Q2P1 - b2 Q2P1 Q1P0)
     // (src/core/DifferentialIntegrator.cpp:58-65)
-    std::vector<double> a2(B), b2(B), h2(B);
     g.clear();
     for (size_t b = 0; b < B; ++b) {
       const DiffReq& r = reqs[c0 + b];
@@ -1729,34 +1728,17 @@ void Engine::diff_slices(std::vector<DiffReq>& reqs, int n, std::vector<int>* st
       g.push_back({Q2P1[b], r.Q1, U4[b], nullptr, nullptr, nullptr});   // Q2P1Q1
     }
     gemm(g, n, mk(1, 0), mk(0, 0), 0.0);
-    // Combine with per-slice scalars (one axpby launch per distinct scalar set)
-    for (size_t b = 0; b < B; ++b) {
-      const DiffReq& r = reqs[c0 + b];
-      const double k0 = r.k0, dz = r.dz;
-      const double A2 = dz * dz / (6. * k0 * k0), B2 = dz * dz / (4. * k0 * k0), H2 = dz * dz / (2. * k0 * k0);
-      const cplx c = mk(0.0, dz / (6. * k0));
-      auto ax = [&](const cplx* A, const cplx* Bv, cplx* C, cplx al, cplx be, double de) {
-        std::vector<const cplx*> va = {A}, vb = {Bv};
-        std::vector<cplx*> vc = {C};
-        axpby(va, vb, vc, al, be, de, n);
-      };
-      // S = P1Q0 + P1Q1 + P2Q1 - b2 X4 ; L11 = I - a2 S
-      ax(P1Q0[b], P1Q1[b], L11[b], mk(1, 0), mk(1, 0), 0.0);
-      ax(L11[b], P2Q1[b], L11[b], mk(1, 0), mk(1, 0), 0.0);
-      ax(L11[b], X4[b], L11[b], mk(-A2, 0), mk(A2 * B2, 0), 1.0);
-      ax(Q1P0[b], Q1P1[b], L22[b], mk(1, 0), mk(1, 0), 0.0);
-      ax(L22[b], Q2P1[b], L22[b], mk(1, 0), mk(1, 0), 0.0);
-      ax(L22[b], Y4[b], L22[b], mk(-A2, 0), mk(A2 * B2, 0), 1.0);
-      // L12 = c (P0 + 4 P1 + P2 - h2 (P1Q1P0 + P2Q1P1))
-      ax(r.P0, r.P1, L12[b], mk(1, 0), mk(4, 0), 0.0);
-      ax(L12[b], r.P2, L12[b], mk(1, 0), mk(1, 0), 0.0);
-      ax(U1[b], U2[b], U1[b], mk(1, 0), mk(1, 0), 0.0);
-      ax(L12[b], U1[b], L12[b], c, cmul(c, mk(-H2, 0)), 0.0);
-      ax(r.Q0, r.Q1, L21[b], mk(1, 0), mk(4, 0), 0.0);
-      ax(L21[b], r.Q2, L21[b], mk(1, 0), mk(1, 0), 0.0);
-      ax(U3[b], U4[b], U3[b], mk(1, 0), mk(1, 0), 0.0);
-      ax(L21[b], U3[b], L21[b], c, cmul(c, mk(-H2, 0)), 0.0);
-      (void)a2; (void)b2; (void)h2;
+    // S = P1Q0 + P1Q1 + P2Q1 - b2 X4 ; L11 = I - a2 S (L22 alike from Q)
+    // L12 = c (P0 + 4 P1 + P2 - h2 (P1Q1P0 + P2Q1P1)) (L21 alike from Q)
+    {
+      std::vector<DiffDesc> dd;
+      for (size_t b = 0; b < B; ++b) {
+        const DiffReq& r = reqs[c0 + b];
+        dd.push_back({P1Q0[b], P1Q1[b], P2Q1[b], X4[b], r.P0, r.P1, r.P2, U1[b], U2[b], L11[b], L12[b], r.k0, r.dz});
+        dd.push_back({Q1P0[b], Q1P1[b], Q2P1[b], Y4[b], r.Q0, r.Q1, r.Q2, U3[b], U4[b], L22[b], L21[b], r.k0, r.dz});
+      }
+      Prof pr(*this, "elementwise", 0.0, 16.0 * 11.0 * nn * dd.size());
+      diff_combine_batched(upload(dd), (int)dd.size(), n, stream_);
     }
     g.clear();
     for (size_t b = 0; b < B; ++b) {

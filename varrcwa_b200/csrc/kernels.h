@@ -130,6 +130,15 @@ struct PowerDesc {
   cplx eps_in, eps_out;
   double k0, tnorm;
 };
+// Propagator blocks of a differential-method slice (src/core/
+// DifferentialIntegrator.cpp:58-65): D = I - a2 (s0 + s1 + s2 - b2 x) and
+// O = c (p0 + 4 p1 + p2 - h2 (t0 + t1)), a2 = dz^2 / 6 k0^2, b2 = dz^2 / 4 k0^2,
+// h2 = dz^2 / 2 k0^2, c = i dz / 6 k0.
+struct DiffDesc {
+  const cplx *s0, *s1, *s2, *x, *p0, *p1, *p2, *t0, *t1;
+  cplx *D, *O;
+  double k0, dz;
+};
 struct MatVecDesc {
   const cplx* A;
   const cplx* x;
@@ -146,6 +155,7 @@ void phase_rows_batched(const cplx* const* A, const cplx* const* gam, const doub
 void set_identity_batched(cplx* const* A, int batch, int n, double diag, cudaStream_t st);
 void axpby_batched(const cplx* const* A, const cplx* const* B, cplx* const* C, cplx alpha, cplx beta, double delta,
                    int batch, int n, cudaStream_t st);
+void diff_combine_batched(const DiffDesc* d, int batch, int n, cudaStream_t st);
 void order_power_batched(const PowerDesc* d, int batch, int m, cudaStream_t st);
 void matvec_batched(const MatVecDesc* d, int batch, int n, cudaStream_t st);
 

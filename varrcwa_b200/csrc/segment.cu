@@ -179,6 +179,26 @@ __global__ void matvec_kernel(const MatVecDesc* __restrict__ ds, int n) {
   }
 }
 
+// One pass over a slice's eleven matrices (bound by memory); a launch per term
+// and slice, each with its own argument uploads, left the GPU idle most of a
+// differential solve: 460 launches and 31 ms for 32 slices at n = 126, of which
+// 14 ms were kernels.
+__global__ void diff_combine_kernel(const DiffDesc* __restrict__ ds, int n) {
+  const DiffDesc d = ds[blockIdx.y];
+  const double q = d.dz * d.dz / (d.k0 * d.k0), a2 = q / 6.0, b2 = q / 4.0, h2 = q / 2.0, c = d.dz / (6.0 * d.k0);
+  const long long total = (long long)n * n;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
+       e += (long long)gridDim.x * blockDim.x) {
+    cplx s = csub(cadd(cadd(d.s0[e], d.s1[e]), d.s2[e]), cscale(d.x[e], b2));
+    s = cscale(s, -a2);
+    if (e % (n + 1) == 0) s.x += 1.0;
+    d.D[e] = s;
+    const cplx p = cadd(cadd(d.p0[e], cscale(d.p1[e], 4.0)), d.p2[e]);
+    const cplx o = csub(p, cscale(cadd(d.t0[e], d.t1[e]), h2));
+    d.O[e] = mk(-c * o.y, c * o.x);
+  }
+}
+
 }  // namespace
 
 void gamma_batched(const cplx* const* lams, cplx* const* gams, cplx* const* invgams, int batch, int n,
@@ -221,6 +241,11 @@ void axpby_batched(const cplx* const* A, const cplx* const* B, cplx* const* C, c
                    int batch, int n, cudaStream_t st) {
   if (batch <= 0) return;
   axpby_kernel<<<grid_for((long long)n * n, batch), 256, 0, st>>>(A, B, C, alpha, beta, delta, n);
+  VRC_CUDA_CHECK(cudaGetLastError());
+}
+void diff_combine_batched(const DiffDesc* d, int batch, int n, cudaStream_t st) {
+  if (batch <= 0) return;
+  diff_combine_kernel<<<grid_for((long long)n * n, batch), 256, 0, st>>>(d, n);
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 void order_power_batched(const PowerDesc* d, int batch, int m, cudaStream_t st) {
