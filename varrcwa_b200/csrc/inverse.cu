@@ -189,11 +189,12 @@ __global__ void __launch_bounds__(INV_THREADS)
 // a += M X for all columns at once.
 //
 // The panel kernel holds a row (or RPT rows) per thread, so the multiplier of
-// a step is the thread's own register and a pivot passes two barriers: the
+// a step is the thread's own register and a pivot passes one barrier: the
 // candidates are compared by their upper 32 bits (a pivot within 1e-6 of the
-// largest is as good) with one warp reduction each side of the first, and the
-// pivot row is scaled by the one thread that has it before the second.  Bound
-// by that chain for few matrices and by the FP64 issue of the update for many.
+// largest is as good) with one warp reduction each side of it, and every warp's
+// candidate puts out its row and the reciprocal of its pivot before it is known
+// which one is taken.  Bound by that chain for few matrices and by the FP64
+// issue of the update for many.
 // With rows split over two threads, exchanges, and every thread reducing the
 // candidates and forming the reciprocal, a pivot took 4,700 cycles at n = 162,
 // the row moves 25,000 cycles per panel and the final column exchanges one
@@ -203,9 +204,11 @@ template <int THREADS, int RPT, int W>
 __global__ void __launch_bounds__(THREADS, 1)
     zinv_panel_kernel(cplx* const* __restrict__ mats, cplx* __restrict__ scratch, size_t per, int n, int k, int w,
                       int* __restrict__ status) {
-  __shared__ cplx s_prow[W];
-  __shared__ unsigned s_key[16];
-  __shared__ int s_row[16], s_piv[W], s_bad;
+  // every warp's candidate of a step: key, row, and its entries with the
+  // reciprocal of the first in front; two steps' worth
+  __shared__ cplx s_cand[2][16][W];
+  __shared__ unsigned s_key[2][16];
+  __shared__ int s_row[2][16], s_piv[W], s_bad;
 
   cplx* a = mats[blockIdx.x];
   cplx* M = scratch + (size_t)blockIdx.x * per;  // [w][n] (room for W)
@@ -226,53 +229,70 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int c = 0; c < W; ++c) r[q][c] = (i < n && c < w) ? a[(size_t)(k + c) * n + i] : mk(0.0, 0.0);
   }
   if (tid == 0) s_bad = 0;
-#pragma unroll
+  // The step loop stays rolled (unrolled, its code left the instruction cache:
+  // 1,590 cycles per pivot at n = 98 with two barriers): a step's column is always r[.][0], and
+  // the update writes every column one place down, the finished one last, so
+  // that W steps bring them back into order.
+#pragma unroll 1
   for (int s = 0; s < W; ++s) {
-    if (s < w) {
-      unsigned key = 0;  // rows that may be pivots have keys from 1 up
-      int row = 0;
+    if (s >= w) {  // columns beyond the matrix
 #pragma unroll
-      for (int q = 0; q < RPT; ++q)
-        if (open[q]) {
-          const unsigned kq = max(1u, (unsigned)__double2hiint(cabs1(r[q][s])));
-          if (kq > key) {
-            key = kq;
-            row = tid + q * nth;
-          }
-        }
-      const unsigned wmax = __reduce_max_sync(0xffffffffu, key);
-      const unsigned eq = __ballot_sync(0xffffffffu, key == wmax);
-      if (lane == __ffs(eq) - 1) {
-        s_key[warp] = key;
-        s_row[warp] = row;
+      for (int q = 0; q < RPT; ++q) {
+        const cplx r0 = r[q][0];
+#pragma unroll
+        for (int c = 1; c < W; ++c) r[q][c - 1] = r[q][c];
+        r[q][W - 1] = r0;
       }
-      __syncthreads();
-      const unsigned kw = lane < nwarps ? s_key[lane] : 0u;
-      const unsigned top = __reduce_max_sync(0xffffffffu, kw);
-      const int p = s_row[__ffs(__ballot_sync(0xffffffffu, kw == top)) - 1];
-      const bool bad = top <= 1u || top >= 0x7ff00000u;
+      continue;
+    }
+    unsigned key = 0;  // rows that may be pivots have keys from 1 up
+    int row = 0;
+#pragma unroll
+    for (int q = 0; q < RPT; ++q)
+      if (open[q]) {
+        const unsigned kq = max(1u, (unsigned)__double2hiint(cabs1(r[q][0])));
+        if (kq > key) {
+          key = kq;
+          row = tid + q * nth;
+        }
+      }
+    const int buf = s & 1;
+    const unsigned wmax = __reduce_max_sync(0xffffffffu, key);
+    const unsigned eq = __ballot_sync(0xffffffffu, key == wmax);
+    if (lane == __ffs(eq) - 1) {  // this warp's candidate
+      s_key[buf][warp] = key;
+      s_row[buf][warp] = row;
 #pragma unroll
       for (int q = 0; q < RPT; ++q)
-        if (p == tid + q * nth) {
-          const cplx ip = bad ? mk(1.0, 0.0) : cinv_fast(r[q][s]);
+        if (q == 0 || row == tid + q * nth) {
 #pragma unroll
-          for (int c = 0; c < W; ++c) {
-            r[q][c] = c == s ? ip : cmul(r[q][c], ip);
-            s_prow[c] = r[q][c];
-          }
-          step[q] = s;
-          open[q] = false;
-          s_piv[s] = p;
-          if (bad) s_bad = 1;
+          for (int c = 1; c < W; ++c) s_cand[buf][warp][c] = r[q][c];
+          s_cand[buf][warp][0] = (key <= 1u || key >= 0x7ff00000u) ? mk(1.0, 0.0) : cinv_fast(r[q][0]);
         }
-      __syncthreads();
+    }
+    __syncthreads();
+    const unsigned kw = lane < nwarps ? s_key[buf][lane] : 0u;
+    const unsigned top = __reduce_max_sync(0xffffffffu, kw);
+    const int ww = __ffs(__ballot_sync(0xffffffffu, kw == top)) - 1;
+    const int p = s_row[buf][ww];
+    const cplx* prow = s_cand[buf][ww];
+    const cplx ip = prow[0];
 #pragma unroll
-      for (int q = 0; q < RPT; ++q)
-        if (step[q] != s) {
-          const cplx f = mk(-r[q][s].x, -r[q][s].y);
+    for (int q = 0; q < RPT; ++q) {
+      if (p == tid + q * nth) {
 #pragma unroll
-          for (int c = 0; c < W; ++c) r[q][c] = c == s ? cmul(f, s_prow[c]) : cfma(f, s_prow[c], r[q][c]);
-        }
+        for (int c = 1; c < W; ++c) r[q][c - 1] = cmul(r[q][c], ip);
+        r[q][W - 1] = ip;
+        step[q] = s;
+        open[q] = false;
+        s_piv[s] = p;
+        if (top <= 1u || top >= 0x7ff00000u) s_bad = 1;
+      } else {
+        const cplx f = cneg(cmul(r[q][0], ip));
+#pragma unroll
+        for (int c = 1; c < W; ++c) r[q][c - 1] = cfma(f, prow[c], r[q][c]);
+        r[q][W - 1] = f;
+      }
     }
   }
 #pragma unroll
@@ -291,9 +311,14 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
   __syncthreads();
   if (tid < w) piv[k + tid] = s_piv[tid];
-  for (int e = tid; e < n * w; e += nth) {
-    const int j = e / w, s = e - j * w;
-    X[e] = (j >= k && j < k + w) ? mk(0.0, 0.0) : a[(size_t)j * n + s_piv[s]];
+  for (int j = tid; j < n; j += nth) {  // a thread per column, its gathers in flight together
+    const bool own = j >= k && j < k + w;
+    cplx x[W];
+#pragma unroll
+    for (int s = 0; s < W; ++s) x[s] = (own || s >= w) ? mk(0.0, 0.0) : a[(size_t)j * n + s_piv[s]];
+#pragma unroll
+    for (int s = 0; s < W; ++s)
+      if (s < w) X[(size_t)j * w + s] = x[s];
   }
   if (tid == 0 && status && s_bad) status[blockIdx.x] = ST_ESINGULAR;
 }
