@@ -95,3 +95,70 @@ def test_blocks(ctx, monkeypatch, call, ends, nx, ny):
         F, G = fourier_blocks(a), fourier_blocks(b)
         for k in F:
             assert np.abs(F[k] - G[k]).max() <= 1e-9 * max(np.abs(G[k]).max(), 1e-3), k
+
+
+def _taper(nx=15):
+    return st.taper_2d(norders=nx, length=0.6)
+
+
+def _waveguide(spline):
+    d = st.waveguide_pml(5, norders=5, ncontrol=4, length=0.4, spline=spline)
+    w = 0.6 + 0.05 * d["widths"]
+    d["xrules"] = [(i, zs, 2.0 + s * 0.5 * w) for (i, zs, _), s in zip(d["xrules"], (-1.0, 1.0))]
+    return d
+
+
+def _mesa():
+    """Both axes moving, half-spaces, coordinates around the origin."""
+    return dict(kind="grid", lam=1.1, nx=5, ny=7, pml=False, x=np.array([-0.5, -0.2, 0.2, 0.5]),
+                y=np.array([-0.35, -0.1, 0.1, 0.35]),
+                eps=np.array([[2.0, 2.0, 2.0], [2.0, 9.0 + 0.1j, 2.0], [2.0, 2.0, 2.0]], dtype=complex),
+                xrules=[(1, [0.0, 0.2], [-0.2, -0.24]), (2, [0.0, 0.2], [0.2, 0.24])],
+                yrules=[(1, [0.0, 0.2], [-0.1, -0.08]), (2, [0.0, 0.2], [0.1, 0.08])], z0=0.0, z1=0.2, end0=2.085,
+                end1=1.0)
+
+
+def _raster():
+    rng = np.random.default_rng(3)
+    q = rng.uniform(2.0, 8.0, (6, 5)) + 0j
+    e = np.block([[q, q[:, ::-1]], [q[::-1], q[::-1, ::-1]]])
+    return dict(kind="pixels", lam=1.0, nx=5, ny=5, pml=False, Lx=0.9, Ly=0.8, eps=e, z0=0.0, z1=0.2)
+
+
+def _almost():
+    """Symmetric at its ends and its middle only."""
+    d = _mesa()
+    d["xrules"] = [(1, [0.0, 0.05, 0.1, 0.2], [-0.2, -0.23, -0.2, -0.2]), (2, [0.0, 0.2], [0.2, 0.2])]
+    return d
+
+
+@pytest.mark.parametrize("make", [_taper, lambda: _waveguide(False), lambda: _waveguide(True), _mesa, _raster, _almost,
+                                  lambda: st.planar_taper(w0=0.5, w1=0.6, length=0.6, norders=(7, 3))])
+def test_tabulated_cells(ctx, monkeypatch, make):
+    from tests.conftest import fourier_blocks
+    d = make()
+    out = []
+    for env in (None, "1"):
+        monkeypatch.delenv("VRC_NO_FOLD", raising=False) if env is None else monkeypatch.setenv("VRC_NO_FOLD", env)
+        out.append((ctx.redheffer([d], pe=1e-2)[0], ctx.tree(0)))
+    (a, ta), (b, tb) = out
+    for k in ("status", "n", "N", "n_eig", "n_samples", "n_nodes"):
+        assert a[k] == b[k], k
+    assert [(x[0], x[1], x[3]) for x in ta] == [(x[0], x[1], x[3]) for x in tb]
+    F, G = fourier_blocks(a), fourier_blocks(b)
+    for k in F:
+        assert np.linalg.norm(F[k] - G[k]) <= 1e-9 * max(np.linalg.norm(G[k]), 1e-3), k
+
+
+def test_shifted_symmetry_takes_the_general_way(ctx, monkeypatch):
+    """Symmetric about a point that is not the lattice origin: bit for bit the
+    general way's result."""
+    d = _mesa()
+    d["x"] = d["x"] + 0.123
+    d["xrules"] = [(i, zs, [v + 0.123 for v in vals]) for i, zs, vals in d["xrules"]]
+    monkeypatch.delenv("VRC_NO_FOLD", raising=False)
+    a = ctx.redheffer([d], pe=1e-2)[0]
+    monkeypatch.setenv("VRC_NO_FOLD", "1")
+    b = ctx.redheffer([d], pe=1e-2)[0]
+    for k in ("Tdd", "Tuu", "Rud", "Rdu"):
+        assert np.array_equal(a[k], b[k])

@@ -133,6 +133,7 @@ struct Book {
           const CellSpec& c = cells[b.cell];
           fd[{c.nx, c.ny}].push_back({sr[g - g0].P, sr[g - g0].Q, b.P, b.Q, c.k0() * c.k0(), b.cell % 4});
           if (st[g - g0]) cell_status[b.cell] = st[g - g0];
+          if (!b.homog && c.kind != GEOM_PILLAR && !c.mirrored(b.z)) cell_status[b.cell] = ST_ASYMMETRIC;
         }
       for (auto& kv : fd) {
         const FoldDesc* d = E.upload(kv.second);
@@ -814,18 +815,24 @@ void Engine::order_powers(const std::vector<CellSpec>& cells, const std::vector<
   }
 }
 
-// A pillar's raster is its own mirror image along x and y, so its solve splits
-// into four parity classes of a quarter of the order each (fold.cu): an
-// eigen-decomposition costs a sixteenth of the operations.  Every other
-// structure, and a pillar whose raster turns out not to be symmetric (a pixel
-// centre within rounding of the rim), takes the general way.  Below nine
-// harmonics there is nothing to split.  Order powers: one 7 x 7-order pillar
-// 38 -> 12 ms, 16 at 11 x 11 orders 348 -> 72, 16 slices of two at 13 x 9
-// orders 59 -> 9.  On a square lattice the modes of two classes are degenerate
-// in pairs; apart in their classes, the adaptive tree no longer depends on how a
-// solver's rounding mixes them.
+// A cell that is its own mirror image along x and y splits into four parity
+// classes of a quarter of the order each (fold.cu): an eigen-decomposition costs
+// a sixteenth of the operations.  A pillar's raster is symmetric unless a pixel
+// centre lies within rounding of the rim (checked on the device, sample by
+// sample); a grid, a pixel raster or a planar section is where its coordinates
+// are, to rounding, and its table is, exactly (CellSpec::mirrored, here at three
+// heights and again at every sample).  Every other structure, and a cell found
+// asymmetric on the way, takes the general way.  Below nine harmonics there is
+// nothing to split.  General / folded: one 7 x 7-order pillar 38 / 11 ms, 16 at
+// 11 x 11 orders 348 / 71, 16 slices of two at 13 x 9 orders 59 / 9, a taper of
+// 41 orders 24.7 / 14.9, a planar taper of 11 x 5 orders 16.4 / 12.4.  On a square
+// lattice the modes of two classes are degenerate in pairs; apart in their
+// classes, the adaptive tree no longer depends on how a solver's rounding mixes
+// them.
 static bool mirror_symmetric(const CellSpec& c) {
-  return c.kind == GEOM_PILLAR && !c.pml && c.m() >= 9 && !std::getenv("VRC_NO_FOLD");
+  if (c.m() < 9 || std::getenv("VRC_NO_FOLD")) return false;
+  if (c.kind == GEOM_PILLAR) return !c.pml;
+  return c.mirrored(c.z0) && c.mirrored(0.5 * (c.z0 + c.z1)) && c.mirrored(c.z1);
 }
 
 namespace {

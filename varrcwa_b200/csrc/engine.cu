@@ -123,6 +123,40 @@ void CellSpec::geometry(double z, std::vector<double>& xo, std::vector<double>& 
   if (geom_cb) geom_cb(z, xo.data(), yo.data());
 }
 
+bool CellSpec::mirrored(double z) const {
+  if ((kind != GEOM_GRID && kind != GEOM_PIXELS && kind != GEOM_PLANAR) || geom_cb) return false;
+  std::vector<double> xs, ys;
+  std::vector<cplx> sect;
+  if (kind == GEOM_PLANAR) planar_section(z, xs, ys, &sect);
+  else geometry(z, xs, ys);
+  // ascending coordinates (crossed ones are refilled in painter's order), each
+  // the mirror image of its counterpart to rounding, about a point that is the
+  // origin up to half periods
+  auto even = [](const std::vector<double>& v) {
+    const double a = v.front(), b = v.back(), L = b - a;
+    const double tol = 2e-15 * std::max(std::fabs(a), std::fabs(b));
+    if (!(L > 0.0)) return false;
+    const double half = (a + b) / L;
+    if (std::fabs(half - std::round(half)) * L > tol) return false;
+    const size_t n = v.size();
+    for (size_t i = 0; i < n; ++i) {
+      if (i && v[i] < v[i - 1]) return false;
+      if (std::fabs((v[i] - a) - (b - v[n - 1 - i])) > tol) return false;
+    }
+    return true;
+  };
+  if (xs.size() < 2 || ys.size() < 2 || !even(xs) || !even(ys)) return false;
+  const std::vector<cplx>& e = kind == GEOM_PLANAR ? sect : eps;
+  const size_t nc = xs.size() - 1, nr = ys.size() - 1;
+  if (e.size() != nc * nr) return false;
+  for (size_t r = 0; r < nr; ++r)
+    for (size_t c = 0; c < nc; ++c) {
+      const cplx v = e[r * nc + c], x = e[r * nc + nc - 1 - c], y = e[(nr - 1 - r) * nc + c];
+      if (v.x != x.x || v.y != x.y || v.x != y.x || v.y != y.y) return false;
+    }
+  return true;
+}
+
 double CellSpec::radius(double z) const {
   double t = (z1 == z0) ? 0.0 : (z - z0) / (z1 - z0);
   return r0 + (r1 - r0) * t;

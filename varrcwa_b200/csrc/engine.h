@@ -76,6 +76,9 @@ struct CellSpec {
   double k0() const { return 2.0 * 3.1415926535897932 / lambda; }
   void geometry(double z, std::vector<double>& xo, std::vector<double>& yo) const;
   double radius(double z) const;
+  // Whether the section at z is its own mirror image along x and y about the
+  // lattice origin (rules and tables the engine evaluates itself; not pillars).
+  bool mirrored(double z) const;
 };
 
 // BOUNDARY and BOX polygons of a GDSII file's first structure, coordinates
