@@ -225,6 +225,23 @@ __device__ __forceinline__ void cpa_wait() {
 template <bool ROWOP>
 __device__ __forceinline__ void strip_rounds(cplx* p, int r0, int r1, int ra0, int ra1, const double* cs,
                                              const cplx* ss) {
+  if (__all_sync(0xffffffffu, ra0 == r0 && ra1 == r0 + QB)) {
+    // a whole chunk inside the window for all bulges: no bounds to look at
+    // (half the instructions of a round)
+    cplx x = p[0], y = p[FV];
+#pragma unroll 4
+    for (int u = 0; u < QB; ++u) {
+      const cplx nx = p[(min(u, QB - 2) + 2) * FV];
+      rotate2<ROWOP>(x, y, cs[u * NBMAX], ss[u * NBMAX]);
+      p[u * FV] = x;
+      x = y;
+      y = nx;
+      __syncwarp();
+    }
+    p[QB * FV] = x;
+    __syncwarp();
+    return;
+  }
   cplx x = mk(0.0, 0.0), y = x;
   for (int r = r0; r < r1; ++r, cs += NBMAX, ss += NBMAX) {
     if (r >= ra0 && r < ra1) {
