@@ -452,17 +452,19 @@ __device__ __forceinline__ double warp_sum(double x) {
 __device__ int aed_deflate_warp(cplx* T, cplx* U, cplx* v, cplx* ev, int nw, cplx s0, int lane, double smlnum) {
   auto t = [&](int r, int c) -> cplx& { return T[c * ALD + r]; };
   auto u = [&](int r, int c) -> cplx& { return U[c * ALD + r]; };
-  int ns = nw, ilst = 0;
+  int ns = nw;
   const double as0 = cabs1(s0);
-  for (int knt = 0; knt < nw; ++knt) {
-    double foo = cabs1(t(ns - 1, ns - 1));
+  // bottom up: an entry that looks converged is brought to the bottom of the
+  // undeflated block and tested there
+  auto converged = [&](int j) {
+    double foo = cabs1(t(j, j));
     if (foo == 0.0) foo = as0;
-    if (as0 * cabs1(u(0, ns - 1)) <= fmax(smlnum, EIG_ULP * foo)) {
-      --ns;  // converged: stays below the undeflated block
-    } else {
-      for (int k = ns - 2; k >= ilst; --k) schur_swap_warp(T, U, nw, k, lane);  // move it to position ilst
-      ++ilst;
-    }
+    return as0 * cabs1(u(0, j)) <= fmax(smlnum, EIG_ULP * foo);
+  };
+  for (int j = nw - 1; j >= 0; --j) {
+    if (!converged(j)) continue;
+    for (int k = j; k < ns - 1; ++k) schur_swap_warp(T, U, nw, k, lane);
+    if (converged(ns - 1)) --ns;
   }
   if (lane < ns) ev[lane] = t(lane, lane);
   __syncwarp();
