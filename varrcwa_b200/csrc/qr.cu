@@ -1106,21 +1106,23 @@ void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* c
     return (e && std::atoi(e) == 3) ? 3 : 2;
   }();
   auto hqr = minb == 3 ? hqr_kernel<3> : hqr_kernel<2>;
-  // order of the deflation window (VRC_QR_AEDW, 4..32): measured on B200,
-  // 12 balances the window's cost (one warp) against the sweeps it saves
+  // Order of the deflation window (VRC_QR_AEDW, 4..32) and the order of the
+  // active window from which it is taken (VRC_QR_AED; 0: never).  By default 10
+  // and 48 for n > 128, never below: ms of iteration and replay for windows of
+  // 0 / 8 / 10 / 12 / 16, n = 98 (11 matrices) 4.5 / 4.3 / 4.5 / 5.0 / 5.6, n = 162
+  // (5) 10.1 / 9.5 / 9.3 / 10.2 / 11.3, n = 162 (74) 14.7 / 13.0 / 12.7 / 13.4 /
+  // 14.5, n = 242 (8) 20.7 / 18.7 / 18.2 / 19.2 / 21.2, n = 450 (5) 71.2 / 64.2 /
+  // 56.5 / 58.2 / 61.0: a window's cost (one warp) against the sweeps it saves.
   static const int aed_w_env = [] {
     const char* e = std::getenv("VRC_QR_AEDW");
     return e ? std::min(AW, std::max(4, std::atoi(e))) : 0;
   }();
-  const int aed_w = aed_w_env ? aed_w_env : 12;
-  // aggressive early deflation on active windows of at least this order
-  // (VRC_QR_AED; 0 turns it off; by default the window's order for n > 128,
-  // off below, where the sweeps it saves cost less than the windows)
+  const int aed_w = aed_w_env ? aed_w_env : 10;
   static const int aed_env = [] {
     const char* e = std::getenv("VRC_QR_AED");
     return e ? std::max(0, std::atoi(e)) : -1;
   }();
-  const int aed_min = aed_env >= 0 ? aed_env : (n <= 128 ? 0 : aed_w);
+  const int aed_min = aed_env >= 0 ? aed_env : (n <= 128 ? 0 : 48);
   ensure_smem((const void*)hqr, QR_SMEM);
   const size_t rp_smem = replay_smem(n);
   const int rp_threads = 32 * replay_warps(n);
