@@ -46,8 +46,8 @@ namespace {
 
 constexpr int QR_THREADS = 256;
 constexpr int NBMAX = QR_THREADS / 32;           // bulges per sweep (one warp each)
-constexpr int QB = 32;                           // rounds per chunk
-constexpr int QD = QB + 3 * (NBMAX - 1) + 3;     // diagonal window size (56)
+constexpr int QB = 40;                           // rounds per chunk
+constexpr int QD = QB + 3 * (NBMAX - 1) + 3;     // diagonal window size (64: two entries per lane)
 // leading dimension of the window: odd in 16-byte units, so that the lanes
 // of a row access (stride QLD) fall in distinct shared-memory banks
 constexpr int QLD = QD + 1;
