@@ -913,9 +913,9 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
       cplx* ws = (cplx*)workspace(B * per * 16);
       // host geometry
       std::vector<double> coords((size_t)B * (2 * ncx + ncy));
-      std::vector<double> radius(B, 0.0), k0sq(B);
+      std::vector<double> k0sq(B);
+      std::vector<RasterDesc> rasters;  // pillars: one per sample
       std::vector<const cplx*> epsp(B), invp(B);
-      std::vector<cplx*> epsw(B);
       std::vector<const double*> xp(B), xsp(B), yp(B);
       std::vector<cplx> homog_eps(B);
       std::vector<std::vector<cplx>> refilled;  // keep alive until sync
@@ -958,8 +958,7 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
             if (rindex[i] != i) need = true;
           for (int i = 0; i < ncx; ++i) xso[i] = xv[index[i]];
           if (k.pillar) {
-            radius[b] = s.radius(r.z);
-            epsw[b] = base + o_eps;
+            rasters.push_back({base + o_eps, s.radius(r.z), s.Lx, s.Ly, s.eps_in, s.eps_out});
             epsp[b] = base + o_eps;
           } else if (s.kind == GEOM_PLANAR) {  // crossings come sorted: no refill
             std::vector<double> px, py;
@@ -1008,22 +1007,7 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
       std::unique_ptr<Prof> asm_prof(
           new Prof(*this, "assembly", asm_flops, asm_bytes, 12 + (k.pillar ? 1 : 0) + (gjobs.empty() ? 0 : 1)));
       if (!gjobs.empty()) grid_geometry(upload(gjobs), (int)gjobs.size(), ncx, ncy, d_eps, stream_);
-      if (k.pillar) {
-        const CellSpec& s0 = *reqs[idx[c0]].spec;
-        double* drad = upload(radius);
-        pillar_raster(drad, upload(epsw), (int)B, s0.npx, s0.npy, s0.Lx, s0.Ly, s0.eps_in, s0.eps_out, stream_);
-        // pillar cells of one group may differ in eps_in/eps_out: rasterise per
-        // distinct material pair
-        for (size_t b = 1; b < B; ++b) {
-          const CellSpec& sb = *reqs[idx[c0 + b]].spec;
-          if (sb.eps_in.x != s0.eps_in.x || sb.eps_in.y != s0.eps_in.y || sb.eps_out.x != s0.eps_out.x ||
-              sb.eps_out.y != s0.eps_out.y || sb.Lx != s0.Lx || sb.Ly != s0.Ly) {
-            std::vector<cplx*> one = {epsw[b]};
-            pillar_raster(drad + b, upload(one), 1, sb.npx, sb.npy, sb.Lx, sb.Ly, sb.eps_in, sb.eps_out, stream_);
-            ++launches;  // extra raster for a different material pair
-          }
-        }
-      }
+      if (k.pillar) pillar_raster(upload(rasters), (int)B, nc, nr, stream_);
       int* dstat = nullptr;
       if (status) {
         dstat = (int*)bytes(B * sizeof(int));

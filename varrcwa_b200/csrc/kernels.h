@@ -74,8 +74,13 @@ void trevc_batched(cplx* const* d_T, cplx* const* d_Y, int batch, int n, cudaStr
 void vecnorm_batched(cplx* const* d_X, int batch, int n, cudaStream_t st);
 
 // ---- assembly -------------------------------------------------------------------
-void pillar_raster(const double* d_radius, cplx* const* d_eps, int batch, int npx, int npy, double Lx,
-                   double Ly, cplx eps_in, cplx eps_out, cudaStream_t st);
+// one sample's circular pillar on its npy x npx raster
+struct RasterDesc {
+  cplx* eps;
+  double radius, Lx, Ly;
+  cplx eps_in, eps_out;
+};
+void pillar_raster(const RasterDesc* d, int batch, int npx, int npy, cudaStream_t st);
 // per-sample grid geometry from a structure's rule tables (one job each)
 struct GridGeomJob {
   double z;
