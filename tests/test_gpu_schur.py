@@ -32,6 +32,18 @@ def test_orders(ctx, n):
     _check(ctx, rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n)))
 
 
+@pytest.mark.parametrize("n", [2, 3, 8, 9, 32, 33, 64, 65, 94, 95, 96])
+def test_reduced_columns(ctx, n):
+    """Reflectors at the edges of the small reduction's lanes and columns,
+    with columns that need none."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((4, n, n)) + 1j * rng.standard_normal((4, n, n))
+    A[1] = np.triu(A[1], -1)
+    A[2, 2:, : n // 2] = 0
+    A[3] = np.diag(np.diagonal(A[3]))
+    _check(ctx, A)
+
+
 @pytest.mark.parametrize("scale", [1e-120, 1e-75, 1e60])
 @pytest.mark.parametrize("n", [13, 140])
 def test_scaled(ctx, n, scale):

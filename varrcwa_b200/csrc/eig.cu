@@ -195,6 +195,179 @@ __global__ void __launch_bounds__(HESS_THREADS)
   }
 }
 
+// The same reduction for n <= 95 with the matrix in shared memory, Q accumulated
+// in its place.  Eight lanes take a column (a row in eight each, the rows padded
+// with zeros to 32 NT) and the CTA 32 columns at a time: both products in one
+// pass, v^H a_j kept in registers for the update, and every warp forms the
+// reflector for itself.  A column passes three barriers (the warps' shares of
+// A v, their sum, the next reflector's column).  Bound by that chain (1.8 us per
+// column at n = 21) and, at the upper end, by the products (4.7 us at n = 82).
+// A launch at n = 61 takes 0.30 ms, with hess_kernel 0.51; one pass of sixteen pillars
+// at 11 x 11 orders takes 58.6 ms with it, 60.5 without.
+constexpr int HS_MAXN = 95;
+
+__device__ __forceinline__ cplx shfl_xor(cplx z, int o) {
+  return mk(__shfl_xor_sync(0xffffffffu, z.x, o), __shfl_xor_sync(0xffffffffu, z.y, o));
+}
+
+__device__ __forceinline__ cplx sum8(cplx z) {
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) z = cadd(z, shfl_xor(z, o));
+  return z;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(HESS_THREADS)
+    hess_smem_kernel(cplx* const* __restrict__ Hs, cplx* const* __restrict__ Zs, int n) {
+  constexpr int LD = 32 * NT, RT = 4 * NT;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx* A = reinterpret_cast<cplx*>(smem_raw);  // [n][LD]
+  cplx* yp = A + n * LD;                        // [HESS_WARPS][LD]
+  cplx* ys = yp + HESS_WARPS * LD;              // [LD]
+  cplx* taus = ys + LD;                         // [LD]
+  cplx* sp = taus + LD;                         // [HESS_WARPS]
+  cplx* H = Hs[blockIdx.x];
+  cplx* Z = Zs[blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int l8 = lane & 7, col = 4 * warp + (lane >> 3);
+  const bool b0 = lane & 8, b1 = lane & 16;
+  const cplx zero = mk(0.0, 0.0);
+  for (int c = warp; c < n; c += HESS_WARPS)
+    for (int r = lane; r < LD; r += 32) A[c * LD + r] = r < n ? H[(size_t)c * n + r] : zero;
+  __syncthreads();
+  for (int k = 0; k + 2 < n; ++k) {
+    const int j0 = k + 1;  // J = [j0, n)
+    const cplx* x = A + k * LD;
+    cplx v[RT];
+    double part = 0.0;
+#pragma unroll
+    for (int t = 0; t < RT; ++t) {
+      v[t] = x[l8 + 8 * t];
+      if (l8 + 8 * t > j0) part += cabs2(v[t]);
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    double beta;
+    cplx tau, scale;
+    householder(x[j0], part, &beta, &tau, &scale);
+    if (tid == 0) taus[k] = tau;
+    if (tau.x == 0.0 && tau.y == 0.0) continue;  // (every thread alike)
+#pragma unroll
+    for (int t = 0; t < RT; ++t) {
+      const int i = l8 + 8 * t;
+      v[t] = i > j0 ? cmul(v[t], scale) : mk(i == j0 ? 1.0 : 0.0, 0.0);
+    }
+    // shares of y = A[:, J] v and of s = v^H y, and u_j = v^H a_j
+    cplx y[RT], u[NT], vj[NT], s = zero;
+#pragma unroll
+    for (int t = 0; t < RT; ++t) y[t] = zero;
+#pragma unroll
+    for (int p = 0; p < NT; ++p) {
+      u[p] = vj[p] = zero;
+      if (j0 + 32 * p + 4 * warp < n) {  // (a warp alike)
+        const int j = j0 + 32 * p + col;
+        const cplx* a = A + min(j, n - 1) * LD + l8;
+        cplx u2[2] = {zero, zero};  // (two chains)
+        if (j < n) vj[p] = j == j0 ? mk(1.0, 0.0) : cmul(x[j], scale);
+#pragma unroll
+        for (int t = 0; t < RT; ++t) {
+          const cplx h = a[8 * t];
+          y[t] = cfma(h, vj[p], y[t]);
+          u2[t & 1] = cfma(cconj(v[t]), h, u2[t & 1]);
+        }
+        u[p] = sum8(cadd(u2[0], u2[1]));
+        s = cfma(u[p], vj[p], s);
+      }
+    }
+    // over the warp's four columns: each group of lanes ends with a row in four
+    cplx half[RT / 2];
+#pragma unroll
+    for (int q = 0; q < RT / 2; ++q)
+      half[q] = cadd(b1 ? y[2 * q + 1] : y[2 * q], shfl_xor(b1 ? y[2 * q] : y[2 * q + 1], 16));
+#pragma unroll
+    for (int q = 0; q < NT; ++q)
+      yp[warp * LD + l8 + 8 * (4 * q + 2 * b0 + b1)] =
+          cadd(b0 ? half[2 * q + 1] : half[2 * q], shfl_xor(b0 ? half[2 * q] : half[2 * q + 1], 8));
+    s = cadd(s, shfl_xor(s, 8));
+    s = cadd(s, shfl_xor(s, 16));
+    if (lane == 0) sp[warp] = s;
+    __syncthreads();
+    if (tid < LD) {
+      cplx sum = zero;
+#pragma unroll
+      for (int w = 0; w < HESS_WARPS; ++w) sum = cadd(sum, yp[w * LD + tid]);
+      ys[tid] = sum;
+    }
+    s = zero;
+#pragma unroll
+    for (int w = 0; w < HESS_WARPS; ++w) s = cadd(s, sp[w]);
+    const cplx ts = cmul(tau, s), tauc = cconj(tau);
+    if (warp == HESS_WARPS - 1 && lane < 8) {  // column k: its reflector stays below the subdiagonal
+#pragma unroll
+      for (int t = 0; t < RT; ++t)
+        if (l8 + 8 * t >= j0) A[k * LD + l8 + 8 * t] = l8 + 8 * t == j0 ? mk(beta, 0.0) : v[t];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < RT; ++t) y[t] = ys[l8 + 8 * t];
+    // rank-2 update
+#pragma unroll
+    for (int p = 0; p < NT; ++p) {
+      const int j = j0 + 32 * p + col;
+      if (j < n) {
+        cplx* a = A + j * LD + l8;
+        const cplx vc = cconj(vj[p]), tv = cmul(cneg(tau), vc),
+                   tz = cmul(tauc, csub(cmul(ts, vc), u[p]));
+#pragma unroll
+        for (int t = 0; t < RT; ++t)
+          a[8 * t] = cfma(y[t], tv, cfma(v[t], tz, a[8 * t]));
+      }
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  for (int c = warp; c < n; c += HESS_WARPS)
+    for (int r = lane; r < n; r += 32) H[(size_t)c * n + r] = r <= c + 1 ? A[c * LD + r] : zero;
+  __syncthreads();
+  // Q = H_0 H_1 ... H_(n-3) backward, in place: step k turns column k + 1 into
+  // Q's and leaves column k, which holds v_k, for the step after
+  if (tid == 0) A[(n - 1) * LD + n - 1] = mk(1.0, 0.0);
+  __syncthreads();
+  for (int k = n - 3; k >= 0; --k) {
+    const int j0 = k + 1;
+    const cplx tau = taus[k];
+    cplx v[RT];
+#pragma unroll
+    for (int t = 0; t < RT; ++t) {
+      const int i = l8 + 8 * t;
+      v[t] = i > j0 ? A[k * LD + i] : mk(i == j0 ? 1.0 : 0.0, 0.0);
+    }
+#pragma unroll
+    for (int p = 0; p < NT; ++p) {
+      if (j0 + 32 * p + 4 * warp < n) {  // (a warp alike)
+        const int j = j0 + 32 * p + col;
+        cplx* a = A + min(j, n - 1) * LD + l8;
+        cplx h[RT], w[2] = {zero, zero};
+#pragma unroll
+        for (int t = 0; t < RT; ++t) {
+          const int i = l8 + 8 * t;
+          h[t] = j == j0 ? mk(i == j0 ? 1.0 : 0.0, 0.0) : i > j0 ? a[8 * t] : zero;
+          w[t & 1] = cfma(cconj(v[t]), h[t], w[t & 1]);
+        }
+        const cplx z = sum8(cadd(w[0], w[1]));
+        const cplx tw = cneg(j == j0 ? tau : cmul(tau, z));
+#pragma unroll
+        for (int t = 0; t < RT; ++t)
+          if (j < n && l8 + 8 * t >= j0) a[8 * t] = cfma(v[t], tw, h[t]);
+      }
+    }
+    __syncthreads();
+  }
+  for (int c = warp; c < n; c += HESS_WARPS)
+    for (int r = lane; r < n; r += 32)
+      Z[(size_t)c * n + r] = (c == 0 || r == 0) ? mk(c == r ? 1.0 : 0.0, 0.0) : A[c * LD + r];
+}
+
 constexpr double ULP = EIG_ULP;
 constexpr double SMLNUM_BASE = EIG_SAFMIN;
 
@@ -264,6 +437,13 @@ __global__ void vecnorm_kernel(cplx* const* __restrict__ Xs, int n) {
 }
 
 template <int NT>
+void launch_hess_smem(cplx* const* H, cplx* const* Z, int batch, int n, cudaStream_t st) {
+  const size_t smem = ((size_t)(n + HESS_WARPS + 2) * 32 * NT + HESS_WARPS) * sizeof(cplx);
+  ensure_smem((const void*)hess_smem_kernel<NT>, smem);
+  hess_smem_kernel<NT><<<batch, HESS_THREADS, smem, st>>>(H, Z, n);
+}
+
+template <int NT>
 void launch_hess(cplx* const* H, cplx* const* Z, int batch, int n, cudaStream_t st) {
   size_t smem = (size_t)(4 + HESS_WARPS) * n * 16;
   ensure_smem((const void*)hess_kernel<NT>, smem);
@@ -278,7 +458,7 @@ void launch_hess(cplx* const* H, cplx* const* Z, int batch, int n, cudaStream_t 
 void hessenberg_batched(cplx* const* d_H, cplx* const* d_Z, int batch, int n, cudaStream_t st) {
   if (batch <= 0) return;
   // Cluster or single-CTA reduction, by measured crossovers on B200 (ms per
-  // batch, both variants): the single-CTA kernel wins for n <= 128 at every
+  // batch, both variants): a single CTA wins for n <= 128 at every
   // batch (4-9x at n = 50..98 once the batch fills the SMs, because eight
   // CTAs of a few columns each spend the reduction in cluster barriers); for
   // 128 < n <= 192 and 256 < n < 400 it wins only once the batch gives every
@@ -296,6 +476,15 @@ void hessenberg_batched(cplx* const* d_H, cplx* const* d_Z, int batch, int n, cu
                        ((n > 192 && n <= 256) || n >= 400 || !full);
   if (cluster && !std::getenv("VRC_HESS_SINGLE_CTA")) {
     hessenberg_cluster_batched(d_H, d_Z, batch, n, st);
+    return;
+  }
+  // In shared memory it takes a third to a half of hess_kernel's time at n = 21
+  // to 82, at every batch.
+  if (n <= HS_MAXN) {
+    if (n <= 32) launch_hess_smem<1>(d_H, d_Z, batch, n, st);
+    else if (n <= 64) launch_hess_smem<2>(d_H, d_Z, batch, n, st);
+    else launch_hess_smem<3>(d_H, d_Z, batch, n, st);
+    VRC_CUDA_CHECK(cudaGetLastError());
     return;
   }
   if (n <= 256) launch_hess<8>(d_H, d_Z, batch, n, st);
