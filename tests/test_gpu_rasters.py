@@ -27,6 +27,19 @@ def test_pq(ctx, npy, npx, nx, ny):
         assert relerr(P[k], oP) < 1e-12 and relerr(Q[k], oQ) < 1e-12
 
 
+@pytest.mark.parametrize("nx,ny", [(7, 9), (11, 3), (1, 13), (15, 1), (1, 17), (23, 1), (1, 25), (31, 1), (33, 1), (1, 41),
+                                   (63, 1)])
+def test_toeplitz_orders(ctx, nx, ny):
+    """The Toeplitz inverses at the edges of their widths."""
+    rng = np.random.default_rng(nx + ny)
+    eps = rng.uniform(2.0, 12.0, (2, 5, 7)) + 1j * rng.uniform(0.0, 0.5, (2, 5, 7))
+    for e in eps:
+        d = dict(kind="pixels", lam=1.1, nx=nx, ny=ny, pml=False, Lx=0.9, Ly=0.7, eps=e, z0=0.0, z1=0.4)
+        P, Q = ctx.sample_pq(d, [0.1])
+        oP, oQ = make_sampler(d).sample(0.1)
+        assert relerr(P[0], oP) < 1e-12 and relerr(Q[0], oQ) < 1e-12
+
+
 @pytest.mark.parametrize("npy,npx,nx,ny", [(7, 12, 3, 3), (12, 7, 3, 5), (9, 33, 5, 1), (16, 8, 1, 5), (10, 17, 5, 3)])
 def test_pixel_gradients(ctx, npy, npx, nx, ny):
     rng = np.random.default_rng(npx)

@@ -247,93 +247,161 @@ __global__ void __launch_bounds__(SG_THREADS)
 // ---------------------------------------------------------------------------
 // Toeplitz inverses: for each column r of F (P x nmat, P = 2t-1), build
 // T[i][k] = F[t-1+i-k][r] and write inv(T) column-major (t x t) at
-// out + r*t*t.  One warp per matrix (t <= 64, lanes own columns j and
-// j+32); Gauss-Jordan with partial pivoting, pivot search by warp shuffle.
+// out + r*t*t.  Gauss-Jordan in place with partial pivoting; rows stay where
+// they are, the pivot's row goes to all through shared memory, and the
+// permutation is undone by the stores.  Bound by the chain of one step (pivot
+// search, reciprocal, the row's way round) and, with many matrices, by the FP64
+// pipe: the strips of sixteen pillars at t = 11 take 45 us a launch, with a warp
+// per matrix in shared memory and a lane per column 118; one taper pass at
+// t = 41 spends 1.7 ms in its assembly, before 2.9.
 // ---------------------------------------------------------------------------
-constexpr int TI_WARPS = 8;
+constexpr int TI_WARPS = 4;
 constexpr int TI_MAXT = 64;
 
+// t <= T: a row per lane in registers, L lanes to a matrix.  The columns rotate
+// through the registers, so that the step's column is always the first one: the
+// loop stays rolled.
+template <int T, int L>
 __global__ void __launch_bounds__(TI_WARPS * 32)
     toeplitz_inv_kernel(const cplx* const* __restrict__ Fs, cplx* const* __restrict__ outs, int t,
                         int nmat, int* __restrict__ status) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  cplx* a = reinterpret_cast<cplx*>(smem_raw) + warp * (t * t + t);
-  cplx* fcol = a + t * t;
-  int* piv = reinterpret_cast<int*>(reinterpret_cast<cplx*>(smem_raw) + nw * (t * t + t)) + warp * TI_MAXT;
+  constexpr int PER = TI_WARPS * 32 / L;  // matrices of the CTA
+  __shared__ cplx rows[2][PER][T];
+  const int m = threadIdx.x / L, l = threadIdx.x % L, base = (threadIdx.x & 31) - l;
   const int s = blockIdx.y;
-  const int r = blockIdx.x * nw + warp;
-  if (r >= nmat) return;
-  const int P = 2 * t - 1;
-  const cplx* F = Fs[s] + (size_t)r * P;
-  for (int idx = lane; idx < t * t; idx += 32) {
-    int k = idx / t, i = idx - k * t;
-    a[k * t + i] = F[t - 1 + i - k];
-  }
-  __syncwarp();
-  bool bad = false;
+  const int r = blockIdx.x * PER + m;
+  const bool act = r < nmat && l < t;
+  const cplx* F = Fs[s] + (size_t)min(r, nmat - 1) * (2 * t - 1);
+  cplx a[T];
+#pragma unroll
+  for (int k = 0; k < T; ++k) a[k] = act && k < t ? F[t - 1 + l - k] : mk(0.0, 0.0);
+  bool used = l >= t, bad = false;
+  int step = 0, prow = 0;  // the step this row was the pivot of; lane k: the pivot of step k
   for (int k = 0; k < t; ++k) {
-    // pivot search over rows k..t-1 of column k
+    const cplx f = a[0];
+    const double v = cabs1(f);
+    double best = used ? -1.0 : v > 0.0 ? v : 0.0;
+    int p = l;
+#pragma unroll
+    for (int o = L / 2; o > 0; o >>= 1) {
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int op = __shfl_xor_sync(0xffffffffu, p, o);
+      if (ob > best || (ob == best && op < p)) {
+        best = ob;
+        p = op;
+      }
+    }
+    if (!(best > 0.0)) bad = true;
+    const bool mine = l == p;
+    if (l == k) prow = p;
+    cplx* row = rows[k & 1][m];
+    if (mine) {
+      const cplx ip = best > 0.0 ? cinv_fast(f) : mk(1.0, 0.0);
+      used = true;
+      step = k;
+      row[0] = ip;
+#pragma unroll
+      for (int j = 1; j < T; ++j) row[j] = cmul(a[j], ip);
+    }
+    __syncwarp();
+    const cplx nf = mine ? mk(0.0, 0.0) : cneg(f), z = row[0];
+#pragma unroll
+    for (int j = 1; j < T; ++j) {
+      const cplx q = row[j];
+      a[j - 1] = cfma(nf, q, mine ? q : a[j]);
+    }
+    a[T - 1] = mine ? z : cmul(nf, z);
+  }
+  // column c sits at T - t + c; this row is row `step` of the inverse, and column
+  // c belongs to the row that was the pivot of step c
+  cplx* out = outs[s] + (size_t)min(r, nmat - 1) * t * t + step;
+#pragma unroll
+  for (int q = 0; q < T; ++q) {
+    const int c = q - (T - t);
+    const int pc = __shfl_sync(0xffffffffu, prow, base + (c > 0 ? c : 0));
+    if (act && c >= 0) out[pc * t] = a[q];
+  }
+  if (bad && act && l == 0 && status) status[s] = ST_ESINGULAR;
+}
+
+// 32 < t <= TI_MAXT: a CTA per matrix in shared memory, columns over the warps
+// and rows over the lanes.  Every warp searches the pivot for itself; the step's
+// column is handed on in a buffer of its own, so a step passes one barrier.
+constexpr int TI_WIDE_WARPS = 8;
+__global__ void __launch_bounds__(TI_WIDE_WARPS * 32)
+    toeplitz_inv_wide_kernel(const cplx* const* __restrict__ Fs, cplx* const* __restrict__ outs, int t,
+                             int nmat, int* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx* a = reinterpret_cast<cplx*>(smem_raw);  // [t][TI_MAXT]
+  __shared__ cplx col[2][TI_MAXT];
+  __shared__ int prow[TI_MAXT], step[TI_MAXT];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int s = blockIdx.y, r = blockIdx.x;
+  const cplx* F = Fs[s] + (size_t)r * (2 * t - 1);
+  for (int k = warp; k < t; k += TI_WIDE_WARPS)
+#pragma unroll
+    for (int i = lane; i < TI_MAXT; i += 32) {
+      const cplx v = i < t ? F[t - 1 + i - k] : mk(0.0, 0.0);
+      a[k * TI_MAXT + i] = v;
+      if (k == 0) col[0][i] = v;
+    }
+  __syncthreads();
+  bool used[2] = {lane >= t, lane + 32 >= t}, bad = false;
+  for (int k = 0; k < t; ++k) {
+    cplx f[2];
     double best = -1.0;
-    int p = t;
-    for (int i = k + lane; i < t; i += 32) {
-      double v = cabs1(a[k * t + i]);
-      if (v > best) { best = v; p = i; }
+    int p = TI_MAXT;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      f[h] = col[k & 1][lane + 32 * h];
+      const double v = cabs1(f[h]), w = used[h] ? -1.0 : v > 0.0 ? v : 0.0;
+      if (w > best) {
+        best = w;
+        p = lane + 32 * h;
+      }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      double ob = __shfl_xor_sync(0xffffffffu, best, o);
-      int op = __shfl_xor_sync(0xffffffffu, p, o);
-      if (ob > best || (ob == best && op < p)) { best = ob; p = op; }
-    }
-    if (!(best > 0.0)) {
-      bad = true;
-      p = k;
-    }
-    if (lane == 0) piv[k] = p;
-    // swap rows k, p
-    if (p != k) {
-      for (int j = lane; j < t; j += 32) {
-        cplx tmp = a[j * t + k];
-        a[j * t + k] = a[j * t + p];
-        a[j * t + p] = tmp;
+      const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+      const int op = __shfl_xor_sync(0xffffffffu, p, o);
+      if (ob > best || (ob == best && op < p)) {
+        best = ob;
+        p = op;
       }
     }
-    __syncwarp();
-    const cplx pv = a[k * t + k];
-    const cplx ip = (best > 0.0) ? cinv(pv) : mk(1.0, 0.0);
-    for (int i = lane; i < t; i += 32) fcol[i] = a[k * t + i];
-    __syncwarp();
-    for (int j = lane; j < t; j += 32) {
-      cplx v = (j == k) ? mk(1.0, 0.0) : a[j * t + k];
-      a[j * t + k] = cmul(v, ip);
+    if (!(best > 0.0)) bad = true;
+    const cplx ip = best > 0.0 ? cinv_fast(col[k & 1][p]) : mk(1.0, 0.0);
+    if (warp == 0 && lane == 0) {
+      prow[k] = p;
+      step[p] = k;
     }
-    __syncwarp();
-    for (int j = lane; j < t; j += 32) {
-      const cplx prow = a[j * t + k];
-      for (int i = 0; i < t; ++i) {
-        if (i == k) continue;
-        cplx v = (j == k) ? mk(0.0, 0.0) : a[j * t + i];
-        a[j * t + i] = csub(v, cmul(fcol[i], prow));
+    bool mine[2];
+    cplx nf[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      mine[h] = lane + 32 * h == p;
+      used[h] = used[h] || mine[h];
+      nf[h] = mine[h] ? mk(0.0, 0.0) : cneg(f[h]);
+    }
+#pragma unroll 4
+    for (int j = warp; j < t; j += TI_WIDE_WARPS) {
+      cplx* x = a + j * TI_MAXT;
+      const cplx q = j == k ? ip : cmul(x[p], ip);
+      __syncwarp();
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;
+        const cplx v = cfma(nf[h], q, mine[h] ? q : j == k ? mk(0.0, 0.0) : x[i]);
+        x[i] = v;
+        if (j == k + 1) col[(k + 1) & 1][i] = v;
       }
     }
-    __syncwarp();
-  }
-  // undo pivoting: swap columns k <-> piv[k], k descending
-  for (int k = t - 1; k >= 0; --k) {
-    const int p = piv[k];
-    if (p != k) {
-      for (int i = lane; i < t; i += 32) {
-        cplx tmp = a[k * t + i];
-        a[k * t + i] = a[p * t + i];
-        a[p * t + i] = tmp;
-      }
-    }
-    __syncwarp();
+    __syncthreads();
   }
   cplx* out = outs[s] + (size_t)r * t * t;
-  for (int idx = lane; idx < t * t; idx += 32) out[idx] = a[idx];
-  if (bad && lane == 0 && status) status[s] = ST_ESINGULAR;
+  for (int c = warp; c < t; c += TI_WIDE_WARPS)
+    for (int i = lane; i < t; i += 32) out[prow[c] * t + step[i]] = a[c * TI_MAXT + i];
+  if (bad && threadIdx.x == 0 && status) status[s] = ST_ESINGULAR;
 }
 
 // ---------------------------------------------------------------------------
@@ -486,12 +554,25 @@ void toeplitz_inverses(const cplx* const* d_F, cplx* const* d_out, int t, int nm
                        cudaStream_t st) {
   if (batch <= 0 || nmat <= 0) return;
   if (t > TI_MAXT) throw StatusError(ST_EINVAL, "harmonics per axis must be <= 64");
-  const size_t per_warp = (size_t)(t * t + t) * 16 + TI_MAXT * sizeof(int);
-  int nw = (int)std::min<size_t>(TI_WARPS, std::max<size_t>(1, (200u << 10) / per_warp));
-  size_t smem = per_warp * nw;
-  ensure_smem((const void*)toeplitz_inv_kernel, smem);
-  dim3 grid((nmat + nw - 1) / nw, batch);
-  toeplitz_inv_kernel<<<grid, nw * 32, smem, st>>>(d_F, d_out, t, nmat, d_status);
+  const auto rows = [&](auto kernel, int lanes) {
+    const int per = TI_WARPS * 32 / lanes;
+    kernel<<<dim3((nmat + per - 1) / per, batch), TI_WARPS * 32, 0, st>>>(d_F, d_out, t, nmat, d_status);
+  };
+  if (t <= 8) {
+    rows(toeplitz_inv_kernel<8, 8>, 8);
+  } else if (t <= 12) {
+    rows(toeplitz_inv_kernel<12, 16>, 16);
+  } else if (t <= 16) {
+    rows(toeplitz_inv_kernel<16, 16>, 16);
+  } else if (t <= 24) {
+    rows(toeplitz_inv_kernel<24, 32>, 32);
+  } else if (t <= 32) {
+    rows(toeplitz_inv_kernel<32, 32>, 32);
+  } else {
+    const size_t smem = (size_t)t * TI_MAXT * sizeof(cplx);
+    ensure_smem((const void*)toeplitz_inv_wide_kernel, smem);
+    toeplitz_inv_wide_kernel<<<dim3(nmat, batch), TI_WIDE_WARPS * 32, smem, st>>>(d_F, d_out, t, nmat, d_status);
+  }
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 
