@@ -63,3 +63,18 @@ def test_structured(ctx, n):
     block[: n // 2, : n // 2] += np.tril(G[: n // 2, : n // 2], -1)
     shift = np.roll(np.eye(n), 1, axis=0).astype(complex)
     _check(ctx, np.stack([graded, diag, block, shift]))
+
+
+@pytest.mark.parametrize("n", [2, 18, 70, 150])
+def test_equal_diagonals(ctx, n):
+    """Multiple eigenvalues up to rounding: the modes of a uniform medium, and
+    blocks with equal diagonal entries whose off-diagonal product is below
+    their rounding."""
+    rng = np.random.default_rng(n)
+    d = -2e4 * np.repeat(rng.uniform(0.1, 1.0, n // 2), 2)
+    A = np.tile(np.diag(d).astype(complex), (12, 1, 1))
+    A[:8] += 2e-12 * rng.standard_normal((8, n, n))
+    i = np.arange(0, n, 2)
+    A[8:, i, i + 1] = -1.85e-12 * 10.0 ** rng.uniform(-1, 1, (4, n // 2))
+    A[8:, i + 1, i] = -1.05e-13 * 10.0 ** rng.uniform(-1, 1, (4, n // 2))
+    _check(ctx, A)

@@ -282,7 +282,10 @@ constexpr int ALD = AW + 1;  // its leading dimension in shared memory (odd in 1
 
 // Negligible subdiagonal entry sub = T[k][k-1] between the diagonal entries
 // dkm = T[k-1][k-1] and dk = T[k][k], with sup = T[k-1][k] and the
-// neighbouring subdiagonals below and above (Ahues-Tisseur, LAPACK xLAHQR).
+// neighbouring subdiagonals below and above (Ahues-Tisseur, LAPACK xLAHQR).  The
+// diagonal entries count as apart by their rounding at least: with equal ones
+// and sub sup below its square the shift rounds to the diagonal and a step only
+// exchanges the two, for ever.
 __device__ __forceinline__ bool negligible(cplx sub, cplx dkm, cplx dk, cplx sup, cplx sub_up, cplx sub_dn,
                                            double smlnum) {
   const double cs = cabs1(sub);
@@ -294,7 +297,7 @@ __device__ __forceinline__ bool negligible(cplx sub, cplx dkm, cplx dk, cplx sup
   const double ab = fmax(cs, a2), ba = fmin(cs, a2);
   const double b1 = cabs1(dk), b2 = cabs1(csub(dkm, dk));
   const double aa = fmax(b1, b2), bb = fmin(b1, b2);
-  return ba * ab <= fmax(smlnum * (aa + ab), EIG_ULP * (bb * aa));
+  return ba * ab <= fmax(smlnum * (aa + ab), EIG_ULP * aa * fmax(bb, EIG_ULP * aa));
 }
 __device__ __forceinline__ bool small_negligible(const cplx* T, int nw, int k, double smlnum) {
   auto t = [&](int r, int c) { return T[c * ALD + r]; };
