@@ -30,6 +30,33 @@ def test_orders(ctx, n):
     _check(ctx, rng.standard_normal((2, n, n)) + 1j * rng.standard_normal((2, n, n)))
 
 
+@pytest.mark.parametrize("n", [2, 3, 7, 8, 9, 30, 63, 66, 95, 96, 97])
+def test_small_orders(ctx, n):
+    """The registers' edges, more matrices than one wave takes."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((300, n, n)) + 1j * rng.standard_normal((300, n, n))
+    A[:, np.arange(n), np.arange(n)] += 2.0 * n
+    _check(ctx, A)
+
+
+@pytest.mark.parametrize("n", [2, 20, 63, 90])
+def test_small_pivots(ctx, n):
+    """Pivots far from the diagonal and far from one; singular, infinite and
+    undefined entries are reported for their own matrix alone."""
+    rng = np.random.default_rng(n)
+    G = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    P = np.eye(n)[::-1] * rng.uniform(0.5, 2.0, n)[:, None] + 0j
+    for A in (P, P + 1e-3 * G, 1e-160 * G, 1e160 * G):
+        X, st = ctx.zinv(A)
+        bound = 50 * 2.2e-16 * n * np.linalg.cond(A / np.abs(A).max())
+        assert st == 0 and np.abs(A @ X - np.eye(n)).max() < bound
+    A = np.stack([G] * 5)
+    A[1, :, 0] = 0.0
+    A[2, 1, 0] = np.inf
+    A[3, :, 0] = np.nan
+    assert list(ctx.zinv(A)[1]) == [0, 4, 4, 4, 0]
+
+
 @pytest.mark.parametrize("n", [40, 70, 300, 530])
 def test_far_pivots(ctx, n):
     """A scaled permutation (every pivot off the diagonal), and rows of very

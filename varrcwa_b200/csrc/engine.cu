@@ -527,7 +527,7 @@ void Engine::inverse(const std::vector<cplx*>& mats, int n, std::vector<int>* st
   {
     const double nn3 = (double)n * n * n;
     const int W = zinv_blocked_width(n);
-    if (n >= 2 * W && !std::getenv("VRC_ZINV_SINGLE_CTA")) {
+    if (n > zinv_small_maxn()) {
       // blocked: rank-W updates on the tensor cores, in chunks of a fixed
       // number of matrices so that the scratch block is reused
       const size_t per = zinv_blocked_scratch(n);
@@ -547,7 +547,7 @@ void Engine::inverse(const std::vector<cplx*>& mats, int n, std::vector<int>* st
       free_bytes(scr, CH * per);
     } else {
       Prof pr(*this, "zinv", 8.0 * nn3 * mats.size(), 32.0 * n * (double)n * mats.size());
-      zinv_batched(dm, (int)mats.size(), n, dst, stream_);
+      zinv_small_batched(dm, (int)mats.size(), n, dst, stream_);
     }
   }
   if (status) {

@@ -1,181 +1,152 @@
-// Batched in-place matrix inversion: blocked Gauss-Jordan with partial
-// (row) pivoting, one CTA per matrix.
+// Batched in-place matrix inversion: Gauss-Jordan with partial (row) pivoting.
 //
 // The reference inverts through Eigen PartialPivLU (explicit inverse of
 // I - rdu*Rud, src/core/RedhefferIntegrator.cpp:267-270) and uses LU solves
 // elsewhere; here every W^{-1}X / M^{-1}X of the hot path is an explicit
 // inverse followed by a tensor-core GEMM (same 8n^3 flops as getrf+getrs).
 //
-// Blocking: a panel of nb columns is reduced in shared memory (pivot search
-// by warp-shuffle max reduction); the nb accumulated row operations are then
-// applied to every other column as one rank-nb update
-//     a[:, j] <- P a[:, j];  a[:, j] += (Tp - E) a[k:k+nb, j]
-// so the matrix is streamed once per panel instead of once per pivot.
-#include <cstdlib>
-
+// Small matrices stay in one CTA's registers; larger ones are reduced a panel
+// at a time, the panel's accumulated row operations applied to every other
+// column as one rank-w update on the tensor cores.
 #include "common.cuh"
 #include "kernels.h"
 
 namespace vrc {
 namespace {
 
-constexpr int INV_THREADS = 512;
+// ---------------------------------------------------------------------------
+// n <= 96: one CTA per matrix, the matrix in registers (rows over the lanes,
+// columns over the warps).  Rows are never exchanged: step k takes as pivot row
+// the largest entry of column k among the rows not yet used, and the permutation
+// comes out with the stores.  A step passes one barrier: the warp that owns the
+// next column updates it first, finds its pivot and the reciprocal while the
+// others still update, and hands all three on through shared memory; the pivot's
+// row comes from the lane that holds it.  Bound by the chain of a step (row,
+// update of a column, search, reciprocal: 0.7 us at n = 25, 1.1 at 96) for few
+// matrices, by the FP64 pipe for many.
+// ---------------------------------------------------------------------------
+constexpr int ZS_MAXN = 96;
 
-struct PivotCand {
-  double v;
-  int i;
-};
+// bits of infinity, 1e-150 and 1e150
+constexpr unsigned long long INF_BITS = 0x7ff0000000000000ull, MID_LO = 0x20ca2fe76a3f9475ull,
+                             MID_HI = 0x5f138d352e5096afull;
 
-__device__ __forceinline__ PivotCand warp_argmax(PivotCand c) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    double ov = __shfl_xor_sync(0xffffffffu, c.v, o);
-    int oi = __shfl_xor_sync(0xffffffffu, c.i, o);
-    if (ov > c.v || (ov == c.v && oi < c.i)) {
-      c.v = ov;
-      c.i = oi;
-    }
-  }
-  return c;
+__device__ __forceinline__ cplx cinv_mid(cplx b) {  // the plain form of cinv_fast
+  const double r = 1.0 / (b.x * b.x + b.y * b.y);
+  return mk(b.x * r, -b.y * r);
 }
 
-__global__ void __launch_bounds__(INV_THREADS)
-    zinv_kernel(cplx* const* __restrict__ mats, int n, int nb, int* __restrict__ status) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx* panel = reinterpret_cast<cplx*>(smem_raw);  // [nb][n] column-major panel
-  cplx* fcol = panel + (size_t)nb * n;                       // [n] multipliers
-  int* piv = reinterpret_cast<int*>(fcol + n);                // [n]
-  __shared__ PivotCand red[INV_THREADS / 32];
-  __shared__ cplx s_inv;
-  __shared__ int s_p;
-  __shared__ int s_bad;
-
-  cplx* a = mats[blockIdx.x];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nwarps = INV_THREADS / 32;
-  if (tid == 0) s_bad = 0;
-
-  for (int k = 0; k < n; k += nb) {
-    const int w = min(nb, n - k);
-    // Load panel columns k..k+w-1.
-    for (int idx = tid; idx < w * n; idx += INV_THREADS) {
-      int c = idx / n, r = idx - c * n;
-      panel[c * n + r] = a[(size_t)(k + c) * n + r];
-    }
-    __syncthreads();
-    for (int s = 0; s < w; ++s) {
-      const int r0 = k + s;
-      cplx* col = panel + s * n;
-      // Pivot search over rows >= r0 (|re|+|im|, as izamax).
-      PivotCand c{-1.0, n};
-      for (int i = r0 + tid; i < n; i += INV_THREADS) {
-        double v = cabs1(col[i]);
-        if (v > c.v) { c.v = v; c.i = i; }
-      }
-      c = warp_argmax(c);
-      if (lane == 0) red[warp] = c;
-      __syncthreads();
-      if (warp == 0) {
-        PivotCand cc = lane < nwarps ? red[lane] : PivotCand{-1.0, n};
-        cc = warp_argmax(cc);
-        if (lane == 0) {
-          int p = cc.i;
-          cplx pv = col[p];
-          if (!(cc.v > 0.0) || !isfinite(cc.v)) {
-            s_bad = 1;
-            pv = mk(1.0, 0.0);
-            p = r0;
-          }
-          s_p = p;
-          s_inv = cinv(pv);
-          piv[r0] = p;
-        }
-      }
-      __syncthreads();
-      const int p = s_p;
-      const cplx ip = s_inv;
-      // Swap rows r0 and p inside the panel.
-      if (p != r0) {
-        for (int c2 = tid; c2 < w; c2 += INV_THREADS) {
-          cplx t = panel[c2 * n + r0];
-          panel[c2 * n + r0] = panel[c2 * n + p];
-          panel[c2 * n + p] = t;
-        }
-      }
-      __syncthreads();
-      // Save the multipliers (column s), then scale the pivot row:
-      // a[r0][s] := 1, row *= 1/piv.
-      for (int i = tid; i < n; i += INV_THREADS) fcol[i] = col[i];
-      __syncthreads();
-      for (int c2 = tid; c2 < w; c2 += INV_THREADS) {
-        cplx v = (c2 == s) ? mk(1.0, 0.0) : panel[c2 * n + r0];
-        panel[c2 * n + r0] = cmul(v, ip);
-      }
-      __syncthreads();
-      // Eliminate column s from the other rows (panel columns only).
-      for (int idx = tid; idx < n * w; idx += INV_THREADS) {
-        int c2 = idx / n, i = idx - c2 * n;
-        if (i == r0) continue;
-        cplx prow = panel[c2 * n + r0];
-        cplx v = (c2 == s) ? mk(0.0, 0.0) : panel[c2 * n + i];
-        panel[c2 * n + i] = csub(v, cmul(fcol[i], prow));
-      }
-      __syncthreads();
-    }
-    // Write the panel back.
-    for (int idx = tid; idx < w * n; idx += INV_THREADS) {
-      int c = idx / n, r = idx - c * n;
-      a[(size_t)(k + c) * n + r] = panel[c * n + r];
-    }
-    // Rank-w update of all other columns: one warp per column.
-    for (int j = warp; j < n; j += nwarps) {
-      if (j >= k && j < k + w) continue;
-      cplx* colj = a + (size_t)j * n;
-      // Row swaps in order.
-      if (lane == 0) {
-        for (int s = 0; s < w; ++s) {
-          int p = piv[k + s];
-          if (p != k + s) {
-            cplx t = colj[k + s];
-            colj[k + s] = colj[p];
-            colj[p] = t;
-          }
-        }
-      }
-      __syncwarp();
-      cplx x[16];
+template <int R, int W>
+__global__ void __launch_bounds__(32 * W)
+    zinv_small_kernel(cplx* const* __restrict__ mats, int n, int* __restrict__ status) {
+  constexpr int C = 32 * R / W;  // columns of a warp: W c + warp
+  __shared__ cplx col[2][32 * R], row[W][C], inv[2];
+  __shared__ int prow[32 * R];
+  cplx* g = mats[blockIdx.x];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const cplx zero = mk(0.0, 0.0);
+  cplx a[R][C], x[R];
+  bool used[R], bad = false;
+  int step[R];  // the step that this row was the pivot of
+  // the largest |re| + |im| of column k in x, by its high word, then its low
+  // word; meanwhile each lane takes the reciprocal of its own candidate
+  const auto search = [&](int k) {
+    cplx xb = zero;
+    unsigned long long best = 0;  // 1 + the bits of the candidate (as integers they order alike)
+    int hb = 0;
 #pragma unroll
-      for (int s = 0; s < 16; ++s) x[s] = (s < w) ? colj[k + s] : mk(0.0, 0.0);
-      __syncwarp();
-      for (int i = lane; i < n; i += 32) {
-        cplx v = colj[i];
-        cplx acc = mk(0.0, 0.0);
+    for (int h = 0; h < R; ++h) {
+      col[k & 1][lane + 32 * h] = x[h];
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(cabs1(x[h]));
+      const unsigned long long key = used[h] ? 0 : bits > INF_BITS ? 1 : bits + 1;  // (a NaN counts as zero)
+      if (key > best) {
+        best = key;
+        xb = x[h];
+        hb = h;
+      }
+    }
+    const bool ok = best > 1 && best <= INF_BITS;
+    const cplx ib = best - MID_LO < MID_HI - MID_LO ? cinv_mid(xb) : ok ? cinv(xb) : mk(1.0, 0.0);
+    const unsigned hi = (unsigned)(best >> 32), lo = (unsigned)best;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    const int p = __ffs(__ballot_sync(0xffffffffu, hi == mh && lo == ml)) - 1;
+    if (lane == p) {
+      inv[k & 1] = ib;
+      prow[k] = lane + 32 * hb;
+      if (!ok) bad = true;
+    }
+  };
 #pragma unroll
-        for (int s = 0; s < 16; ++s) {
-          if (s < w) {
-            cplx t = panel[s * n + i];
-            if (i == k + s) t.x -= 1.0;
-            acc = cfma(t, x[s], acc);
+  for (int h = 0; h < R; ++h) {
+    const int i = lane + 32 * h;
+    used[h] = i >= n;
+    step[h] = 0;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const int j = W * c + warp;
+      a[h][c] = i < n && j < n ? g[(size_t)j * n + i] : zero;
+    }
+    x[h] = a[h][0];
+  }
+  if (warp == 0) search(0);
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    for (int w = 0; w < W; ++w) {
+      const int k = W * c + w;
+      if (k >= n) break;
+      const int p = prow[k];
+      const cplx ip = inv[k & 1];
+      cplx nf[R];
+#pragma unroll
+      for (int h = 0; h < R; ++h) nf[h] = lane + 32 * h == p ? ip : cneg(cmul(col[k & 1][lane + 32 * h], ip));
+      // the pivot's row, left empty (its lane adds 1 / pivot times it below)
+#pragma unroll
+      for (int h = 0; h < R; ++h) {
+          const bool mine = lane + 32 * h == p;
+          if (R > 1 && !__any_sync(0xffffffffu, mine)) continue;
+          if (mine) {
+#pragma unroll
+            for (int d = 0; d < C; ++d) row[warp][d] = a[h][d];
           }
+#pragma unroll
+          for (int d = 0; d < C; ++d) a[h][d] = mine ? zero : a[h][d];
+          used[h] = used[h] || mine;
+          step[h] = mine ? k : step[h];
         }
-        colj[i] = cadd(v, acc);
+      __syncwarp();
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) {
+        const int d = (c + cc) % C;
+        const cplx q = row[warp][d];
+#pragma unroll
+        for (int h = 0; h < R; ++h) a[h][d] = cfma(nf[h], q, a[h][d]);
+        if (cc == 0 ? warp == w + 1 : cc == 1 && warp == 0 && w == W - 1) {
+#pragma unroll
+          for (int h = 0; h < R; ++h) x[h] = a[h][d];
+          if (k + 1 < n) search(k + 1);
+        }
       }
-    }
-    __syncthreads();
-  }
-  // Undo the row interchanges as column interchanges, in reverse order.
-  for (int k = n - 1; k >= 0; --k) {
-    int p = piv[k];
-    if (p != k) {
-      for (int i = tid; i < n; i += INV_THREADS) {
-        cplx t = a[(size_t)k * n + i];
-        a[(size_t)k * n + i] = a[(size_t)p * n + i];
-        a[(size_t)p * n + i] = t;
+      if (warp == w) {
+#pragma unroll
+        for (int h = 0; h < R; ++h) a[h][c] = nf[h];
       }
+      __syncthreads();
     }
-    __syncthreads();
   }
-  if (tid == 0 && status && s_bad) status[blockIdx.x] = ST_ESINGULAR;
+  // inverse(step of a row, pivot row of a column)
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int j = W * c + warp;
+    if (j < n) {
+      cplx* o = g + (size_t)prow[j] * n;
+#pragma unroll
+      for (int h = 0; h < R; ++h)
+        if (lane + 32 * h < n) o[step[h]] = a[h][c];
+    }
+  }
+  if (bad && status) status[blockIdx.x] = ST_ESINGULAR;
 }
 
 // ---------------------------------------------------------------------------
@@ -352,11 +323,18 @@ __global__ void __launch_bounds__(PERM_THREADS)
 
 }  // namespace
 
-int zinv_panel_width(int n) {
-  // panel (nb x n complex) + pivots must fit comfortably in shared memory.
-  int nb = 16;
-  while (nb > 1 && (size_t)(nb + 1) * n * 16 + (size_t)n * 4 > 200 * 1024) nb >>= 1;
-  return nb;
+// One launch up to here, panels and updates above.  Measured, small against
+// blocked, 1 / 148 / 600 matrices: n = 25 19 / 21 / 27 us against 52 / 56 / 124,
+// n = 49 50 / 52 / 164 against 95 / 112 / 307, n = 96 109 / 115 / 548 against
+// 153 / 251 / 880.  Four rows a lane would not fit the register file.
+int zinv_small_maxn() { return ZS_MAXN; }
+
+void zinv_small_batched(cplx* const* d_mats, int batch, int n, int* d_status, cudaStream_t stream) {
+  if (batch <= 0) return;
+  if (n <= 32) zinv_small_kernel<1, 4><<<batch, 128, 0, stream>>>(d_mats, n, d_status);
+  else if (n <= 64) zinv_small_kernel<2, 8><<<batch, 256, 0, stream>>>(d_mats, n, d_status);
+  else zinv_small_kernel<3, 16><<<batch, 512, 0, stream>>>(d_mats, n, d_status);
+  VRC_CUDA_CHECK(cudaGetLastError());
 }
 
 // Panel columns: what a thread's registers hold with a row per thread up to
@@ -397,19 +375,6 @@ void zinv_blocked_batched(cplx* const* d_mats, int batch, int n, int* d_status, 
     const dim3 grid((n + 3) / 4, nb);
     zinv_permute_kernel<false><<<grid, PERM_THREADS, psm, stream>>>(d_mats + b0, sb, per, n, W);
     zinv_permute_kernel<true><<<grid, PERM_THREADS, psm, stream>>>(d_mats + b0, sb, per, n, W);
-  }
-  VRC_CUDA_CHECK(cudaGetLastError());
-}
-
-void zinv_batched(cplx* const* d_mats, int batch, int n, int* d_status, cudaStream_t stream) {
-  if (batch <= 0) return;
-  int nb = zinv_panel_width(n);
-  size_t smem = (size_t)(nb + 1) * n * 16 + (size_t)n * 4;
-  ensure_smem((const void*)zinv_kernel, smem);
-  for (int b0 = 0; b0 < batch; b0 += 65535) {
-    int nbat = batch - b0 < 65535 ? batch - b0 : 65535;
-    zinv_kernel<<<nbat, INV_THREADS, smem, stream>>>(d_mats + b0, n, nb,
-                                                      d_status ? d_status + b0 : nullptr);
   }
   VRC_CUDA_CHECK(cudaGetLastError());
 }

@@ -36,9 +36,9 @@ void zgemm_rect_batched(const GemmDesc* d_descs, int batch, int M, int N, int K,
                         cplx alpha, cplx beta, cudaStream_t stream, int opA = 0, int opB = 0, int tile = 0);
 
 // ---- inverse (in place) -------------------------------------------------------
-int zinv_panel_width(int n);
-void zinv_batched(cplx* const* d_mats, int batch, int n, int* d_status, cudaStream_t stream);
-// Blocked inversion with the rank-w updates as tensor-core GEMMs.  scratch:
+int zinv_small_maxn();
+void zinv_small_batched(cplx* const* d_mats, int batch, int n, int* d_status, cudaStream_t stream);
+// Above zinv_small_maxn(): blocked inversion with the rank-w updates as tensor-core GEMMs.  scratch:
 // zinv_blocked_scratch(n) bytes per matrix; d_descs[b] = {M_b, M_b + n W,
 // mat_b, mat_b} with M_b = scratch + b * zinv_blocked_scratch(n) and
 // W = zinv_blocked_width(n).
