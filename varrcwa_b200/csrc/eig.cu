@@ -195,16 +195,16 @@ __global__ void __launch_bounds__(HESS_THREADS)
   }
 }
 
-// The same reduction for n <= 95 with the matrix in shared memory, Q accumulated
+// The same reduction for n <= 112 with the matrix in shared memory, Q accumulated
 // in its place.  Eight lanes take a column (a row in eight each, the rows padded
-// with zeros to 32 NT) and the CTA 32 columns at a time: both products in one
+// with zeros to 8 RV) and the CTA 32 columns at a time: both products in one
 // pass, v^H a_j kept in registers for the update, and every warp forms the
 // reflector for itself.  A column passes three barriers (the warps' shares of
-// A v, their sum, the next reflector's column).  Bound by that chain (1.8 us per
-// column at n = 21) and, at the upper end, by the products (4.7 us at n = 82).
-// A launch at n = 61 takes 0.30 ms, with hess_kernel 0.51; one pass of sixteen pillars
-// at 11 x 11 orders takes 58.6 ms with it, 60.5 without.
-constexpr int HS_MAXN = 95;
+// A v, their sum, the next reflector's column).  Bound by that chain and, with
+// the SMs full, by shared memory and the FP64 pipe.  One / 600 matrices take
+// 0.11 / 0.37 ms at n = 42, 0.21 / 0.73 at 61 (hess_kernel 0.51 for some 60) and
+// 0.58 / 2.9 at 98 (panels and GEMM updates 0.93 / 4.1).
+constexpr int HS_MAXN = 112;  // (what shared memory holds)
 
 __device__ __forceinline__ cplx shfl_xor(cplx z, int o) {
   return mk(__shfl_xor_sync(0xffffffffu, z.x, o), __shfl_xor_sync(0xffffffffu, z.y, o));
@@ -216,10 +216,10 @@ __device__ __forceinline__ cplx sum8(cplx z) {
   return z;
 }
 
-template <int NT>
-__global__ void __launch_bounds__(HESS_THREADS)
+template <int RV>
+__global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
     hess_smem_kernel(cplx* const* __restrict__ Hs, cplx* const* __restrict__ Zs, int n) {
-  constexpr int LD = 32 * NT, RT = 4 * NT;
+  constexpr int LD = 8 * RV, RT = (RV + 3) / 4 * 4, NT = RT / 4;  // rows and column passes of a lane
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* A = reinterpret_cast<cplx*>(smem_raw);  // [n][LD]
   cplx* yp = A + n * LD;                        // [HESS_WARPS][LD]
@@ -238,22 +238,23 @@ __global__ void __launch_bounds__(HESS_THREADS)
   for (int k = 0; k + 2 < n; ++k) {
     const int j0 = k + 1;  // J = [j0, n)
     const cplx* x = A + k * LD;
-    cplx v[RT];
-    double part = 0.0;
+    cplx v[RV];
+    double part[2] = {0.0, 0.0};
 #pragma unroll
-    for (int t = 0; t < RT; ++t) {
+    for (int t = 0; t < RV; ++t) {
       v[t] = x[l8 + 8 * t];
-      if (l8 + 8 * t > j0) part += cabs2(v[t]);
+      if (l8 + 8 * t > j0) part[t & 1] += cabs2(v[t]);
     }
+    double x2 = part[0] + part[1];
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    for (int o = 1; o < 8; o <<= 1) x2 += __shfl_xor_sync(0xffffffffu, x2, o);
     double beta;
     cplx tau, scale;
-    householder(x[j0], part, &beta, &tau, &scale);
+    householder(x[j0], x2, &beta, &tau, &scale);
     if (tid == 0) taus[k] = tau;
     if (tau.x == 0.0 && tau.y == 0.0) continue;  // (every thread alike)
 #pragma unroll
-    for (int t = 0; t < RT; ++t) {
+    for (int t = 0; t < RV; ++t) {
       const int i = l8 + 8 * t;
       v[t] = i > j0 ? cmul(v[t], scale) : mk(i == j0 ? 1.0 : 0.0, 0.0);
     }
@@ -270,7 +271,7 @@ __global__ void __launch_bounds__(HESS_THREADS)
         cplx u2[2] = {zero, zero};  // (two chains)
         if (j < n) vj[p] = j == j0 ? mk(1.0, 0.0) : cmul(x[j], scale);
 #pragma unroll
-        for (int t = 0; t < RT; ++t) {
+        for (int t = 0; t < RV; ++t) {
           const cplx h = a[8 * t];
           y[t] = cfma(h, vj[p], y[t]);
           u2[t & 1] = cfma(cconj(v[t]), h, u2[t & 1]);
@@ -285,9 +286,12 @@ __global__ void __launch_bounds__(HESS_THREADS)
     for (int q = 0; q < RT / 2; ++q)
       half[q] = cadd(b1 ? y[2 * q + 1] : y[2 * q], shfl_xor(b1 ? y[2 * q] : y[2 * q + 1], 16));
 #pragma unroll
-    for (int q = 0; q < NT; ++q)
-      yp[warp * LD + l8 + 8 * (4 * q + 2 * b0 + b1)] =
+    for (int q = 0; q < NT; ++q) {
+      const int t = 4 * q + 2 * b0 + b1;
+      const cplx z =
           cadd(b0 ? half[2 * q + 1] : half[2 * q], shfl_xor(b0 ? half[2 * q] : half[2 * q + 1], 8));
+      if (t < RV) yp[warp * LD + l8 + 8 * t] = z;
+    }
     s = cadd(s, shfl_xor(s, 8));
     s = cadd(s, shfl_xor(s, 16));
     if (lane == 0) sp[warp] = s;
@@ -304,12 +308,12 @@ __global__ void __launch_bounds__(HESS_THREADS)
     const cplx ts = cmul(tau, s), tauc = cconj(tau);
     if (warp == HESS_WARPS - 1 && lane < 8) {  // column k: its reflector stays below the subdiagonal
 #pragma unroll
-      for (int t = 0; t < RT; ++t)
+      for (int t = 0; t < RV; ++t)
         if (l8 + 8 * t >= j0) A[k * LD + l8 + 8 * t] = l8 + 8 * t == j0 ? mk(beta, 0.0) : v[t];
     }
     __syncthreads();
 #pragma unroll
-    for (int t = 0; t < RT; ++t) y[t] = ys[l8 + 8 * t];
+    for (int t = 0; t < RV; ++t) y[t] = ys[l8 + 8 * t];
     // rank-2 update
 #pragma unroll
     for (int p = 0; p < NT; ++p) {
@@ -319,7 +323,7 @@ __global__ void __launch_bounds__(HESS_THREADS)
         const cplx vc = cconj(vj[p]), tv = cmul(cneg(tau), vc),
                    tz = cmul(tauc, csub(cmul(ts, vc), u[p]));
 #pragma unroll
-        for (int t = 0; t < RT; ++t)
+        for (int t = 0; t < RV; ++t)
           a[8 * t] = cfma(y[t], tv, cfma(v[t], tz, a[8 * t]));
       }
     }
@@ -336,9 +340,9 @@ __global__ void __launch_bounds__(HESS_THREADS)
   for (int k = n - 3; k >= 0; --k) {
     const int j0 = k + 1;
     const cplx tau = taus[k];
-    cplx v[RT];
+    cplx v[RV];
 #pragma unroll
-    for (int t = 0; t < RT; ++t) {
+    for (int t = 0; t < RV; ++t) {
       const int i = l8 + 8 * t;
       v[t] = i > j0 ? A[k * LD + i] : mk(i == j0 ? 1.0 : 0.0, 0.0);
     }
@@ -347,9 +351,9 @@ __global__ void __launch_bounds__(HESS_THREADS)
       if (j0 + 32 * p + 4 * warp < n) {  // (a warp alike)
         const int j = j0 + 32 * p + col;
         cplx* a = A + min(j, n - 1) * LD + l8;
-        cplx h[RT], w[2] = {zero, zero};
+        cplx h[RV], w[2] = {zero, zero};
 #pragma unroll
-        for (int t = 0; t < RT; ++t) {
+        for (int t = 0; t < RV; ++t) {
           const int i = l8 + 8 * t;
           h[t] = j == j0 ? mk(i == j0 ? 1.0 : 0.0, 0.0) : i > j0 ? a[8 * t] : zero;
           w[t & 1] = cfma(cconj(v[t]), h[t], w[t & 1]);
@@ -357,7 +361,7 @@ __global__ void __launch_bounds__(HESS_THREADS)
         const cplx z = sum8(cadd(w[0], w[1]));
         const cplx tw = cneg(j == j0 ? tau : cmul(tau, z));
 #pragma unroll
-        for (int t = 0; t < RT; ++t)
+        for (int t = 0; t < RV; ++t)
           if (j < n && l8 + 8 * t >= j0) a[8 * t] = cfma(v[t], tw, h[t]);
       }
     }
@@ -436,11 +440,11 @@ __global__ void vecnorm_kernel(cplx* const* __restrict__ Xs, int n) {
   if (lane == 0) x[bi] = mk(x[bi].x, 0.0);
 }
 
-template <int NT>
+template <int RV>
 void launch_hess_smem(cplx* const* H, cplx* const* Z, int batch, int n, cudaStream_t st) {
-  const size_t smem = ((size_t)(n + HESS_WARPS + 2) * 32 * NT + HESS_WARPS) * sizeof(cplx);
-  ensure_smem((const void*)hess_smem_kernel<NT>, smem);
-  hess_smem_kernel<NT><<<batch, HESS_THREADS, smem, st>>>(H, Z, n);
+  const size_t smem = ((size_t)(n + HESS_WARPS + 2) * 8 * RV + HESS_WARPS) * sizeof(cplx);
+  ensure_smem((const void*)hess_smem_kernel<RV>, smem);
+  hess_smem_kernel<RV><<<batch, HESS_THREADS, smem, st>>>(H, Z, n);
 }
 
 template <int NT>
@@ -478,12 +482,14 @@ void hessenberg_batched(cplx* const* d_H, cplx* const* d_Z, int batch, int n, cu
     hessenberg_cluster_batched(d_H, d_Z, batch, n, st);
     return;
   }
-  // In shared memory it takes a third to a half of hess_kernel's time at n = 21
-  // to 82, at every batch.
+  // Within it the kernel in shared memory, at every batch (its figures above).
   if (n <= HS_MAXN) {
-    if (n <= 32) launch_hess_smem<1>(d_H, d_Z, batch, n, st);
-    else if (n <= 64) launch_hess_smem<2>(d_H, d_Z, batch, n, st);
-    else launch_hess_smem<3>(d_H, d_Z, batch, n, st);
+    if (n <= 32) launch_hess_smem<4>(d_H, d_Z, batch, n, st);
+    else if (n <= 48) launch_hess_smem<6>(d_H, d_Z, batch, n, st);
+    else if (n <= 64) launch_hess_smem<8>(d_H, d_Z, batch, n, st);
+    else if (n <= 80) launch_hess_smem<10>(d_H, d_Z, batch, n, st);
+    else if (n <= 96) launch_hess_smem<12>(d_H, d_Z, batch, n, st);
+    else launch_hess_smem<14>(d_H, d_Z, batch, n, st);
     VRC_CUDA_CHECK(cudaGetLastError());
     return;
   }

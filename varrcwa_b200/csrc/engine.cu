@@ -1127,14 +1127,15 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
 // ---------------------------------------------------------------------------
 // Eigen-decomposition of PQ (A7)
 // ---------------------------------------------------------------------------
-// Blocked Hessenberg reduction (panels + DMMA GEMM updates) from this order
-// up, the single-CTA kernel below it: busy ms per pass of whole solves,
-// single-CTA / blocked, n = 61 (80 matrices at a time) 7.9 / 13.2, n = 82 (20)
-// 3.70 / 3.66, n = 98 (3) 8.7 / 7.3, n = 110 (3) 3.45 / 2.31, n = 126 (8) 2.65 /
-// 1.48.  VRC_HESS_BLOCKED=0 / 1 turns it off / on for every order.
+// Blocked Hessenberg reduction (panels + DMMA GEMM updates) from the order up at
+// which the matrix no longer fits the shared memory of one CTA: one / 600
+// matrices in ms, shared memory against blocked, n = 61 0.21 / 0.73 against 0.49 /
+// 1.6, n = 98 0.58 / 2.9 against 0.93 / 4.1, n = 112 0.70 / 3.6 against 1.12 / 5.0;
+// from global memory, against blocked, 2.65 / 1.48 for eight at n = 126.
+// VRC_HESS_BLOCKED=0 / 1 turns it off / on for every order.
 static bool use_blocked_hessenberg(int n) {
   if (const char* e = std::getenv("VRC_HESS_BLOCKED")) return std::atoi(e) != 0 && n >= 3;
-  return n >= 96;
+  return n > 112;
 }
 
 void Engine::eig(std::vector<EigReq>& reqs, int n, std::vector<int>* status) {
