@@ -44,6 +44,13 @@ def test_reduced_columns(ctx, n):
     _check(ctx, A)
 
 
+@pytest.mark.parametrize("n,batch", [(114, 1), (127, 150), (160, 2), (192, 1), (193, 1), (256, 1), (257, 1), (513, 1)])
+def test_panels(ctx, n, batch):
+    """Row slots and column groups of the reduction's panels."""
+    rng = np.random.default_rng(n)
+    _check(ctx, rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n)))
+
+
 @pytest.mark.parametrize("scale", [1e-120, 1e-75, 1e60])
 @pytest.mark.parametrize("n", [13, 140])
 def test_scaled(ctx, n, scale):

@@ -454,8 +454,7 @@ __global__ void __cluster_dims__(HC_CS, 1, 1) __launch_bounds__(HC_THREADS, 1)
 // pass over the trailing matrix per column is that product with A0, which
 // reads columns j+1 .. n-1, not yet written in this panel.
 constexpr int HB_NB = 32;
-constexpr int HB_THREADS = 256;
-constexpr int HB_WARPS = HB_THREADS / 32;
+constexpr int HB_THREADS = 1024;  // at most
 
 struct HbLayout {
   size_t V, Y, X, W, T, total;  // complex-element offsets in a matrix's scratch
@@ -477,13 +476,26 @@ __host__ __device__ inline HbLayout hb_layout(int n) {
   return L;
 }
 
+// Thread tid takes the rows tid % RL + RL t (t < NT) and, of the sums over
+// columns, reflectors included, every G-th term (G = threads / RL groups, their
+// shares added up in shared memory).  Bound by the product with A0, whose
+// columns come from L2, and by the chain of nine barriers a column.  With 256
+// threads a CTA kept too few loads in flight: the whole reduction, one / 32
+// matrices, took 2.29 / 2.42 ms at n = 162 (now 1.93 / 2.06), and 16 at n = 450
+// took 21.2 (now 14.7).
 template <int NT>
 __global__ void __launch_bounds__(HB_THREADS)
-    hb_panel_kernel(cplx* const* __restrict__ Hs, cplx* __restrict__ scratch, size_t stride, int n, int k, int nbp) {
+    hb_panel_kernel(cplx* const* __restrict__ Hs, cplx* __restrict__ scratch, size_t stride, int n, int k, int nbp,
+                    int RL) {
+  constexpr int TLD = HB_NB + 1;
+  constexpr int U = NT <= 2 ? 4 : 2;  // columns in flight
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* c = reinterpret_cast<cplx*>(smem_raw);  // [n] column being reduced
   cplx* v = c + n;                              // [n] its reflector
-  __shared__ cplx s_w[HB_NB], s_w2[HB_NB], s_red[HB_WARPS];
+  cplx* Ts = v + n;                             // [HB_NB][TLD] T (entry (q, l) at l TLD + q)
+  cplx* part = Ts + HB_NB * TLD;                // [G][n] shares
+  __shared__ cplx s_w[HB_NB], s_w2[HB_NB];
+  __shared__ double s_red[HB_THREADS / 32];
   __shared__ cplx s_tau, s_scale;
   __shared__ double s_beta;
   const HbLayout L = hb_layout(n);
@@ -492,156 +504,173 @@ __global__ void __launch_bounds__(HB_THREADS)
   cplx* V = base + L.V;
   cplx* Y = base + L.Y;
   cplx* T = base + L.T;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int G = blockDim.x / RL, g = tid / RL, rl = tid - g * RL;
   const int J0 = k + 1;
+  const cplx zero = mk(0.0, 0.0);
+  auto wsum = [](cplx z) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      z.x += __shfl_xor_sync(0xffffffffu, z.x, o);
+      z.y += __shfl_xor_sync(0xffffffffu, z.y, o);
+    }
+    return z;
+  };
   // w[l] = sum_{r >= J0} conj(V[r, l]) x[r] for l < i (warp per l)
   auto vh_dot = [&](const cplx* x, int i, cplx* w) {
-    for (int l = warp; l < i; l += HB_WARPS) {
+    for (int l = warp; l < i; l += nw) {
       const cplx* vl = V + (size_t)l * n;
-      cplx sacc = mk(0.0, 0.0);
-      for (int r = J0 + lane; r < n; r += 32) sacc = cadd(sacc, cmulc(vl[r], x[r]));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sacc.x += __shfl_xor_sync(0xffffffffu, sacc.x, o);
-        sacc.y += __shfl_xor_sync(0xffffffffu, sacc.y, o);
-      }
+      cplx sacc = zero;
+      for (int r = J0 + lane; r < n; r += 32) sacc = cfma(cconj(vl[r]), x[r], sacc);
+      sacc = wsum(sacc);
       if (lane == 0) w[l] = sacc;
     }
+  };
+  auto total = [&](int r) {
+    cplx a = part[r];
+    for (int q = 1; q < G; ++q) a = cadd(a, part[q * n + r]);
+    return a;
   };
   for (int i = 0; i < nbp; ++i) {
     const int j = k + i;
     // 1-2. column j, updated from the right by the panel's previous reflectors
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-      const int r = tid + HB_THREADS * t;
-      if (r < n) {
-        cplx a = H[(size_t)j * n + r];
-        for (int l = 0; l < i; ++l) a = csub(a, cmul(Y[(size_t)l * n + r], cconj(V[(size_t)l * n + j])));
-        c[r] = a;
+      const int r = rl + RL * t;
+      if (r < n && g < G) {
+        cplx a = g == 0 ? H[(size_t)j * n + r] : zero;
+        for (int l = g; l < i; l += G) a = cfma(cneg(Y[(size_t)l * n + r]), cconj(V[(size_t)l * n + j]), a);
+        part[g * n + r] = a;
       }
     }
+    __syncthreads();
+    for (int r = tid; r < n; r += blockDim.x) c[r] = total(r);
     __syncthreads();
     // 3. and from the left: c[J] -= V T^H V^H c[J]
     if (i > 0) {
       vh_dot(c, i, s_w);
       __syncthreads();
-      if (tid < i) {  // w2 = T^H w, T upper triangular (T(q, l) at T[l * HB_NB + q])
-        cplx a = mk(0.0, 0.0);
-        for (int q = 0; q <= tid; ++q) a = cadd(a, cmulc(T[(size_t)tid * HB_NB + q], s_w[q]));
-        s_w2[tid] = a;
+      for (int l = warp; l < i; l += nw) {  // w2 = T^H w, T upper triangular
+        const cplx a = wsum(lane <= l ? cmulc(Ts[l * TLD + lane], s_w[lane]) : zero);
+        if (lane == 0) s_w2[l] = a;
       }
       __syncthreads();
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        const int r = tid + HB_THREADS * t;
-        if (r >= J0 && r < n) {
-          cplx a = c[r];
-          for (int l = 0; l < i; ++l) a = csub(a, cmul(V[(size_t)l * n + r], s_w2[l]));
-          c[r] = a;
+        const int r = rl + RL * t;
+        if (r >= J0 && r < n && g < G) {
+          cplx a = g == 0 ? c[r] : zero;
+        for (int l = g; l < i; l += G) a = cfma(cneg(V[(size_t)l * n + r]), s_w2[l], a);
+          part[g * n + r] = a;
         }
       }
       __syncthreads();
     }
     // 4. reflector from c[j+1 ..]
     {
-      double part = 0.0;
-      for (int r = j + 2 + tid; r < n; r += HB_THREADS) part += cabs2(c[r]);
+      double sq = 0.0;
+      for (int r = J0 + tid; r < n; r += blockDim.x) {
+        if (i > 0) c[r] = total(r);
+        if (r >= j + 2) sq += cabs2(c[r]);
+      }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-      if (lane == 0) s_red[warp] = mk(part, 0.0);
+      for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+      if (lane == 0) s_red[warp] = sq;
       __syncthreads();
-      if (tid == 0) {
-        double xn = 0.0;
-        for (int w = 0; w < HB_WARPS; ++w) xn += s_red[w].x;
+      if (warp == 0) {
+        double xn = lane < nw ? s_red[lane] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) xn += __shfl_xor_sync(0xffffffffu, xn, o);
         double beta;
         cplx tau, scale;
         householder(c[j + 1], xn, &beta, &tau, &scale);
-        s_beta = beta;
-        s_tau = tau;
-        s_scale = scale;
+        if (lane == 0) {
+          s_beta = beta;
+          s_tau = tau;
+          s_scale = scale;
+        }
       }
       __syncthreads();
     }
     const cplx tau = s_tau;
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      const int r = tid + HB_THREADS * t;
-      if (r < n) {
-        cplx vr = mk(0.0, 0.0), hr = c[r];
-        if (r == j + 1) {
-          vr = mk(1.0, 0.0);
-          hr = mk(s_beta, 0.0);
-        } else if (r > j + 1) {
-          vr = cmul(c[r], s_scale);
-          hr = mk(0.0, 0.0);
-        }
-        v[r] = vr;
-        V[(size_t)i * n + r] = vr;
-        H[(size_t)j * n + r] = hr;  // column j is final
+    for (int r = tid; r < n; r += blockDim.x) {
+      cplx vr = zero, hr = c[r];
+      if (r == j + 1) {
+        vr = mk(1.0, 0.0);
+        hr = mk(s_beta, 0.0);
+      } else if (r > j + 1) {
+        vr = cmul(c[r], s_scale);
+        hr = zero;
       }
+      v[r] = vr;
+      V[(size_t)i * n + r] = vr;
+      H[(size_t)j * n + r] = hr;  // column j is final
     }
     __syncthreads();
-    // 5. y = A0[:, j+1:] v (columns right of j are untouched in this panel);
-    // four partial sums over interleaved columns keep four independent FMA
-    // chains (and their loads) in flight, added in a fixed order
+    // 5. y = A0[:, j+1:] v (columns right of j are untouched in this panel), the
+    // group's columns in U chains
     cplx y[NT];
     {
-      cplx ya[4][NT];
+      cplx ya[U][NT];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int t = 0; t < NT; ++t) ya[u][t] = mk(0.0, 0.0);
-      if (!(tau.x == 0.0 && tau.y == 0.0)) {
-        int col = j + 1;
-        for (; col + 3 < n; col += 4) {
+        for (int t = 0; t < NT; ++t) ya[u][t] = zero;
+      if (!(tau.x == 0.0 && tau.y == 0.0) && g < G) {
+        int col = j + 1 + g;
+        for (; col + (U - 1) * G < n; col += U * G) {
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const cplx vc = v[col + u];
-            const cplx* hc = H + (size_t)(col + u) * n;
+          for (int u = 0; u < U; ++u) {
+            const cplx vc = v[col + u * G];
+            const cplx* hc = H + (size_t)(col + u * G) * n;
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
-              const int r = tid + HB_THREADS * t;
+              const int r = rl + RL * t;
               if (r < n) ya[u][t] = cfma(hc[r], vc, ya[u][t]);
             }
           }
         }
-        for (; col < n; ++col) {
+        for (; col < n; col += G) {
           const cplx vc = v[col];
           const cplx* hc = H + (size_t)col * n;
 #pragma unroll
           for (int t = 0; t < NT; ++t) {
-            const int r = tid + HB_THREADS * t;
+            const int r = rl + RL * t;
             if (r < n) ya[0][t] = cfma(hc[r], vc, ya[0][t]);
           }
         }
       }
 #pragma unroll
-      for (int t = 0; t < NT; ++t) y[t] = cadd(cadd(ya[0][t], ya[1][t]), cadd(ya[2][t], ya[3][t]));
+      for (int t = 0; t < NT; ++t) {
+        y[t] = ya[0][t];
+#pragma unroll
+        for (int u = 1; u < U; ++u) y[t] = cadd(y[t], ya[u][t]);
+      }
     }
     // 6. Y[:, i] = tau (y - Y[:, :i] w'), w' = V[:, :i]^H v; T column i
     if (i > 0) vh_dot(v, i, s_w);
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-      const int r = tid + HB_THREADS * t;
-      if (r < n) {
+      const int r = rl + RL * t;
+      if (r < n && g < G) {
         cplx a = y[t];
-        for (int l = 0; l < i; ++l) a = csub(a, cmul(Y[(size_t)l * n + r], s_w[l]));
-        Y[(size_t)i * n + r] = cmul(tau, a);
+        for (int l = g; l < i; l += G) a = cfma(cneg(Y[(size_t)l * n + r]), s_w[l], a);
+        part[g * n + r] = a;
       }
     }
-    if (tid <= i) {
-      cplx a = tau;
-      if (tid < i) {  // T(q, i) = -tau sum_{p = q}^{i-1} T(q, p) w'[p]
-        a = mk(0.0, 0.0);
-        for (int p = tid; p < i; ++p) a = cadd(a, cmul(T[(size_t)p * HB_NB + tid], s_w[p]));
-        a = cneg(cmul(tau, a));
+    for (int q = warp; q < HB_NB; q += nw) {
+      // T(q, i) = -tau sum_{p = q}^{i-1} T(q, p) w'[p], T(i, i) = tau; zero below
+      // (the GEMM stages read T as a full block)
+      const cplx a = wsum(lane >= q && lane < i ? cmul(Ts[lane * TLD + q], s_w[lane]) : zero);
+      if (lane == 0) {
+        const cplx e = q < i ? cneg(cmul(tau, a)) : q == i ? tau : zero;
+        Ts[i * TLD + q] = e;
+        T[(size_t)i * HB_NB + q] = e;
       }
-      T[(size_t)i * HB_NB + tid] = a;
-    } else if (tid < HB_NB) {
-      // the strictly lower part: the GEMM stages read T as a full block
-      T[(size_t)i * HB_NB + tid] = mk(0.0, 0.0);
     }
+    __syncthreads();
+    for (int r = tid; r < n; r += blockDim.x) Y[(size_t)i * n + r] = cmul(tau, total(r));
     __syncthreads();
   }
 }
@@ -670,10 +699,12 @@ __global__ void hb_desc_kernel(cplx* const* __restrict__ Hs, cplx* const* __rest
 }
 
 template <int NT>
-void launch_hb_panel(cplx* const* H, cplx* scratch, size_t stride, int batch, int n, int k, int nbp, cudaStream_t st) {
-  const size_t smem = 2 * (size_t)n * sizeof(cplx);
+void launch_hb_panel(cplx* const* H, cplx* scratch, size_t stride, int batch, int n, int k, int nbp, int threads,
+                     cudaStream_t st) {
+  const int RL = std::min(256, ((n + NT - 1) / NT + 31) / 32 * 32), G = std::max(1, threads / RL);
+  const size_t smem = ((size_t)(2 + G) * n + HB_NB * (HB_NB + 1)) * sizeof(cplx);
   ensure_smem((const void*)hb_panel_kernel<NT>, smem);
-  hb_panel_kernel<NT><<<batch, HB_THREADS, smem, st>>>(H, scratch, stride, n, k, nbp);
+  hb_panel_kernel<NT><<<batch, RL * G, smem, st>>>(H, scratch, stride, n, k, nbp, RL);
 }
 
 }  // namespace
@@ -691,13 +722,23 @@ void hessenberg_blocked_batched(cplx* const* d_H, cplx* const* d_Z, int batch, i
   cplx* scr = static_cast<cplx*>(scratch);
   GemmDesc* dd = static_cast<GemmDesc*>(descs);
   set_identity_batched(d_Z, batch, n, 1.0, st);
+  // A CTA of 1024 threads fills the SM; two of 512 are better where more than one
+  // matrix waits for each SM and a column is short: 160 matrices at n = 120 2.0 ms
+  // against 2.3, 300 at n = 162 8.8 against 6.9.
+  static const int sms = [] {
+    int dev = 0, v = 0;
+    VRC_CUDA_CHECK(cudaGetDevice(&dev));
+    VRC_CUDA_CHECK(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+    return v;
+  }();
+  const int threads = n <= 128 && batch > sms ? HB_THREADS / 2 : HB_THREADS;
   const cplx one = mk(1.0, 0.0), mone = mk(-1.0, 0.0), zero = mk(0.0, 0.0);
   for (int k = 0; k < n - 2; k += HB_NB) {
     const int nbp = std::min(HB_NB, n - 2 - k);
     const int J0 = k + 1, MJ = n - J0, c0 = k + nbp, N2 = n - c0;
-    if (n <= 256) launch_hb_panel<1>(d_H, scr, stride, batch, n, k, nbp, st);
-    else if (n <= 512) launch_hb_panel<2>(d_H, scr, stride, batch, n, k, nbp, st);
-    else launch_hb_panel<4>(d_H, scr, stride, batch, n, k, nbp, st);
+    if (n <= 256) launch_hb_panel<1>(d_H, scr, stride, batch, n, k, nbp, threads, st);
+    else if (n <= 512) launch_hb_panel<2>(d_H, scr, stride, batch, n, k, nbp, threads, st);
+    else launch_hb_panel<4>(d_H, scr, stride, batch, n, k, nbp, threads, st);
     VRC_CUDA_CHECK(cudaGetLastError());
     hb_desc_kernel<<<(batch + 127) / 128, 128, 0, st>>>(d_H, d_Z, scr, stride, n, k, nbp, batch, dd);
     VRC_CUDA_CHECK(cudaGetLastError());
