@@ -51,6 +51,18 @@ def test_panels(ctx, n, batch):
     _check(ctx, rng.standard_normal((batch, n, n)) + 1j * rng.standard_normal((batch, n, n)))
 
 
+@pytest.mark.parametrize("n", [159, 160, 230])
+def test_teams(ctx, n):
+    """However many CTAs a matrix gets, the eigenvalues are the same bits."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((1, n, n)) + 1j * rng.standard_normal((1, n, n))
+    _check(ctx, A)
+    one = ctx.eig(A)[0][0]
+    for batch in (9, 10, 29, 30, 37, 38):
+        lam = ctx.eig(np.repeat(A, batch, axis=0))[0]
+        assert all(np.array_equal(x, one) for x in lam)
+
+
 @pytest.mark.parametrize("scale", [1e-120, 1e-75, 1e60])
 @pytest.mark.parametrize("n", [13, 140])
 def test_scaled(ctx, n, scale):

@@ -34,12 +34,16 @@
 // its unconverged ones are the sweep's shifts.  Its similarity transform U is
 // applied eagerly inside the active window and logged as a dense block for
 // the replay, in sequence with the sweeps' rotations.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstdlib>
 
 #include "common.cuh"
 #include "householder.cuh"
 #include "kernels.h"
+
+namespace cg = cooperative_groups;
 
 namespace vrc {
 namespace {
@@ -197,10 +201,15 @@ __device__ __forceinline__ cplx single_shift(const cplx* H, int n, int l, int i,
   return wilkinson(h(i - 1, i - 1), h(i - 1, i), h(i, i - 1), h(i, i));
 }
 
-// cp.async copies of 16 bytes into shared memory, one commit group each.
+// cp.async copies of 16 bytes into shared memory, one commit group each; SHARED:
+// past L1, for data that other CTAs of the cluster write.
+template <bool SHARED = false>
 __device__ __forceinline__ void cpa16(cplx* smem, const cplx* g) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(g) : "memory");
+  if (SHARED)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(g) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(g) : "memory");
 }
 __device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -511,8 +520,83 @@ __device__ int aed_deflate_warp(cplx* T, cplx* U, cplx* v, cplx* ev, int nw, cpl
   return ns;
 }
 
-// MINB: resident CTAs per SM the registers are sized for.
-template <int MINB>
+// One chunk of a sweep, for the CTAs that transform what lies outside D.
+struct Chunk {
+  int m, i, nb, r0, r1, kmin, kmax, ds, de;  // m < 0: the matrix is done
+};
+
+// The rest of the active window: columns de+1..i (row transforms) and rows
+// m..ds-1 (column transforms), FV vectors per warp at a time; every step-th
+// group from first on.
+__device__ __forceinline__ int far_groups(const Chunk& c) {
+  return (c.i - c.de + FV - 1) / FV + (c.ds - c.m + FV - 1) / FV;
+}
+template <bool TEAM>
+__device__ __forceinline__ void far_strips(cplx* H, int n, const Chunk& ch, cplx* D, const double* s_c,
+                                           const cplx* s_s, int first, int step) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cnt = ch.kmax + 2 - ch.kmin;  // entries kmin..kmax+1 of each vector
+  const int gr = (ch.i - ch.de + FV - 1) / FV, ng = far_groups(ch);
+  cplx* buf = D + (size_t)warp * 2 * FV * FE;
+  auto where = [&](int g, cplx*& x, size_t& es, size_t& vs, int& nv) {
+    if (g < gr) {  // columns
+      const int c0 = ch.de + 1 + g * FV;
+      x = H + (size_t)c0 * n + ch.kmin;
+      es = 1;
+      vs = n;
+      nv = min(FV, ch.i + 1 - c0);
+    } else {  // rows
+      const int q0 = ch.m + (g - gr) * FV;
+      x = H + (size_t)ch.kmin * n + q0;
+      es = n;
+      vs = 1;
+      nv = min(FV, ch.ds - q0);
+    }
+  };
+  auto fetch = [&](int g, int half) {
+    cplx* x;
+    size_t es, vs;
+    int nv;
+    where(g, x, es, vs, nv);
+    const int v = lane % FV;
+    if (v < nv)
+      for (int e = lane / FV; e < cnt; e += 32 / FV)
+        cpa16<TEAM>(buf + half * FV * FE + e * FV + v, x + (size_t)e * es + (size_t)v * vs);
+    cpa_commit();
+  };
+  const int b = lane / FV;  // this lane's bulge
+  const int ra0 = max(ch.r0, 3 * b), ra1 = b < ch.nb ? min(ch.r1, 3 * b + (ch.i - ch.m)) : ch.r0;
+  const int off = (ch.m + ra0 - 3 * b - ch.kmin) * FV + lane % FV;
+  if (first < ng) fetch(first, 0);
+  for (int g = first, half = 0; g < ng; g += step, half ^= 1) {
+    if (g + step < ng) {
+      fetch(g + step, half ^ 1);
+      cpa_wait<1>();
+    } else {
+      cpa_wait<0>();
+    }
+    __syncwarp();
+    cplx* vec = buf + half * FV * FE;
+    if (g < gr)
+      strip_rounds<true>(vec + off, ch.r0, ch.r1, ra0, ra1, s_c + b, s_s + b);
+    else
+      strip_rounds<false>(vec + off, ch.r0, ch.r1, ra0, ra1, s_c + b, s_s + b);
+    cplx* x;
+    size_t es, vs;
+    int nv;
+    where(g, x, es, vs, nv);
+    const int v = lane % FV;
+    if (v < nv)
+      for (int e = lane / FV; e < cnt; e += 32 / FV) x[(size_t)e * es + (size_t)v * vs] = vec[e * FV + v];
+    __syncwarp();  // the buffer is free for the group after next
+  }
+}
+
+// MINB: resident CTAs per SM the registers are sized for.  TEAM: a cluster per
+// matrix.  Its first CTA iterates; the others wait for its chunks and take their
+// share of the strips outside D (at n = 450 on one CTA 44% of the iteration),
+// which changes nothing in the arithmetic.
+template <int MINB, bool TEAM>
 __global__ void __launch_bounds__(QR_THREADS, MINB)
     hqr_kernel(cplx* const* __restrict__ Hs, void* const* __restrict__ logs, cplx* const* __restrict__ Ws, int n,
                int sweep_cap, long long rot_cap, int* __restrict__ status, int aed_min, int aed_w) {
@@ -531,11 +615,40 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
   __shared__ long long s_clk[7];  // statistics: phase timers (defl, shift, rounds, far), the last stamp,
                                   // window Schur form and window deflation
 
-  cplx* H = Hs[blockIdx.x];
-  char* logb = static_cast<char*>(logs[blockIdx.x]);
+  __shared__ Chunk s_chunk;
+  const int team = TEAM ? (int)cg::this_cluster().num_blocks() : 1;
+  const int mat = blockIdx.x / team;
+  // every CTA's writes to H are visible to the whole cluster
+  auto team_sync = [&] {
+    __threadfence();
+    cg::this_cluster().sync();
+    __threadfence();
+  };
+  cplx* H = Hs[mat];
+  if (TEAM && cg::this_cluster().block_rank() != 0) {
+    const int rank = (int)cg::this_cluster().block_rank(), wp = threadIdx.x >> 5;
+    const Chunk* rc = cg::this_cluster().map_shared_rank(&s_chunk, 0);
+    const cplx* rs = cg::this_cluster().map_shared_rank(s_s, 0);
+    const double* rcs = cg::this_cluster().map_shared_rank(s_c, 0);
+    for (;;) {
+      team_sync();
+      const Chunk ch = *rc;
+      if (ch.m >= 0) {
+        for (int q = threadIdx.x; q < NBMAX * (ch.r1 - ch.r0); q += QR_THREADS) {
+          s_s[q] = rs[q];
+          s_c[q] = rcs[q];
+        }
+        __syncthreads();
+        far_strips<TEAM>(H, n, ch, D, s_c, s_s, NBMAX * rank + wp, NBMAX * team);
+      }
+      team_sync();
+      if (ch.m < 0) return;
+    }
+  }
+  char* logb = static_cast<char*>(logs[mat]);
   QrSweep* sweeps = log_sweeps(logb);
   cplx* rot = log_rot(logb, sweep_cap);
-  cplx* W = Ws[blockIdx.x];
+  cplx* W = Ws[mat];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double smlnum = EIG_SAFMIN * ((double)n / EIG_ULP);
   const int itmax = 30 * max(10, n);       // per eigenvalue
@@ -738,7 +851,7 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
         const int dn = de - ds + 1;
         for (int c = warp; c < dn; c += QR_THREADS / 32) {
           const cplx* hc = &h(ds, ds + c);
-          for (int r = lane; r < dn; r += 32) cpa16(D + c * QLD + r, hc + r);
+          for (int r = lane; r < dn; r += 32) cpa16<TEAM>(D + c * QLD + r, hc + r);
         }
         cpa_commit();
         cpa_wait<0>();
@@ -834,68 +947,17 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
           rot[2 * ri] = mk(s_c[u * NBMAX + b], 0.0);  // (the identity where the bulge is outside the window)
           rot[2 * ri + 1] = s_s[u * NBMAX + b];
         }
-        __syncthreads();  // D is free
-        // Rest of the active window: columns de+1..i (row transforms) and rows
-        // m..ds-1 (column transforms), FV vectors per warp at a time.
-        {
-          const int cnt = kmax + 2 - kmin;  // entries kmin..kmax+1 of each vector
-          const int nright = i - de, nabove = ds - m;
-          const int gr = (nright + FV - 1) / FV, ng = gr + (nabove + FV - 1) / FV;
-          cplx* buf = D + (size_t)warp * 2 * FV * FE;
-          auto where = [&](int g, cplx*& x, size_t& es, size_t& vs, int& nv) {
-            if (g < gr) {  // columns
-              const int c0 = de + 1 + g * FV;
-              x = H + (size_t)c0 * n + kmin;
-              es = 1;
-              vs = n;
-              nv = min(FV, i + 1 - c0);
-            } else {  // rows
-              const int q0 = m + (g - gr) * FV;
-              x = H + (size_t)kmin * n + q0;
-              es = n;
-              vs = 1;
-              nv = min(FV, ds - q0);
-            }
-          };
-          auto fetch = [&](int g, int half) {
-            cplx* x;
-            size_t es, vs;
-            int nv;
-            where(g, x, es, vs, nv);
-            const int v = lane % FV;
-            if (v < nv)
-              for (int e = lane / FV; e < cnt; e += 32 / FV)
-                cpa16(buf + half * FV * FE + e * FV + v, x + (size_t)e * es + (size_t)v * vs);
-            cpa_commit();
-          };
-          const int b = lane / FV;  // this lane's bulge
-          const int ra0 = max(r0, 3 * b), ra1 = b < nb ? min(r1, 3 * b + (i - m)) : r0;
-          const int off = (m + ra0 - 3 * b - kmin) * FV + lane % FV;
-          if (warp < ng) fetch(warp, 0);
-          for (int g = warp, half = 0; g < ng; g += NBMAX, half ^= 1) {
-            if (g + NBMAX < ng) {
-              fetch(g + NBMAX, half ^ 1);
-              cpa_wait<1>();
-            } else {
-              cpa_wait<0>();
-            }
-            __syncwarp();
-            cplx* vec = buf + half * FV * FE;
-            if (g < gr)
-              strip_rounds<true>(vec + off, r0, r1, ra0, ra1, s_c + b, s_s + b);
-            else
-              strip_rounds<false>(vec + off, r0, r1, ra0, ra1, s_c + b, s_s + b);
-            cplx* x;
-            size_t es, vs;
-            int nv;
-            where(g, x, es, vs, nv);
-            const int v = lane % FV;
-            if (v < nv)
-              for (int e = lane / FV; e < cnt; e += 32 / FV) x[(size_t)e * es + (size_t)v * vs] = vec[e * FV + v];
-            __syncwarp();  // the buffer is free for the group after next
-          }
+        const Chunk ch{m, i, nb, r0, r1, kmin, kmax, ds, de};
+        if (TEAM && far_groups(ch) > NBMAX) {
+          if (tid == 0) s_chunk = ch;
+          team_sync();  // D is free; the others read the chunk
+          far_strips<TEAM>(H, n, ch, D, s_c, s_s, warp, NBMAX * team);
+          team_sync();
+        } else {
+          __syncthreads();  // D is free
+          far_strips<TEAM>(H, n, ch, D, s_c, s_s, warp, NBMAX);
+          __syncthreads();
         }
-        __syncthreads();
         if (tid == 0) stamp(3);
       }
       if (s_over) {
@@ -923,7 +985,12 @@ __global__ void __launch_bounds__(QR_THREADS, MINB)
     hdr->t_far = s_clk[3];
     hdr->t_wschur = s_clk[5];
     hdr->t_wdefl = s_clk[6];
-    if (failed && status) status[blockIdx.x] = ST_ENOCONV;
+    if (failed && status) status[mat] = ST_ENOCONV;
+    s_chunk.m = -1;
+  }
+  if (TEAM) {
+    team_sync();  // the others see that the matrix is done
+    team_sync();  // and have read it
   }
 }
 
@@ -1099,6 +1166,25 @@ __global__ void __launch_bounds__(RP_MAXW * 32)
 
 }  // namespace
 
+// CTAs per matrix of the iteration: clusters of 8 on half of the SMs, of 4 on four
+// fifths, of 2 on half (with 66 matrices at n = 162 on all of them, beside another
+// stream's work, 13.4 ms for 10.4 alone).
+// ms for 1 / 2 / 4 / 8: n = 450, 4 matrices 72.7 / 61.3 / 56.5 / 52.4, 16 matrices
+// 72.1 / 61.2 / 54.3 / 59.9; n = 242, 18 matrices 22.8 / 19.9 / 19.1 / 20.9; n = 162,
+// 4 matrices 10.9 / 10.8 / 10.6 / 10.6; 37 matrices 10.8 / 10.7 / 11.3 / 20.3 (the
+// clusters no longer fit side by side); below, the strips are too few: n = 120, 3
+// matrices 5.98 / 6.10 / 6.07 / 6.12.
+static int team_size(int n, int batch) {
+  static const int sms = [] {
+    int dev = 0, v = 0;
+    VRC_CUDA_CHECK(cudaGetDevice(&dev));
+    VRC_CUDA_CHECK(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+    return v;
+  }();
+  if (n < 160) return 1;
+  return 2LL * batch * 8 <= sms ? 8 : 5LL * batch * 4 <= 4LL * sms ? 4 : 4LL * batch <= sms ? 2 : 1;
+}
+
 void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* const* d_logs, int batch, int n,
                    int* d_status, cudaStream_t st, int parts) {
   if (batch <= 0) return;
@@ -1108,7 +1194,7 @@ void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* c
     const char* e = std::getenv("VRC_QR_CTAS");
     return (e && std::atoi(e) == 3) ? 3 : 2;
   }();
-  auto hqr = minb == 3 ? hqr_kernel<3> : hqr_kernel<2>;
+  auto hqr = minb == 3 ? hqr_kernel<3, false> : hqr_kernel<2, false>;
   // Order of the deflation window (VRC_QR_AEDW, 4..32) and the order of the
   // active window from which it is taken (VRC_QR_AED; 0: never).  By default 10
   // and 48 for n > 128, never below: ms of iteration and replay for windows of
@@ -1136,9 +1222,28 @@ void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* c
   const int row_blocks = (n + rp_threads / 32 * FV - 1) / (rp_threads / 32 * FV);
   for (int b0 = 0; b0 < batch; b0 += 65535) {
     const int nb = min(65535, batch - b0);
-    if (parts & SCHUR_ITERATE)
-      hqr<<<nb, QR_THREADS, QR_SMEM, st>>>(d_H + b0, d_logs + b0, d_W + b0, n, cc, rc,
-                                                  d_status ? d_status + b0 : nullptr, aed_min, aed_w);
+    if (parts & SCHUR_ITERATE) {
+      int* stat = d_status ? d_status + b0 : nullptr;
+      const int team = team_size(n, nb);
+      if (team > 1) {
+        ensure_smem((const void*)hqr_kernel<2, true>, QR_SMEM);
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)team;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(nb * team));
+        cfg.blockDim = dim3(QR_THREADS);
+        cfg.dynamicSmemBytes = QR_SMEM;
+        cfg.stream = st;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        VRC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, hqr_kernel<2, true>, d_H + b0, d_logs + b0, d_W + b0, n, cc, rc, stat,
+                                          aed_min, aed_w));
+      } else {
+        hqr<<<nb, QR_THREADS, QR_SMEM, st>>>(d_H + b0, d_logs + b0, d_W + b0, n, cc, rc, stat, aed_min, aed_w);
+      }
+    }
     if (parts & SCHUR_REPLAY) {
       qr_replay_rows_kernel<<<dim3(2 * row_blocks, nb), rp_threads, rp_smem, st>>>(d_H + b0, d_Z + b0, d_logs + b0,
                                                                                   n, cc, row_blocks);
