@@ -26,23 +26,6 @@ __device__ __forceinline__ void householder(cplx alpha, double xnorm2, double* b
   *scale = mk(ux * rd, -alpha.y * rd);
 }
 
-// Two-element reflector for (a, b): returns the new leading entry, tau and
-// v2 (v = (1, v2)).
-__device__ __forceinline__ void refl2(cplx a, cplx b, cplx* beta, cplx* tau, cplx* v2) {
-  double b0;
-  cplx t, sc;
-  householder(a, cabs2(b), &b0, &t, &sc);
-  if (t.x == 0.0 && t.y == 0.0) {
-    *beta = a;
-    *tau = t;
-    *v2 = mk(0.0, 0.0);
-    return;
-  }
-  *beta = mk(b0, 0.0);
-  *tau = t;
-  *v2 = cmul(b, sc);
-}
-
 constexpr double EIG_ULP = 2.220446049250313e-16;  // 2^-52
 constexpr double EIG_SAFMIN = 2.2250738585072014e-308;
 
