@@ -32,7 +32,7 @@ def test_orders(ctx, n):
     _check(ctx, rng.standard_normal((3, n, n)) + 1j * rng.standard_normal((3, n, n)))
 
 
-@pytest.mark.parametrize("n", [2, 3, 8, 9, 32, 33, 48, 49, 64, 65, 80, 81, 95, 96, 97, 111, 112, 113])
+@pytest.mark.parametrize("n", [2, 3, 8, 9, 32, 33, 48, 49, 64, 65, 80, 81, 95, 96, 97, 111, 112, 113, 114])
 def test_reduced_columns(ctx, n):
     """Reflectors at the edges of the small reduction's lanes and columns,
     with columns that need none."""

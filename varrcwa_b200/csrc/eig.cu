@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(HESS_THREADS)
   }
 }
 
-// The same reduction for n <= 112 with the matrix in shared memory, Q accumulated
+// The same reduction for n <= 113 with the matrix in shared memory, Q accumulated
 // in its place.  Eight lanes take a column (a row in eight each, the rows padded
 // with zeros to 8 RV) and the CTA 32 columns at a time: both products in one
 // pass, v^H a_j kept in registers for the update, and every warp forms the
@@ -203,8 +203,9 @@ __global__ void __launch_bounds__(HESS_THREADS)
 // A v, their sum, the next reflector's column).  Bound by that chain and, with
 // the SMs full, by shared memory and the FP64 pipe.  One / 600 matrices take
 // 0.11 / 0.37 ms at n = 42, 0.21 / 0.73 at 61 (hess_kernel 0.51 for some 60) and
-// 0.58 / 2.9 at 98 (panels and GEMM updates 0.93 / 4.1).
-constexpr int HS_MAXN = 112;  // (what shared memory holds)
+// 0.58 / 2.9 at 98 (panels and GEMM updates 0.93 / 4.1) and 0.75 / 3.8 at 113 (1.02 /
+// 5.1; there RV = 15 leaves the padding out, the only form that fits).
+constexpr int HS_MAXN = 113;  // (what shared memory holds)
 
 __device__ __forceinline__ cplx shfl_xor(cplx z, int o) {
   return mk(__shfl_xor_sync(0xffffffffu, z.x, o), __shfl_xor_sync(0xffffffffu, z.y, o));
@@ -219,7 +220,9 @@ __device__ __forceinline__ cplx sum8(cplx z) {
 template <int RV>
 __global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
     hess_smem_kernel(cplx* const* __restrict__ Hs, cplx* const* __restrict__ Zs, int n) {
-  constexpr int LD = 8 * RV, RT = (RV + 3) / 4 * 4, NT = RT / 4;  // rows and column passes of a lane
+  constexpr bool TIGHT = RV == 15;  // no room for padding: rows past n are the next column's
+  const int LD = TIGHT ? n : 8 * RV;
+  constexpr int RT = (RV + 3) / 4 * 4, NT = RT / 4;  // rows and column passes of a lane
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* A = reinterpret_cast<cplx*>(smem_raw);  // [n][LD]
   cplx* yp = A + n * LD;                        // [HESS_WARPS][LD]
@@ -232,6 +235,8 @@ __global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
   const int l8 = lane & 7, col = 4 * warp + (lane >> 3);
   const bool b0 = lane & 8, b1 = lane & 16;
   const cplx zero = mk(0.0, 0.0);
+  if (TIGHT)
+    for (int r = tid; r < HESS_WARPS * LD; r += HESS_THREADS) yp[r] = zero;  // (past the last column)
   for (int c = warp; c < n; c += HESS_WARPS)
     for (int r = lane; r < LD; r += 32) A[c * LD + r] = r < n ? H[(size_t)c * n + r] : zero;
   __syncthreads();
@@ -242,7 +247,7 @@ __global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
     double part[2] = {0.0, 0.0};
 #pragma unroll
     for (int t = 0; t < RV; ++t) {
-      v[t] = x[l8 + 8 * t];
+      v[t] = !TIGHT || t < RV - 1 || l8 + 8 * t < n ? x[l8 + 8 * t] : zero;
       if (l8 + 8 * t > j0) part[t & 1] += cabs2(v[t]);
     }
     double x2 = part[0] + part[1];
@@ -290,7 +295,7 @@ __global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
       const int t = 4 * q + 2 * b0 + b1;
       const cplx z =
           cadd(b0 ? half[2 * q + 1] : half[2 * q], shfl_xor(b0 ? half[2 * q] : half[2 * q + 1], 8));
-      if (t < RV) yp[warp * LD + l8 + 8 * t] = z;
+      if (t < RV && (!TIGHT || t < RV - 1 || l8 + 8 * t < n)) yp[warp * LD + l8 + 8 * t] = z;
     }
     s = cadd(s, shfl_xor(s, 8));
     s = cadd(s, shfl_xor(s, 16));
@@ -309,7 +314,7 @@ __global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
     if (warp == HESS_WARPS - 1 && lane < 8) {  // column k: its reflector stays below the subdiagonal
 #pragma unroll
       for (int t = 0; t < RV; ++t)
-        if (l8 + 8 * t >= j0) A[k * LD + l8 + 8 * t] = l8 + 8 * t == j0 ? mk(beta, 0.0) : v[t];
+        if (l8 + 8 * t >= j0 && (!TIGHT || t < RV - 1 || l8 + 8 * t < n)) A[k * LD + l8 + 8 * t] = l8 + 8 * t == j0 ? mk(beta, 0.0) : v[t];
     }
     __syncthreads();
 #pragma unroll
@@ -324,7 +329,7 @@ __global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
                    tz = cmul(tauc, csub(cmul(ts, vc), u[p]));
 #pragma unroll
         for (int t = 0; t < RV; ++t)
-          a[8 * t] = cfma(y[t], tv, cfma(v[t], tz, a[8 * t]));
+          if (!TIGHT || t < RV - 1 || l8 + 8 * t < n) a[8 * t] = cfma(y[t], tv, cfma(v[t], tz, a[8 * t]));
       }
     }
     __syncthreads();
@@ -344,7 +349,7 @@ __global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
 #pragma unroll
     for (int t = 0; t < RV; ++t) {
       const int i = l8 + 8 * t;
-      v[t] = i > j0 ? A[k * LD + i] : mk(i == j0 ? 1.0 : 0.0, 0.0);
+      v[t] = i > j0 && (!TIGHT || t < RV - 1 || i < n) ? A[k * LD + i] : mk(i == j0 ? 1.0 : 0.0, 0.0);
     }
 #pragma unroll
     for (int p = 0; p < NT; ++p) {
@@ -362,7 +367,7 @@ __global__ void __launch_bounds__(HESS_THREADS, RV <= 10 ? 2 : 1)
         const cplx tw = cneg(j == j0 ? tau : cmul(tau, z));
 #pragma unroll
         for (int t = 0; t < RV; ++t)
-          if (j < n && l8 + 8 * t >= j0) a[8 * t] = cfma(v[t], tw, h[t]);
+          if (j < n && l8 + 8 * t >= j0 && (!TIGHT || t < RV - 1 || l8 + 8 * t < n)) a[8 * t] = cfma(v[t], tw, h[t]);
       }
     }
     __syncthreads();
@@ -442,7 +447,7 @@ __global__ void vecnorm_kernel(cplx* const* __restrict__ Xs, int n) {
 
 template <int RV>
 void launch_hess_smem(cplx* const* H, cplx* const* Z, int batch, int n, cudaStream_t st) {
-  const size_t smem = ((size_t)(n + HESS_WARPS + 2) * 8 * RV + HESS_WARPS) * sizeof(cplx);
+  const size_t smem = ((size_t)(n + HESS_WARPS + 2) * (RV == 15 ? n : 8 * RV) + HESS_WARPS) * sizeof(cplx);
   ensure_smem((const void*)hess_smem_kernel<RV>, smem);
   hess_smem_kernel<RV><<<batch, HESS_THREADS, smem, st>>>(H, Z, n);
 }
@@ -489,7 +494,8 @@ void hessenberg_batched(cplx* const* d_H, cplx* const* d_Z, int batch, int n, cu
     else if (n <= 64) launch_hess_smem<8>(d_H, d_Z, batch, n, st);
     else if (n <= 80) launch_hess_smem<10>(d_H, d_Z, batch, n, st);
     else if (n <= 96) launch_hess_smem<12>(d_H, d_Z, batch, n, st);
-    else launch_hess_smem<14>(d_H, d_Z, batch, n, st);
+    else if (n <= 112) launch_hess_smem<14>(d_H, d_Z, batch, n, st);
+    else launch_hess_smem<15>(d_H, d_Z, batch, n, st);
     VRC_CUDA_CHECK(cudaGetLastError());
     return;
   }
