@@ -531,8 +531,8 @@ def roofline_of(stats, fp64_peak):
               key=lambda kv: kv[1].get("busy_ms") or kv[1]["ms"])
     hbm_peak, hbm_src = measured_peaks()
     name, f = fam
-    limiter = {"zgemm": "FP64 DMMA tensor pipe", "zinv": "panel reduction (latency) + DMMA rank-32 updates",
-               "hessenberg": "cluster barriers per column (latency)",
+    limiter = {"zgemm": "FP64 DMMA tensor pipe", "zinv": "panel reduction (latency) + DMMA rank-16 updates",
+               "hessenberg": "a column's reflector and barriers (latency)",
                "schur_qr": "sequential bulge chase (latency)", "schur_replay": "FP64 pipe / memory latency",
                "trevc": "sequential back substitution (latency)"}.get(name, "HBM bandwidth")
     traffic = profiled_traffic(name, f["flops"] / max(f["launches"], 1))
