@@ -27,6 +27,17 @@ def test_pq(ctx, npy, npx, nx, ny):
         assert relerr(P[k], oP) < 1e-12 and relerr(Q[k], oQ) < 1e-12
 
 
+@pytest.mark.parametrize("npy,npx,nx,ny", [(33, 70, 3, 5), (64, 17, 9, 1)])
+def test_many_samples(ctx, npy, npx, nx, ny):
+    """The Fourier products of many samples at once, bit for bit those of one."""
+    rng = np.random.default_rng(npx)
+    eps = rng.uniform(2.0, 12.0, (npy, npx)) + 1j * rng.uniform(0.0, 0.5, (npy, npx))
+    d = dict(kind="pixels", lam=1.1, nx=nx, ny=ny, pml=False, Lx=0.9, Ly=0.7, eps=eps, z0=0.0, z1=0.4)
+    P, Q = ctx.sample_pq(d, [0.1])
+    Pm, Qm = ctx.sample_pq(d, np.linspace(0.0, 0.4, 160))
+    assert all(np.array_equal(x, P[0]) for x in Pm) and all(np.array_equal(x, Q[0]) for x in Qm)
+
+
 @pytest.mark.parametrize("nx,ny", [(7, 9), (11, 3), (1, 13), (15, 1), (1, 17), (23, 1), (1, 25), (31, 1), (33, 1), (1, 41),
                                    (63, 1)])
 def test_toeplitz_orders(ctx, nx, ny):

@@ -167,16 +167,17 @@ __global__ void reciprocal_kernel(cplx* const* __restrict__ in, cplx* const* __r
 // Batched contraction C[M x N] = A[M x K] * op(B), column-major, of the Fourier
 // stages (M harmonics, N strips, K pixels: 13..29 x 256 x 256 for a pillar's
 // raster).  transB = 0: B is K x N (ldb); transB = 1: B is N x K (ldb), use B^T.
-// A CTA computes SG_M x SG_N, a row and four columns per thread, its operands
-// staged through shared memory in slices of SG_K, three in flight.  Per slice
-// entry a warp has 16 FP64 instructions to five shared loads, so the FP64 pipe
-// and the shared-memory port are about level.  One thread per output, its
-// operands from global memory one k at a time, waited for memory at every step:
-// 94 us for three samples of 256 x 256 pixels at 7 orders.
+// A CTA computes SG_M x 16 NQ, a row and NQ columns per thread, its operands
+// staged through shared memory in slices of SG_K, ST in flight.  With NQ = 4 a
+// warp has 16 FP64 instructions to five shared loads per slice entry, so the FP64
+// pipe and the shared-memory port are about level; where tiles of 64 columns do
+// not give every SM a CTA, NQ = 1 shortens each CTA's chain and spreads it (few
+// samples of 256 x 256 pixels at 7 orders: 14 and 19 us a launch, transposed or
+// not, against 20 and 24).  One thread per output, its operands from global memory
+// one k at a time, waited for memory at every step: 94 us for three such samples.
 // ---------------------------------------------------------------------------
-constexpr int SG_M = 16, SG_N = 64, SG_K = 16, SG_ST = 3, SG_THREADS = 256;
-constexpr int SG_LDB = SG_N + 1;
-constexpr size_t SG_SMEM = (size_t)SG_ST * SG_K * (SG_M + SG_LDB) * sizeof(cplx);
+constexpr int SG_M = 16, SG_K = 16, SG_THREADS = 256;
+constexpr size_t sg_smem(int nq, int stages) { return (size_t)stages * SG_K * (SG_M + 16 * nq + 1) * sizeof(cplx); }
 
 __device__ __forceinline__ void sg_copy(cplx* s, const cplx* g, bool on) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(s);
@@ -184,10 +185,11 @@ __device__ __forceinline__ void sg_copy(cplx* s, const cplx* g, bool on) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(a), "l"(g), "r"(sz) : "memory");
 }
 
-template <int TRANSB>
+template <int TRANSB, int NQ, int SG_ST>
 __global__ void __launch_bounds__(SG_THREADS)
     small_gemm_kernel(int M, int N, int K, const cplx* const* __restrict__ As, int lda,
                       const cplx* const* __restrict__ Bs, int ldb, cplx* const* __restrict__ Cs, int ldc) {
+  constexpr int SG_N = 16 * NQ, SG_LDB = SG_N + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx* sa = reinterpret_cast<cplx*>(smem_raw);  // [SG_ST][SG_K][SG_M]
   cplx* sb = sa + SG_ST * SG_K * SG_M;           // [SG_ST][SG_K][SG_LDB]
@@ -213,9 +215,9 @@ __global__ void __launch_bounds__(SG_THREADS)
       sg_copy(sb + (st * SG_K + k) * SG_LDB + c, on ? B + at : B, on);
     }
   };
-  cplx acc[4];
+  cplx acc[NQ];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) acc[q] = mk(0.0, 0.0);
+  for (int q = 0; q < NQ; ++q) acc[q] = mk(0.0, 0.0);
 #pragma unroll
   for (int s = 0; s < SG_ST - 1; ++s) {
     if (s < KT) load(s);
@@ -233,12 +235,12 @@ __global__ void __launch_bounds__(SG_THREADS)
     for (int k = 0; k < kn; ++k) {
       const cplx x = a[k * SG_M + i];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] = cfma(x, b[k * SG_LDB + jg + 16 * q], acc[q]);
+      for (int q = 0; q < NQ; ++q) acc[q] = cfma(x, b[k * SG_LDB + jg + 16 * q], acc[q]);
     }
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < NQ; ++q) {
     const int j = n0 + jg + 16 * q;
     if (m0 + i < M && j < N) C[(size_t)j * ldc + m0 + i] = acc[q];
   }
@@ -540,13 +542,32 @@ void reciprocal(cplx* const* d_in, cplx* const* d_out, int batch, int total, cud
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 
+static int sm_count() {
+  static const int sms = [] {
+    int dev = 0, v = 0;
+    VRC_CUDA_CHECK(cudaGetDevice(&dev));
+    VRC_CUDA_CHECK(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+    return v;
+  }();
+  return sms;
+}
+
 void small_gemm(int M, int N, int K, const cplx* const* d_A, int lda, const cplx* const* d_B, int ldb, int transB,
                 cplx* const* d_C, int ldc, int batch, cudaStream_t st) {
   if (batch <= 0) return;
-  auto kern = transB ? small_gemm_kernel<1> : small_gemm_kernel<0>;
-  ensure_smem((const void*)kern, SG_SMEM);
-  const int tiles = ((M + SG_M - 1) / SG_M) * ((N + SG_N - 1) / SG_N);
-  kern<<<dim3(tiles, batch), SG_THREADS, SG_SMEM, st>>>(M, N, K, d_A, lda, d_B, ldb, d_C, ldc);
+  const int rows = (M + SG_M - 1) / SG_M;
+  const auto run = [&](auto kern, int nq, int stages) {
+    ensure_smem((const void*)kern, sg_smem(nq, stages));
+    const int tiles = rows * ((N + 16 * nq - 1) / (16 * nq));
+    kern<<<dim3(tiles, batch), SG_THREADS, sg_smem(nq, stages), st>>>(M, N, K, d_A, lda, d_B, ldb, d_C, ldc);
+  };
+  if ((long long)rows * ((N + 63) / 64) * batch >= sm_count()) {
+    if (transB) run(small_gemm_kernel<1, 4, 3>, 4, 3);
+    else run(small_gemm_kernel<0, 4, 3>, 4, 3);
+  } else {
+    if (transB) run(small_gemm_kernel<1, 1, 6>, 1, 6);
+    else run(small_gemm_kernel<0, 1, 6>, 1, 6);
+  }
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 

@@ -2,7 +2,8 @@
 // CTA per matrix, replacing LAPACKE_zgeev / magma_zgeev of the reference
 // (src/rcwa/MKLEigenSolver.hpp:45-55, src/gpu/RedhefferIntegratorGPU.cpp:220-223).
 //
-//   1. hess_kernel   Householder reduction to upper Hessenberg form
+//   1. hess_smem_kernel, hess_kernel
+//                    Householder reduction to upper Hessenberg form
 //                    (H = Q^H A Q) with the left and right reflector
 //                    applications fused into one rank-2 update per column,
 //                    then backward accumulation of Q.
