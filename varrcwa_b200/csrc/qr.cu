@@ -103,23 +103,13 @@ __device__ __forceinline__ cplx* log_rot(char* logb, int sweep_cap) {
 // dependent FMAs per application against three here) is a longer serial
 // chain at every step.  Outside the range where the squares neither over- nor
 // underflow the pair is scaled first.
-// 1 / sqrt(x) for x well inside the normal range: the hardware's double
-// approximation, then one step of Halley's (cubic) iteration,
-// y (1 + e/2 + 3/8 e^2) with e = 1 - x y^2.
-__device__ __forceinline__ double rsqrt_inrange(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-x * y, y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 struct Rot {
   double c;
   cplx s, r;
 };
 __device__ __forceinline__ Rot givens(cplx f, cplx g) {
   Rot o;
-  const double f2 = cabs2(f), d2 = f2 + cabs2(g), u = rsqrt_inrange(f2 * d2);
+  const double f2 = cabs2(f), d2 = f2 + cabs2(g), u = rsqrt(f2 * d2);
   o.c = f2 * u;
   o.s = cscale(cmul(f, cconj(g)), u);
   o.r = cscale(f, d2 * u);
@@ -160,7 +150,7 @@ __device__ __forceinline__ void rotate2(cplx& a, cplx& b, double c, cplx s) {
 // Principal square root of a value whose square is within range.
 __device__ __forceinline__ cplx csqrt_inrange(cplx a) {
   const double a2 = cabs2(a);
-  const double q = 0.5 * fma(a2, rsqrt_inrange(a2), fabs(a.x)), iq = rsqrt_inrange(q), t = q * iq;
+  const double q = 0.5 * fma(a2, rsqrt(a2), fabs(a.x)), iq = rsqrt(q), t = q * iq;
   const double o = 0.5 * a.y * iq;
   return a.x >= 0.0 ? mk(t, o) : mk(fabs(o), copysign(t, a.y));
 }
@@ -188,7 +178,7 @@ __device__ __forceinline__ cplx wilkinson(cplx p, cplx q, cplx r, cplx t) {
   const cplx den = cadd(x, w);
   const double d2 = cabs2(den);
   if (!(d2 > 1e-280)) return t;
-  const double rd = rsqrt_inrange(d2);
+  const double rd = rsqrt(d2);
   return csub(t, cscale(cmul(qr, cconj(den)), big * rd * rd));
 }
 
