@@ -162,3 +162,101 @@ def test_shifted_symmetry_takes_the_general_way(ctx, monkeypatch):
     b = ctx.redheffer([d], pe=1e-2)[0]
     for k in ("Tdd", "Tuu", "Rud", "Rdu"):
         assert np.array_equal(a[k], b[k])
+
+
+def _rim_pillar():
+    """A pillar whose rim runs through pixel centres: by the rounding of
+    x^2 + y^2 a centre lies inside and one of its mirror images outside.  Held
+    to for every way a compiler may contract the raster's arithmetic."""
+    from fractions import Fraction
+    Lx, Ly, n = 0.41, 0.46, 59
+
+    def fma(a, b, c):
+        return float(Fraction(a) * Fraction(b) + Fraction(c))
+
+    def coord(i, L, fused):
+        h = L / n
+        return fma(i + 0.5, h, -0.5 * L) if fused else (i + 0.5) * h - 0.5 * L
+
+    def ranges(c, r):
+        for fused in (False, True):
+            d = {0: [], 1: [], 2: []}
+            for i in (c, n - 1 - c):
+                for j in (r, n - 1 - r):
+                    x, y = coord(i, Lx, fused), coord(j, Ly, fused)
+                    d[0].append(x * x + y * y)
+                    d[1].append(fma(x, x, y * y))
+                    d[2].append(fma(y, y, x * x))
+            yield from ((min(v), max(v)) for v in d.values())
+
+    for c in range(13, 22):
+        for r in range(13, 22):
+            lohi = list(ranges(c, r))
+            lo, hi = max(a for a, _ in lohi), min(b for _, b in lohi)
+            radius = np.sqrt(0.5 * (lo + hi))
+            for _ in range(5):
+                radius = np.nextafter(radius, 0.0)
+            for _ in range(10):
+                if lo <= radius * radius < hi:
+                    radius = float(radius)
+                    return _pillar(7, 5, 3, npx=n, npy=n, r0=radius, r1=radius, z1=0.2)
+                radius = np.nextafter(radius, 1.0)
+    raise AssertionError("no such radius")
+
+
+def test_rim_pillar_is_asymmetric(ctx):
+    d = _rim_pillar()
+    P, Q = ctx.sample_pq(d, [0.1])
+    m = d["nx"] * d["ny"]
+    a, b = np.divmod(np.arange(m), d["ny"])
+    worst = 0.0
+    for perm in ((d["nx"] - 1 - a) * d["ny"] + b, a * d["ny"] + d["ny"] - 1 - b):
+        q = np.concatenate([perm, m + perm])
+        for M in (P[0], Q[0]):
+            worst = max(worst, np.abs(np.abs(M[np.ix_(q, q)]) - np.abs(M)).max() / np.abs(M).max())
+    assert worst > 1e-6
+
+
+def _same_bits(a, b, keys):
+    return all(np.array_equal(a[k], b[k]) for k in keys)
+
+
+@pytest.mark.parametrize("max_depth", [1, 2])
+@pytest.mark.parametrize("call", ["redheffer", "redheffer_forward", "order_powers"])
+def test_late_asymmetry_with_a_capped_depth(ctx, monkeypatch, call, max_depth):
+    """Found asymmetric below the root, in a tree that ends at its depth limit
+    above the tolerance: bit for bit the general way's best effort."""
+    out = []
+    for env in (None, "1"):
+        monkeypatch.delenv("VRC_NO_FOLD", raising=False) if env is None else monkeypatch.setenv("VRC_NO_FOLD", env)
+        r = getattr(ctx, call)([_almost()], pe=1e-9, max_depth=max_depth)
+        out.append(((r[0] if isinstance(r, tuple) else r)[0], ctx.tree(0)))
+    (a, ta), (b, tb) = out
+    assert a["status"] == b["status"] == 8
+    assert _same_bits(a, b, ("R", "T") if call == "order_powers" else ("Tdd", "Tuu", "Rud", "Rdu", "W0", "W1"))
+    assert ta == tb
+
+
+@pytest.mark.parametrize("beside", [False, True])
+@pytest.mark.parametrize("make", [_almost, _rim_pillar])
+@pytest.mark.parametrize("call", ["order_powers", "blocks"])
+@pytest.mark.parametrize("method", ["redheffer", "rcwa", "differential"])
+def test_late_asymmetry(ctx, monkeypatch, method, call, make, beside):
+    """Found asymmetric during the solve, alone and beside cells that are
+    symmetric: bit for bit the general way's result."""
+    cells = [make()]
+    if beside:
+        cells = [_mesa(), make(), _pillar(31, 5, 3, z1=0.12), make()]
+    out = []
+    for env in (None, "1"):
+        monkeypatch.delenv("VRC_NO_FOLD", raising=False) if env is None else monkeypatch.setenv("VRC_NO_FOLD", env)
+        if call == "order_powers":
+            out.append(ctx.order_powers(cells, method=method, pe=1e-2, nslices=8))
+        else:
+            out.append(ctx.redheffer(cells, pe=1e-2) if method == "redheffer" else getattr(ctx, method)(cells, 8))
+    for c in ((0,) if not beside else (1, 3)):
+        a, b = out[0][c], out[1][c]
+        assert a["status"] == b["status"] == 0
+        assert _same_bits(a, b, ("R", "T") if call == "order_powers" else ("Tdd", "Tuu", "Rud", "Rdu", "W0", "W1"))
+        if call == "blocks":
+            assert all(a[k] == b[k] for k in ("N", "n_eig", "n_samples", "n_nodes"))

@@ -59,10 +59,14 @@ struct Book {
   // cells come four at a time, the parity classes of one mirror-symmetric
   // cell: n is the folded order, a sample is assembled once for all four
   bool folded = false;
+  // of every such cell: whether a section turned out without the mirror planes.
+  // Apart from the status, which later stages write; nothing takes it back.
+  std::vector<char> asym;
 
   Book(Engine& e, int n_, const std::vector<CellSpec>& c, std::vector<Engine::CellDev*>& cd)
       : E(e), n(n_), cells(c), cds(cd) {}
 
+  bool asymmetric(int cell) const { return folded && asym[cell / 4]; }
   int sample(int cell, double z, bool homog = false, cplx eps_h = mk(1, 0)) {
     S.push_back({cell, z, homog, eps_h, E.mat(n), E.mat(n), 0});
     pend_samples.push_back((int)S.size() - 1);
@@ -132,8 +136,10 @@ struct Book {
           const SampleB& b = S[s];
           const CellSpec& c = cells[b.cell];
           fd[{c.nx, c.ny}].push_back({sr[g - g0].P, sr[g - g0].Q, b.P, b.Q, c.k0() * c.k0(), b.cell % 4});
-          if (st[g - g0]) cell_status[b.cell] = st[g - g0];
-          if (!b.homog && c.kind != GEOM_PILLAR && !c.mirrored(b.z)) cell_status[b.cell] = ST_ASYMMETRIC;
+          if (st[g - g0] == ST_ASYMMETRIC || (!b.homog && c.kind != GEOM_PILLAR && !c.mirrored(b.z)))
+            asym[b.cell / 4] = 1;
+          else if (st[g - g0])
+            cell_status[b.cell] = st[g - g0];
         }
       for (auto& kv : fd) {
         const FoldDesc* d = E.upload(kv.second);
@@ -290,6 +296,7 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
     Book bk(*this, n, sub, cds);
     bk.out = &res;
     bk.folded = folded != 0;
+    bk.asym.assign(sub.size() / 4 + 1, 0);
     bk.cell_status.assign(sub.size(), ST_OK);
     const int C = (int)sub.size();
     std::vector<NodeB> N;
@@ -336,6 +343,29 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
       }
     }
     bk.flush();
+    // An asymmetric cell's classes are not a problem worth solving: its tree ends
+    // here, and the caller takes it the general way.
+    auto drop_asymmetric = [&] {
+      if (!folded) return;
+      for (int id : active) {
+        const NodeB& nd = N[id];
+        if (!bk.asymmetric(nd.cell)) continue;
+        bk.release_sample(nd.sa);
+        bk.release_sample(nd.sm);
+        bk.release_sample(nd.sb);
+      }
+      active.erase(std::remove_if(active.begin(), active.end(), [&](int id) { return bk.asymmetric(N[id].cell); }),
+                   active.end());
+      for (int c = 0; c < C; ++c) {
+        if (!bk.asymmetric(c)) continue;
+        for (int id : order[c]) {
+          free_mat(N[id].tdd, n); free_mat(N[id].tuu, n); free_mat(N[id].rud, n); free_mat(N[id].rdu, n);
+          bk.release_ref(N[id].ref);
+        }
+        order[c].clear();
+      }
+    };
+    drop_asymmetric();
     const bool replay = (o.cuts != nullptr);
     while (!active.empty()) {
       // Evaluate every open node of this level.
@@ -423,6 +453,7 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
       }
       bk.flush();
       active.swap(next);
+      drop_asymmetric();
     }
     // Left-end projections of all leaves onto their predecessors' bases.
     std::vector<ProjReq> pr;
@@ -485,7 +516,7 @@ void Engine::redheffer(const std::vector<CellSpec>& cells, const RedhefferOpts& 
       }
       bk.export_basis(e0[c], r.W0, r.V0, r.gam0, r.W0inv);
       bk.export_basis(e1[c], r.W1, r.V1, r.gam1, r.W1inv);
-      r.status = bk.cell_status[c];
+      r.status = bk.asymmetric(c) ? (int)ST_ASYMMETRIC : bk.cell_status[c];
     }
     // samples still referenced by end bases
     for (size_t s = 0; s < bk.S.size(); ++s)
@@ -519,6 +550,7 @@ void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellR
     Book bk(*this, n, sub, cds);
     bk.out = &res;
     bk.folded = folded != 0;
+    bk.asym.assign(sub.size() / 4 + 1, 0);
     const int C = (int)sub.size();
     bk.cell_status.assign(C, ST_OK);
     std::vector<int> e0(C), e1(C);
@@ -542,7 +574,7 @@ void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellR
     std::vector<std::vector<SBlocks>> lists(C);
     std::vector<int> sl_cell;
     for (int c = 0; c < C; ++c) {
-      if (!excited(c, folded)) continue;
+      if (!excited(c, folded) || bk.asymmetric(c)) continue;
       const CellSpec& s = sub[c];
       const double dz = (s.z1 - s.z0) / (double)Nsl;
       for (int si : slices[c]) {
@@ -584,11 +616,13 @@ void Engine::rcwa(const std::vector<CellSpec>& cells, int Nsl, std::vector<CellR
       if (pst[i]) bk.cell_status[pl_cell[i]] = pst[i];
     for (int c = 0; c < C; ++c) {
       CellResult& r = res[c];
-      if (lists[c].empty()) continue;
-      r.Tdd = lists[c][0].tdd; r.Tuu = lists[c][0].tuu; r.Rud = lists[c][0].rud; r.Rdu = lists[c][0].rdu;
+      if (!excited(c, folded)) continue;
+      if (!lists[c].empty()) {
+        r.Tdd = lists[c][0].tdd; r.Tuu = lists[c][0].tuu; r.Rud = lists[c][0].rud; r.Rdu = lists[c][0].rdu;
+      }
       bk.export_basis(e0[c], r.W0, r.V0, r.gam0, r.W0inv);
       bk.export_basis(e1[c], r.W1, r.V1, r.gam1, r.W1inv);
-      r.status = bk.cell_status[c];
+      r.status = bk.asymmetric(c) ? (int)ST_ASYMMETRIC : bk.cell_status[c];
     }
     for (size_t s = 0; s < bk.S.size(); ++s)
       if (bk.S[s].P) { free_mat(bk.S[s].P, n); free_mat(bk.S[s].Q, n); }
@@ -618,6 +652,7 @@ void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vect
     Book bk(*this, n, sub, cds);
     bk.out = &res;
     bk.folded = folded != 0;
+    bk.asym.assign(sub.size() / 4 + 1, 0);
     const int C = (int)sub.size();
     bk.cell_status.assign(C, ST_OK);
     std::vector<int> e0(C), e1(C);
@@ -648,7 +683,7 @@ void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vect
     std::vector<std::vector<SBlocks>> lists(C);
     std::vector<int> dr_cell;
     for (int c = 0; c < C; ++c) {
-      if (!excited(c, folded)) continue;
+      if (!excited(c, folded) || bk.asymmetric(c)) continue;
       const CellSpec& s = sub[c];
       const double dz = (s.z1 - s.z0) / (double)Nsl;
       const RefB& b1 = bk.R[e1[c]];
@@ -683,11 +718,13 @@ void Engine::differential(const std::vector<CellSpec>& cells, int Nsl, std::vect
       if (pst[i]) bk.cell_status[pl_cell[i]] = pst[i];
     for (int c = 0; c < C; ++c) {
       CellResult& r = res[c];
-      if (lists[c].empty()) continue;
-      r.Tdd = lists[c][0].tdd; r.Tuu = lists[c][0].tuu; r.Rud = lists[c][0].rud; r.Rdu = lists[c][0].rdu;
+      if (!excited(c, folded)) continue;
+      if (!lists[c].empty()) {
+        r.Tdd = lists[c][0].tdd; r.Tuu = lists[c][0].tuu; r.Rud = lists[c][0].rud; r.Rdu = lists[c][0].rdu;
+      }
       bk.export_basis(e0[c], r.W0, r.V0, r.gam0, r.W0inv);
       bk.export_basis(e1[c], r.W1, r.V1, r.gam1, r.W1inv);
-      r.status = bk.cell_status[c];
+      r.status = bk.asymmetric(c) ? (int)ST_ASYMMETRIC : bk.cell_status[c];
     }
     for (size_t s = 0; s < bk.S.size(); ++s)
       if (bk.S[s].P) { free_mat(bk.S[s].P, n); free_mat(bk.S[s].Q, n); }
@@ -843,7 +880,8 @@ struct Held {  // device blocks of solves, given back also on errors
     for (auto& x : r) E.release_result(x);
   }
 };
-// Status of a cell from those of its classes; false: not symmetric after all.
+// Status of a cell from those of its classes; false: not symmetric after all
+// (its classes then have no blocks).
 bool class_status(const std::vector<CellResult>& r, size_t i, int* status) {
   *status = ST_OK;
   for (int k = 0; k < 4; ++k) {
@@ -1024,18 +1062,25 @@ void Engine::solve_powers(const std::vector<CellSpec>& cells, int method, const 
     }
     Held h{*this, {}};
     solve(four, method, o, nslices, h.r, FOLD_EXCITED);
-    std::vector<std::vector<double>> Rm, Tm;
-    order_powers(one, h.r, side, flux_norm, Rm, Tm, FOLD_EXCITED);
+    std::vector<int> pick;
+    std::vector<CellSpec> ps;
+    std::vector<CellResult> pr;  // (h keeps the blocks)
     for (size_t i = 0; i < mirrored.size(); ++i) {
-      const int c = mirrored[i];
       int status;
       if (!class_status(h.r, i, &status)) {
-        general.push_back(c);
+        general.push_back(mirrored[i]);
         continue;
       }
-      R[c] = std::move(Rm[i]);
-      T[c] = std::move(Tm[i]);
-      copy_counts(res[c], h.r[4 * i], status);
+      copy_counts(res[mirrored[i]], h.r[4 * i], status);
+      pick.push_back(mirrored[i]);
+      ps.push_back(one[i]);
+      pr.insert(pr.end(), h.r.begin() + 4 * i, h.r.begin() + 4 * i + 4);
+    }
+    std::vector<std::vector<double>> Rm, Tm;
+    order_powers(ps, pr, side, flux_norm, Rm, Tm, FOLD_EXCITED);
+    for (size_t i = 0; i < pick.size(); ++i) {
+      R[pick[i]] = std::move(Rm[i]);
+      T[pick[i]] = std::move(Tm[i]);
     }
   }
   if (general.empty()) return;

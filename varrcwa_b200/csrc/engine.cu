@@ -1013,7 +1013,6 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
         dstat = (int*)bytes(B * sizeof(int));
         VRC_CUDA_CHECK(cudaMemsetAsync(dstat, 0, B * sizeof(int), stream_));
       }
-      if (k.pillar && k.mirrored && dstat) mirror_check(d_eps, (int)B, nc, nr, dstat, stream_);
       auto ex = ptrs(o_ex), exs = ptrs(o_exs), ey = ptrs(o_ey);
       twiddles(upload(xp), upload(ex), (int)B, ncx, P, stream_);
       twiddles(upload(xsp), upload(exs), (int)B, ncx, P, stream_);
@@ -1040,6 +1039,8 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
       auto fe11 = ptrs(o_fe11), fe22 = ptrs(o_fe22), fe33 = ptrs(o_fe33);
       gather_fe(upload(cst(g11)), upload(cst(g22)), upload(cst(f2)), upload(fe11), upload(fe22), upload(fe33), nx,
                 ny, (int)B, stream_);
+      // (after the inverses: an asymmetric raster stays one whatever they report)
+      if (k.pillar && k.mirrored && dstat) mirror_check(d_eps, (int)B, nc, nr, dstat, stream_);
       asm_prof.reset();
       // fe33^{-1} (BDCSVD solve of the square system, Layer.cpp:84-86)
       std::vector<int> inv_status;
