@@ -97,3 +97,20 @@ def test_equal_diagonals(ctx, n):
     A[8:, i, i + 1] = -1.85e-12 * 10.0 ** rng.uniform(-1, 1, (4, n // 2))
     A[8:, i + 1, i] = -1.05e-13 * 10.0 ** rng.uniform(-1, 1, (4, n // 2))
     _check(ctx, A)
+
+
+@pytest.mark.parametrize("n", [114, 115, 116])
+def test_reduction_at_the_end_of_shared_memory(ctx, monkeypatch, n):
+    """The reduction in shared memory takes every order whose matrix has room
+    there, (n + 10) n + 8 entries: bit for bit VRC_HESS_BLOCKED=0 up to it and
+    VRC_HESS_BLOCKED=1 above."""
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((4, n, n)) + 1j * rng.standard_normal((4, n, n))
+    A[1] = np.triu(A[1], -1)
+    A[2, 2:, : n // 2] = 0
+    A[3] = np.diag(np.diagonal(A[3]))
+    monkeypatch.delenv("VRC_HESS_BLOCKED", raising=False)
+    _check(ctx, A)
+    W = ctx.eig(A)[1]
+    monkeypatch.setenv("VRC_HESS_BLOCKED", "0" if 16 * ((n + 10) * n + 8) <= 227 * 1024 else "1")
+    assert np.array_equal(ctx.eig(A)[1], W)

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(HESS_THREADS)
   }
 }
 
-// The same reduction for n <= 113 with the matrix in shared memory, Q accumulated
+// The same reduction for n <= 115 with the matrix in shared memory, Q accumulated
 // in its place.  Eight lanes take a column (a row in eight each, the rows padded
 // with zeros to 8 RV) and the CTA 32 columns at a time: both products in one
 // pass, v^H a_j kept in registers for the update, and every warp forms the
@@ -204,9 +204,19 @@ __global__ void __launch_bounds__(HESS_THREADS)
 // A v, their sum, the next reflector's column).  Bound by that chain and, with
 // the SMs full, by shared memory and the FP64 pipe.  One / 600 matrices take
 // 0.11 / 0.37 ms at n = 42, 0.21 / 0.73 at 61 (hess_kernel 0.51 for some 60) and
-// 0.58 / 2.9 at 98 (panels and GEMM updates 0.93 / 4.1) and 0.75 / 3.8 at 113 (1.02 /
-// 5.1; there RV = 15 leaves the padding out, the only form that fits).
-constexpr int HS_MAXN = 113;  // (what shared memory holds)
+// 0.58 / 2.9 at 98 (panels and GEMM updates 0.93 / 4.1), 0.75 / 3.8 at 113 (1.00 /
+// 5.1) and 0.76 / 3.9 at 115 (1.02 / 5.3).  RV = 15 leaves the padding out, the only form that fits above 112 (a row
+// more in a lane, padded, holds 111).
+constexpr size_t hs_smem(int n, int rv) {
+  return ((size_t)(n + HESS_WARPS + 2) * (rv == 15 ? n : 8 * rv) + HESS_WARPS) * sizeof(cplx);
+}
+constexpr int hs_maxn() {  // the largest order whose matrix a CTA's shared memory holds
+  int n = 113;
+  while (hs_smem(n + 1, 15) <= (size_t)227 * 1024) ++n;
+  return n;
+}
+constexpr int HS_MAXN = hs_maxn();
+static_assert(HS_MAXN <= 8 * 15 && hs_smem(112, 14) <= (size_t)227 * 1024, "rows of the widest forms");
 
 __device__ __forceinline__ cplx shfl_xor(cplx z, int o) {
   return mk(__shfl_xor_sync(0xffffffffu, z.x, o), __shfl_xor_sync(0xffffffffu, z.y, o));
@@ -448,7 +458,7 @@ __global__ void vecnorm_kernel(cplx* const* __restrict__ Xs, int n) {
 
 template <int RV>
 void launch_hess_smem(cplx* const* H, cplx* const* Z, int batch, int n, cudaStream_t st) {
-  const size_t smem = ((size_t)(n + HESS_WARPS + 2) * (RV == 15 ? n : 8 * RV) + HESS_WARPS) * sizeof(cplx);
+  const size_t smem = hs_smem(n, RV);
   ensure_smem((const void*)hess_smem_kernel<RV>, smem);
   hess_smem_kernel<RV><<<batch, HESS_THREADS, smem, st>>>(H, Z, n);
 }
@@ -464,6 +474,8 @@ void launch_hess(cplx* const* H, cplx* const* Z, int batch, int n, cudaStream_t 
 }
 
 }  // namespace
+
+int hessenberg_smem_maxn() { return HS_MAXN; }
 
 void hessenberg_batched(cplx* const* d_H, cplx* const* d_Z, int batch, int n, cudaStream_t st) {
   if (batch <= 0) return;

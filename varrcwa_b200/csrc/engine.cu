@@ -1131,12 +1131,12 @@ void Engine::assemble_grid(std::vector<SampleReq>& reqs, std::vector<int>* statu
 // Blocked Hessenberg reduction (panels + DMMA GEMM updates) from the order up at
 // which the matrix no longer fits the shared memory of one CTA: one / 600
 // matrices in ms, shared memory against blocked, n = 61 0.21 / 0.73 against 0.49 /
-// 1.6, n = 98 0.58 / 2.9 against 0.93 / 4.1, n = 113 0.75 / 3.8 against 1.02 / 5.1;
+// 1.6, n = 98 0.58 / 2.9 against 0.93 / 4.1, n = 115 0.76 / 3.9 against 1.02 / 5.3;
 // from global memory, against blocked, 2.65 / 1.48 for eight at n = 126.
 // VRC_HESS_BLOCKED=0 / 1 turns it off / on for every order.
 static bool use_blocked_hessenberg(int n) {
   if (const char* e = std::getenv("VRC_HESS_BLOCKED")) return std::atoi(e) != 0 && n >= 3;
-  return n > 113;
+  return n > hessenberg_smem_maxn();
 }
 
 void Engine::eig(std::vector<EigReq>& reqs, int n, std::vector<int>* status) {

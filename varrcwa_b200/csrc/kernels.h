@@ -48,6 +48,8 @@ void zinv_blocked_batched(cplx* const* d_mats, int batch, int n, int* d_status, 
                           const GemmDesc* d_descs, cudaStream_t stream);
 
 // ---- eigensolver ---------------------------------------------------------------
+// hessenberg_batched keeps a matrix in one CTA's shared memory up to this order.
+int hessenberg_smem_maxn();
 void hessenberg_batched(cplx* const* d_H, cplx* const* d_Z, int batch, int n, cudaStream_t st);
 // The same reduction by one cluster of CTAs per matrix with the matrix in
 // distributed shared memory (hessenberg.cu); for n where it fits.
