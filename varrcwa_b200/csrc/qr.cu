@@ -582,12 +582,12 @@ __device__ __forceinline__ void far_strips(cplx* H, int n, const Chunk& ch, cplx
   }
 }
 
-// MINB: resident CTAs per SM the registers are sized for.  TEAM: a cluster per
+// Two CTAs per SM, which is what their shared memory allows.  TEAM: a cluster per
 // matrix.  Its first CTA iterates; the others wait for its chunks and take their
 // share of the strips outside D (at n = 450 on one CTA 44% of the iteration),
 // which changes nothing in the arithmetic.
-template <int MINB, bool TEAM>
-__global__ void __launch_bounds__(QR_THREADS, MINB)
+template <bool TEAM>
+__global__ void __launch_bounds__(QR_THREADS, 2)
     hqr_kernel(cplx* const* __restrict__ Hs, void* const* __restrict__ logs, cplx* const* __restrict__ Ws, int n,
                int sweep_cap, long long rot_cap, int* __restrict__ status, int aed_min, int aed_w) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1178,13 +1178,6 @@ static int team_size(int n, int batch) {
 void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* const* d_logs, int batch, int n,
                    int* d_status, cudaStream_t st, int parts) {
   if (batch <= 0) return;
-  // resident Schur CTAs per SM: 2 (default) or 3 (VRC_QR_CTAS=3); the
-  // arithmetic is the same, only the registers differ
-  static const int minb = [] {
-    const char* e = std::getenv("VRC_QR_CTAS");
-    return (e && std::atoi(e) == 3) ? 3 : 2;
-  }();
-  auto hqr = minb == 3 ? hqr_kernel<3, false> : hqr_kernel<2, false>;
   // Order of the deflation window (VRC_QR_AEDW, 4..32) and the order of the
   // active window from which it is taken (VRC_QR_AED; 0: never).  By default 10
   // and 48 for n > 128, never below: ms of iteration and replay for windows of
@@ -1202,7 +1195,7 @@ void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* c
     return e ? std::max(0, std::atoi(e)) : -1;
   }();
   const int aed_min = aed_env >= 0 ? aed_env : (n <= 128 ? 0 : 48);
-  ensure_smem((const void*)hqr, QR_SMEM);
+  ensure_smem((const void*)hqr_kernel<false>, QR_SMEM);
   const size_t rp_smem = replay_smem(n);
   const int rp_threads = 32 * replay_warps(n);
   ensure_smem((const void*)qr_replay_rows_kernel, rp_smem);
@@ -1216,7 +1209,7 @@ void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* c
       int* stat = d_status ? d_status + b0 : nullptr;
       const int team = team_size(n, nb);
       if (team > 1) {
-        ensure_smem((const void*)hqr_kernel<2, true>, QR_SMEM);
+        ensure_smem((const void*)hqr_kernel<true>, QR_SMEM);
         cudaLaunchConfig_t cfg{};
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1228,10 +1221,11 @@ void schur_batched(cplx* const* d_H, cplx* const* d_Z, cplx* const* d_W, void* c
         cfg.stream = st;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        VRC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, hqr_kernel<2, true>, d_H + b0, d_logs + b0, d_W + b0, n, cc, rc, stat,
+        VRC_CUDA_CHECK(cudaLaunchKernelEx(&cfg, hqr_kernel<true>, d_H + b0, d_logs + b0, d_W + b0, n, cc, rc, stat,
                                           aed_min, aed_w));
       } else {
-        hqr<<<nb, QR_THREADS, QR_SMEM, st>>>(d_H + b0, d_logs + b0, d_W + b0, n, cc, rc, stat, aed_min, aed_w);
+        hqr_kernel<false><<<nb, QR_THREADS, QR_SMEM, st>>>(d_H + b0, d_logs + b0, d_W + b0, n, cc, rc, stat, aed_min,
+                                                           aed_w);
       }
     }
     if (parts & SCHUR_REPLAY) {
