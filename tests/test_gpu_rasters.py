@@ -78,3 +78,44 @@ def test_differential_batch_of_unequal_slices(ctx):
         F = fourier_blocks(r)
         for k in F:
             assert relerr(F[k], G[k]) < 1e-9, k
+
+
+def _layers(nx, L, npix, seed, thick):
+    rng = np.random.default_rng(seed)
+    return dict(lam=0.9, Lx=0.7, Ly=0.7, nx=nx, ny=nx, layers=[rng.uniform(2.0, 4.0, (npix, npix)) for _ in range(L)],
+                thick=[thick] * L, eps_in=1.0, eps_out=2.085)
+
+
+def test_many_layers_in_groups(ctx):
+    """Two stacks of 130 layers, whose pixel gradients come in two groups, bit
+    for bit as each stack's alone, in one."""
+    ds = [_layers(3, 130, 6, seed, 0.004) for seed in (1, 2)]
+    w = np.zeros((2, 9))
+    w[:, 4] = 1.0
+    ctx.stack_forward(ds)
+    g, gt = ctx.stack_backward(0.5 * w, w, want_thick=True)
+    for k in range(2):
+        ctx.stack_forward(ds[k:k + 1])
+        g1, gt1 = ctx.stack_backward(0.5 * w[:1], w[:1], want_thick=True)
+        assert np.abs(g1).max() > 0 and np.array_equal(g[k], g1[0]) and np.array_equal(gt[k], gt1[0])
+
+
+def test_memory_of_many_layers():
+    """What the backward pass of five stacks of 200 layers adds to the kept
+    forward pass, in pool chunks: up to two of 64 MB for some 150 matrices of
+    order 162, four of 27 MB for the block adjoints of a group of 255 layers, two
+    of 64 MB for the groups' scratch and the gradients, and small ones; twelve of
+    27 MB if the block adjoints of all 1000 layers were kept."""
+    import torch
+    from varrcwa_b200.capi import Context
+    c = Context(0)
+    try:
+        w = np.zeros((5, 81))
+        w[:, 40] = 1.0
+        c.stack_forward([_layers(9, 200, 16, seed, 0.001) for seed in range(5)])
+        before = torch.cuda.mem_get_info()[0]
+        c.stack_backward(w, w)
+        grown = before - torch.cuda.mem_get_info()[0]
+    finally:
+        c.close()
+    assert grown < 400 << 20

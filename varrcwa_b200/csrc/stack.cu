@@ -345,7 +345,11 @@ void Engine::stack_backward(const double* wR, const double* wT, double* grad, do
   double* dgrad = (double*)bytes((size_t)C * L * npx * npy * 8);
   double* dthick = (double*)bytes((size_t)C * L * 8);
   const size_t kper = pixel_adjoint_scratch(tp.nx, tp.ny);
-  char* kscr = (char*)bytes((size_t)C * L * kper);
+  // The pixels' part waits until the block adjoints of a group of layers are
+  // there: some 256 stack layers, whose strips fill the GPU several times over,
+  // so that its memory does not grow with the layer count.
+  const int LG = std::min(L, std::max(1, 256 / C));
+  char* kscr = (char*)bytes((size_t)C * LG * kper);
   Vec GP[4];
   for (auto& g : GP) g = bt.alloc(n);
   Vec gs[4];
@@ -353,10 +357,10 @@ void Engine::stack_backward(const double* wR, const double* wT, double* grad, do
   Vec C1 = bt.alloc(n), C1r = bt.alloc(n), C2 = bt.alloc(n), X1 = bt.alloc(n), X2 = bt.alloc(n), Y = bt.alloc(n),
       Zm = bt.alloc(n), RC1 = bt.alloc(n), U = bt.alloc(n), gC1 = bt.alloc(n), gC2 = bt.alloc(n), T4 = bt.alloc(n);
   Vec Zq = bt.alloc(m), Tm = bt.alloc(m);
-  // the pixels' part waits until every layer's block adjoints are there
-  std::vector<Vec> g11(L), g22(L), g33(L);
-  for (int l = 0; l < L; ++l) g11[l] = bt.alloc(m), g22[l] = bt.alloc(m), g33[l] = bt.alloc(m);
+  std::vector<Vec> g11(LG), g22(LG), g33(LG);
+  for (int s = 0; s < LG; ++s) g11[s] = bt.alloc(m), g22[s] = bt.alloc(m), g33[s] = bt.alloc(m);
   for (int l = L - 1; l >= 0; --l) {
+    const int slot = (L - 1 - l) % LG;
     Vec pr[4], sg[4];
     for (int k = 0; k < 4; ++k) {
       pr[k] = gather([&](StackCell& s) { return s.lay[l].pre[k]; });
@@ -455,24 +459,25 @@ void Engine::stack_backward(const double* wR, const double* wT, double* grad, do
     {
       std::vector<PQAdjDesc> qd(C);
       for (int c = 0; c < C; ++c)
-        qd[c] = {T2[c], T3[c], tp.cells[c].alpha, tp.cells[c].beta, g11[l][c], g22[l][c], Zq[c],
+        qd[c] = {T2[c], T3[c], tp.cells[c].alpha, tp.cells[c].beta, g11[slot][c], g22[slot][c], Zq[c],
                  2.0 * 3.1415926535897932 / tp.specs[c].lambda};
       Prof pr(*this, "adjoint", 0.0, 16.0 * (2.0 * n * n + 3.0 * m * m) * C);
       pq_adjoint_batched(upload(qd), C, m, stream_);
     }
     Vec fi = gather([&](StackCell& s) { return s.lay[l].fe33inv; });
     bt.mm(Tm, Zq, fi, ONE, 0, 1, nullptr, ZERO, m);                    // Z fe33^-H
-    bt.mm(g33[l], fi, Tm, MONE, 1, 0, nullptr, ZERO, m);               // g33 = -fe33^-H Z fe33^-H
+    bt.mm(g33[slot], fi, Tm, MONE, 1, 0, nullptr, ZERO, m);            // g33 = -fe33^-H Z fe33^-H
     for (int k = 0; k < 4; ++k) std::swap(G[k], GP[k]);
-  }
-  {
-    std::vector<PixAdjDesc> xd;
+    if (slot + 1 < LG && l > 0) continue;
+    std::vector<PixAdjDesc> xd;  // the layers of slots 0 .. slot: l + slot .. l
     for (int c = 0; c < C; ++c)
-      for (int l = 0; l < L; ++l)
-        xd.push_back({tp.cells[c].lay[l].eps, g11[l][c], g22[l][c], g33[l][c], dgrad + ((size_t)c * L + l) * npx * npy,
-                      reinterpret_cast<cplx*>(kscr + ((size_t)c * L + l) * kper), tp.specs[c].Lx, tp.specs[c].Ly});
-    Prof pr(*this, "adjoint", 0.0, 16.0 * (3.0 * m * m + (double)npx * npy) * C * L, 3);
-    pixel_adjoint_batched(upload(xd), C * L, tp.nx, tp.ny, npx, npy, stream_);
+      for (int s = 0; s <= slot; ++s) {
+        const int q = l + slot - s;
+        xd.push_back({tp.cells[c].lay[q].eps, g11[s][c], g22[s][c], g33[s][c], dgrad + ((size_t)c * L + q) * npx * npy,
+                      reinterpret_cast<cplx*>(kscr + ((size_t)c * LG + s) * kper), tp.specs[c].Lx, tp.specs[c].Ly});
+      }
+    Prof prof(*this, "adjoint", 0.0, 16.0 * (3.0 * m * m + (double)npx * npy) * xd.size(), 3);
+    pixel_adjoint_batched(upload(xd), (int)xd.size(), tp.nx, tp.ny, npx, npy, stream_);
   }
   std::vector<double> hg((size_t)C * L * npx * npy), ht((size_t)C * L);
   VRC_CUDA_CHECK(cudaMemcpyAsync(hg.data(), dgrad, hg.size() * 8, cudaMemcpyDeviceToHost, stream_));
@@ -482,7 +487,7 @@ void Engine::stack_backward(const double* wR, const double* wT, double* grad, do
   if (grad_thick) std::memcpy(grad_thick, ht.data(), ht.size() * 8);
   free_bytes(dgrad, (size_t)C * L * npx * npy * 8);
   free_bytes(dthick, (size_t)C * L * 8);
-  free_bytes(kscr, (size_t)C * L * kper);
+  free_bytes(kscr, (size_t)C * LG * kper);
   free_bytes(dw, (size_t)2 * C * m * 8);
   free_bytes(dR, (size_t)2 * C * m * 8);
   for (Vec* v : {&T1, &T2, &T3, &T4, &C1, &C1r, &C2, &X1, &X2, &Y, &Zm, &RC1, &U, &gC1, &gC2}) bt.release(*v, n);
@@ -492,8 +497,8 @@ void Engine::stack_backward(const double* wR, const double* wT, double* grad, do
     bt.release(gs[k], n);
   }
   for (Vec* v : {&Zq, &Tm}) bt.release(*v, m);
-  for (int l = 0; l < L; ++l)
-    for (Vec* v : {&g11[l], &g22[l], &g33[l]}) bt.release(*v, m);
+  for (int s = 0; s < LG; ++s)
+    for (Vec* v : {&g11[s], &g22[s], &g33[s]}) bt.release(*v, m);
 }
 
 }  // namespace vrc
