@@ -73,3 +73,18 @@ def test_singular(ctx, n):
     A[1] = np.eye(n)
     A[1, 5, 5] = 0.0
     assert list(ctx.zinv(A)[1]) == [4, 4]
+
+
+@pytest.mark.parametrize("n", [97, 130, 300, 530])
+def test_undefined_entries(ctx, n):
+    """Panels: infinite and undefined entries are reported for their own matrix
+    alone, wherever the entry's panel is."""
+    rng = np.random.default_rng(n)
+    G = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A = np.stack([G] * 7)
+    A[1, 1, 0] = np.inf
+    A[2, 5, n - 1] = np.nan
+    A[3, :, n // 2] = np.nan
+    A[4, n - 1, n // 2] = complex(0.0, np.inf)
+    A[5, :, n - 2] = 0.0
+    assert list(ctx.zinv(A)[1]) == [0, 4, 4, 4, 4, 4, 0]

@@ -533,8 +533,10 @@ void thick_adjoint_batched(const ThickAdjDesc* d, int batch, int n, cudaStream_t
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 
-// Rasters accepted: both directions' twiddle tables, the coefficients and one
-// strip's matrices within a CTA's shared memory, at most 32 harmonics an axis.
+// Rasters that stacks take, at most 32 harmonics an axis: the bound of a kernel
+// that held both directions' twiddle tables, the coefficients, one strip's
+// matrices and the raster's sums in one CTA's shared memory.  The strips above
+// hold one direction's table and what a warp needs, less at every size within it.
 bool pixel_adjoint_fits(int nx, int ny, int npx, int npy) {
   if (nx > 32 || ny > 32) return false;
   const int P = 2 * nx - 1, Q = 2 * ny - 1, t = nx > ny ? nx : ny;

@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(HB_THREADS)
         const int r = rl + RL * t;
         if (r >= J0 && r < n && g < G) {
           cplx a = g == 0 ? c[r] : zero;
-        for (int l = g; l < i; l += G) a = cfma(cneg(V[(size_t)l * n + r]), s_w2[l], a);
+          for (int l = g; l < i; l += G) a = cfma(cneg(V[(size_t)l * n + r]), s_w2[l], a);
           part[g * n + r] = a;
         }
       }

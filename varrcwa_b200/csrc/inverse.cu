@@ -104,17 +104,17 @@ __global__ void __launch_bounds__(32 * W)
       // the pivot's row, left empty (its lane adds 1 / pivot times it below)
 #pragma unroll
       for (int h = 0; h < R; ++h) {
-          const bool mine = lane + 32 * h == p;
-          if (R > 1 && !__any_sync(0xffffffffu, mine)) continue;
-          if (mine) {
+        const bool mine = lane + 32 * h == p;
+        if (R > 1 && !__any_sync(0xffffffffu, mine)) continue;
+        if (mine) {
 #pragma unroll
-            for (int d = 0; d < C; ++d) row[warp][d] = a[h][d];
-          }
-#pragma unroll
-          for (int d = 0; d < C; ++d) a[h][d] = mine ? zero : a[h][d];
-          used[h] = used[h] || mine;
-          step[h] = mine ? k : step[h];
+          for (int d = 0; d < C; ++d) row[warp][d] = a[h][d];
         }
+#pragma unroll
+        for (int d = 0; d < C; ++d) a[h][d] = mine ? zero : a[h][d];
+        used[h] = used[h] || mine;
+        step[h] = mine ? k : step[h];
+      }
       __syncwarp();
 #pragma unroll
       for (int cc = 0; cc < C; ++cc) {
@@ -162,7 +162,8 @@ __global__ void __launch_bounds__(32 * W)
 // The panel kernel holds a row (or RPT rows) per thread, so the multiplier of
 // a step is the thread's own register and a pivot passes one barrier: the
 // candidates are compared by their upper 32 bits (a pivot within 1e-6 of the
-// largest is as good) with one warp reduction each side of it, and every warp's
+// largest is as good; magnitudes below 4.2e-314, whose reciprocal overflows,
+// count as zero) with one warp reduction each side of it, and every warp's
 // candidate puts out its row and the reciprocal of its pivot before it is known
 // which one is taken.  Bound by that chain for few matrices and by the FP64
 // issue of the update for many.
