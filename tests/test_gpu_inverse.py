@@ -57,6 +57,21 @@ def test_small_pivots(ctx, n):
     assert list(ctx.zinv(A)[1]) == [0, 4, 4, 4, 0]
 
 
+@pytest.mark.parametrize("n", [1025, 1056, 2049, 2767])
+def test_beyond_structures(ctx, n):
+    """Orders that no structure has (six rows per thread, 4 columns): rows of a
+    diagonal in [1, 2] exchanged, and 0.1 / sqrt(n) of noise, whose 2-norm stays
+    below 0.3, so cond < 2.3 / 0.7 < 4.  The next order is refused."""
+    rng = np.random.default_rng(n)
+    A = (rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))) * (0.1 / np.sqrt(n))
+    A[np.arange(n), np.arange(n)] += rng.uniform(1.0, 2.0, n)
+    A = A[rng.permutation(n)]
+    X, st = ctx.zinv(A)
+    assert st == 0 and np.abs(A @ X - np.eye(n)).max() < 50 * 2.2e-16 * n * 4
+    with pytest.raises(Exception):
+        ctx.zinv(np.eye(2768, dtype=complex))
+
+
 @pytest.mark.parametrize("n", [40, 70, 300, 530])
 def test_far_pivots(ctx, n):
     """A scaled permutation (every pivot off the diagonal), and rows of very

@@ -338,9 +338,15 @@ void zinv_small_batched(cplx* const* d_mats, int batch, int n, int* d_status, cu
   VRC_CUDA_CHECK(cudaGetLastError());
 }
 
-// Panel columns: what a thread's registers hold with a row per thread up to
-// n = 512 and two above (512 threads, 128 registers each).
-int zinv_blocked_width(int n) { return n <= 512 ? 16 : 8; }
+// Panel columns: what a thread's registers hold (512 threads, 128 registers
+// each) with a row per thread up to n = 512, two up to 1024, the largest order
+// of a structure, and six above, where only matrices inverted by themselves
+// (vrc_zinv) come in.
+int zinv_blocked_width(int n) { return n <= 512 ? 16 : n <= 1024 ? 8 : 4; }
+
+// The largest order taken: four columns of a matrix, the multipliers and the
+// pivots in one CTA's shared memory, as a panel needed when it was kept there.
+constexpr int ZB_MAXN = 2767;
 
 size_t zinv_blocked_scratch(int n) {
   const int w = zinv_blocked_width(n);
@@ -350,7 +356,7 @@ size_t zinv_blocked_scratch(int n) {
 void zinv_blocked_batched(cplx* const* d_mats, int batch, int n, int* d_status, void* scratch,
                           const GemmDesc* d_descs, cudaStream_t stream) {
   if (batch <= 0) return;
-  if (n > 1024) throw StatusError(ST_EINVAL, "blocked inversion: n <= 1024");
+  if (n > ZB_MAXN) throw StatusError(ST_EINVAL, "inversion: matrix too large");
   const int W = zinv_blocked_width(n);
   const size_t per = zinv_blocked_scratch(n) / 16;
   const size_t psm = (size_t)4 * n * sizeof(cplx);
@@ -363,10 +369,11 @@ void zinv_blocked_batched(cplx* const* d_mats, int batch, int n, int* d_status, 
     for (int k = 0; k < n; k += W) {
       const int w = min(W, n - k);
       int* st = d_status ? d_status + b0 : nullptr;
-      const int threads = (n <= 512 ? n + 31 : (n + 1) / 2 + 31) / 32 * 32;
-      auto panel = n <= 256   ? zinv_panel_kernel<256, 1, 16>
-                   : n <= 512 ? zinv_panel_kernel<512, 1, 16>
-                              : zinv_panel_kernel<512, 2, 8>;
+      const int rows = n <= 512 ? 1 : n <= 1024 ? 2 : 6, threads = ((n + rows - 1) / rows + 31) / 32 * 32;
+      auto panel = n <= 256    ? zinv_panel_kernel<256, 1, 16>
+                   : n <= 512  ? zinv_panel_kernel<512, 1, 16>
+                   : n <= 1024 ? zinv_panel_kernel<512, 2, 8>
+                               : zinv_panel_kernel<512, 6, 4>;
       panel<<<nb, threads, 0, stream>>>(d_mats + b0, sb, per, n, k, w, st);
       VRC_CUDA_CHECK(cudaGetLastError());
       // descriptor b: A = M (n x w, leading dimension n), B = X (w x n,
