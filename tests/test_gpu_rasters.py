@@ -51,6 +51,17 @@ def test_toeplitz_orders(ctx, nx, ny):
         assert relerr(P[0], oP) < 1e-12 and relerr(Q[0], oQ) < 1e-12
 
 
+@pytest.mark.parametrize("nx,ny", [(t, 1) for t in range(35, 64, 2)] + [(1, 47)])
+def test_toeplitz_every_wide_order(ctx, nx, ny):
+    """Above 32 harmonics the shared memory that a launch asks for grows with each."""
+    rng = np.random.default_rng(nx + 100 * ny)
+    eps = rng.uniform(2.0, 12.0, (3, 5)) + 1j * rng.uniform(0.0, 0.5, (3, 5))
+    d = dict(kind="pixels", lam=1.1, nx=nx, ny=ny, pml=False, Lx=0.9, Ly=0.7, eps=eps, z0=0.0, z1=0.4)
+    P, Q = ctx.sample_pq(d, [0.1])
+    oP, oQ = make_sampler(d).sample(0.1)
+    assert relerr(P[0], oP) < 1e-12 and relerr(Q[0], oQ) < 1e-12
+
+
 @pytest.mark.parametrize("npy,npx,nx,ny", [(7, 12, 3, 3), (12, 7, 3, 5), (9, 33, 5, 1), (16, 8, 1, 5), (10, 17, 5, 3)])
 def test_pixel_gradients(ctx, npy, npx, nx, ny):
     rng = np.random.default_rng(npx)

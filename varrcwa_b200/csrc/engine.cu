@@ -487,7 +487,9 @@ size_t Engine::batch_chunk(size_t count, size_t per, size_t most, bool in_worksp
 // Batched primitives
 // ---------------------------------------------------------------------------
 void ensure_smem(const void* kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return;
+  // A launch has 48 KB without asking, what the kernel declares itself included
+  // (at most 8.5 KB here).
+  if (bytes <= 32 * 1024) return;
   static std::mutex mu;
   static std::map<const void*, size_t> limit;
   std::lock_guard<std::mutex> lock(mu);
