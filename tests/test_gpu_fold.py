@@ -260,3 +260,20 @@ def test_late_asymmetry(ctx, monkeypatch, method, call, make, beside):
         assert _same_bits(a, b, ("R", "T") if call == "order_powers" else ("Tdd", "Tuu", "Rud", "Rdu", "W0", "W1"))
         if call == "blocks":
             assert all(a[k] == b[k] for k in ("N", "n_eig", "n_samples", "n_nodes"))
+
+
+def test_first_pass_allocations(monkeypatch):
+    """The classes' many small blocks come in no more pieces than the whole
+    cells' few large ones, which take more memory."""
+    from varrcwa_b200.capi import Context
+    monkeypatch.setenv("VRC_LANES", "1")
+    cells = [_pillar(40 + k, 7, 7, npx=32, npy=32) for k in range(300)]
+    calls = []
+    for env in (None, "1"):
+        monkeypatch.delenv("VRC_NO_FOLD", raising=False) if env is None else monkeypatch.setenv("VRC_NO_FOLD", env)
+        c = Context(0)
+        before = c.kernel_stats()["host_alloc"]["bytes"]
+        c.rcwa(cells, 4, blocks=False)
+        calls.append(c.kernel_stats()["host_alloc"]["bytes"] - before)  # (of this entry: the number of calls)
+        c.close()
+    assert calls[0] <= calls[1]

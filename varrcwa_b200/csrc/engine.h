@@ -110,8 +110,8 @@ class BlockPool {
  public:
   explicit BlockPool(size_t bytes) : bytes_(bytes) {}
   ~BlockPool();
-  // a block (a new 64 MB chunk when none is free); nullptr when the device
-  // has no room for a chunk
+  // a block (when none is free from a new chunk, as large as the pool so far, 256
+  // blocks at least and 64 MB at most); nullptr when the device has no room
   void* get(cudaStream_t st);
   void put(void* p) { free_.push_back(p); }
   // frees the chunks none of whose blocks is handed out (cudaFree, which
