@@ -380,7 +380,7 @@ int vrc_get_kernel_stats(vrc_context* ctx, int max, vrc_kernel_stat* out);
 /* ---- batched kernels (host buffers) --------------------------------------- */
 /* C[b] = A[b] * B[b]  (batch n*n complex GEMMs on FP64 tensor cores). */
 int vrc_zgemm(vrc_context* ctx, int batch, int n, const vrc_complex* A, const vrc_complex* B, vrc_complex* C);
-/* In-place inverse of batch n*n matrices; status[b] = VRC_ESINGULAR on a zero pivot. */
+/* In-place inverse of batch n*n matrices (n <= 2767); status[b] = VRC_ESINGULAR on a zero pivot. */
 int vrc_zinv(vrc_context* ctx, int batch, int n, vrc_complex* A, int* status);
 
 /* ---- eigen-decomposition without device allocation ------------------------

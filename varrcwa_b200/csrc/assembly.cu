@@ -169,8 +169,8 @@ __global__ void reciprocal_kernel(cplx* const* __restrict__ in, cplx* const* __r
 // raster).  transB = 0: B is K x N (ldb); transB = 1: B is N x K (ldb), use B^T.
 // A CTA computes SG_M x 16 NQ, a row and NQ columns per thread, its operands
 // staged through shared memory in slices of SG_K, ST in flight.  With NQ = 4 a
-// warp has 16 FP64 instructions to five shared loads per slice entry, so the FP64
-// pipe and the shared-memory port are about level; where tiles of 64 columns do
+// warp has 16 FP64 instructions to five shared loads per slice entry: bound by the
+// shared-memory port (83 to 88% busy for 256 samples, the FP64 pipe 50%); where tiles of 64 columns do
 // not give every SM a CTA, NQ = 1 shortens each CTA's chain and spreads it (few
 // samples of 256 x 256 pixels at 7 orders: 14 and 19 us a launch, transposed or
 // not, against 20 and 24).  One thread per output, its operands from global memory
@@ -252,8 +252,8 @@ __global__ void __launch_bounds__(SG_THREADS)
 // out + r*t*t.  Gauss-Jordan in place with partial pivoting; rows stay where
 // they are, the pivot's row goes to all through shared memory, and the
 // permutation is undone by the stores.  Bound by the chain of one step (pivot
-// search, reciprocal, the row's way round) and, with many matrices, by the FP64
-// pipe: the strips of sixteen pillars at t = 11 take 45 us a launch, with a warp
+// search, reciprocal, the row's way round) and, with many matrices, by issue
+// (63%; FP64 44%): the strips of sixteen pillars at t = 11 take 45 us a launch, with a warp
 // per matrix in shared memory and a lane per column 118; one taper pass at
 // t = 41 spends 1.7 ms in its assembly, before 2.9.
 // ---------------------------------------------------------------------------

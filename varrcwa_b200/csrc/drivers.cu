@@ -862,7 +862,10 @@ void Engine::order_powers(const std::vector<CellSpec>& cells, const std::vector<
 // asymmetric on the way, takes the general way.  Below nine harmonics there is
 // nothing to split.  General / folded: one 7 x 7-order pillar 38 / 11 ms, 16 at
 // 11 x 11 orders 348 / 71, 16 slices of two at 13 x 9 orders 59 / 9, a taper of
-// 41 orders 24.7 / 14.9, a planar taper of 11 x 5 orders 16.4 / 12.4.  On a square
+// 41 orders 24.7 / 14.9, a planar taper of 11 x 5 orders 16.4 / 12.4.  Plain solves
+// of a few small cells that return blocks, whose end media are solved once more
+// at full order, lose up to 0.9 ms: one differential slice at 3 x 3 orders 1.3 / 1.8,
+// at 7 x 7 4.6 / 5.1, at 41 3.9 / 4.8, one RCWA slice at 3 x 3 1.8 / 2.0.  On a square
 // lattice the modes of two classes are degenerate in pairs; apart in their
 // classes, the adaptive tree no longer depends on how a solver's rounding mixes
 // them.

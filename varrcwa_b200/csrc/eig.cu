@@ -201,12 +201,13 @@ __global__ void __launch_bounds__(HESS_THREADS)
 // with zeros to 8 RV) and the CTA 32 columns at a time: both products in one
 // pass, v^H a_j kept in registers for the update, and every warp forms the
 // reflector for itself.  A column passes three barriers (the warps' shares of
-// A v, their sum, the next reflector's column).  Bound by that chain and, with
-// the SMs full, by shared memory and the FP64 pipe.  One / 600 matrices take
-// 0.11 / 0.37 ms at n = 42, 0.21 / 0.73 at 61 (hess_kernel 0.51 for some 60) and
-// 0.58 / 2.9 at 98 (panels and GEMM updates 0.93 / 4.1), 0.75 / 3.8 at 113 (1.00 /
-// 5.1) and 0.76 / 3.9 at 115 (1.02 / 5.3).  RV = 15 leaves the padding out, the only form that fits above 112 (a row
-// more in a lane, padded, holds 111).
+// A v, their sum, the next reflector's column).  Bound by that chain, with the
+// SMs full too (600 at n = 61: issue and the shared-memory port 46%, FP64 33%).
+// One / 600 matrices take 0.11 / 0.37 ms at n = 42, 0.21 / 0.73 at 61 (hess_kernel
+// 0.51 for some 60) and 0.58 / 2.9 at 98 (panels and GEMM updates 0.93 / 4.1),
+// 0.75 / 3.8 at 113 (1.00 / 5.1) and 0.76 / 3.9 at 115 (1.02 / 5.3).  RV = 15
+// leaves the padding out, the only form that fits above 112 (a row more in a
+// lane, padded, holds 111).
 constexpr size_t hs_smem(int n, int rv) {
   return ((size_t)(n + HESS_WARPS + 2) * (rv == 15 ? n : 8 * rv) + HESS_WARPS) * sizeof(cplx);
 }

@@ -22,8 +22,9 @@ namespace {
 // next column updates it first, finds its pivot and the reciprocal while the
 // others still update, and hands all three on through shared memory; the pivot's
 // row comes from the lane that holds it.  Bound by the chain of a step (row,
-// update of a column, search, reciprocal: 0.7 us at n = 25, 1.1 at 96) for few
-// matrices, by the FP64 pipe for many.
+// update of a column, search, reciprocal: 0.7 us at n = 25, 1.1 at 96), also with
+// the SMs full (600 at n = 96: issue 40%, the FP64 pipe 34%, barriers first among
+// the stalls).
 // ---------------------------------------------------------------------------
 constexpr int ZS_MAXN = 96;
 
@@ -165,8 +166,9 @@ __global__ void __launch_bounds__(32 * W)
 // largest is as good; magnitudes below 4.2e-314, whose reciprocal overflows,
 // count as zero) with one warp reduction each side of it, and every warp's
 // candidate puts out its row and the reciprocal of its pivot before it is known
-// which one is taken.  Bound by that chain for few matrices and by the FP64
-// issue of the update for many.
+// which one is taken.  Bound by that chain and by the loads, whose pivot rows
+// are single entries of every column (64 matrices at n = 450: waits for memory
+// first among the stalls, the FP64 pipe 12%).
 // With rows split over two threads, exchanges, and every thread reducing the
 // candidates and forming the reciprocal, a pivot took 4,700 cycles at n = 162,
 // the row moves 25,000 cycles per panel and the final column exchanges one

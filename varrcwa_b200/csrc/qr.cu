@@ -216,8 +216,8 @@ __device__ __forceinline__ void cpa_wait() {
 // rounds [ra0, ra1) of [r0, r1) are its own.  Bank conflict free: consecutive
 // bulges are 3 FV entries apart.
 //
-// Bounded by the FP64 pipe and issue (12 FP64 instructions of about 30 per
-// round and warp).  One thread per vector and bulge after bulge, straight from
+// Bounded by issue with two CTAs per SM (12 FP64 instructions of about 30 per
+// round and warp), else by a round's latency.  One thread per vector and bulge after bulge, straight from
 // global memory, took 234 cycles per rotation at n = 242: on a row transform
 // every lane walks a column of its own, so each access was 32 sectors, eight
 // times over.
@@ -991,8 +991,9 @@ __global__ void __launch_bounds__(QR_THREADS, 2)
 // as strip_rounds does.  The log is one stream: it comes in through a ring of
 // four chunks, two ahead of the one in use, whatever sweep they belong to.
 //
-// Bounded by the FP64 pipe when several warps share a scheduler, by the
-// latency of a round (some 50 cycles) when the batch is small.  One thread
+// Bounded by issue when several warps share a scheduler (600 matrices at n = 61:
+// 75% of the slots, FP64 27%), by the latency of a round (some 50 cycles) when the
+// batch is small or n leaves two blocks to an SM (n = 450: 32%).  One thread
 // per vector with four bulges in a register ring, its entries streamed from
 // global memory once per four bulges and sweep, took 525 cycles per round and
 // four bulges, and two memory latencies at the start of every sweep.
